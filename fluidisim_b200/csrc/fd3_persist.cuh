@@ -1,0 +1,312 @@
+// The inner CG loop in one cooperative launch, for volumes without the multigrid (Jacobi-PCG and the
+// linear path's CG).
+//
+// Without the multigrid an iteration is four short passes, and as separate kernels each pays a launch
+// boundary, a chain of dependent loads (gate, codes, operands) and the last block's merge of the
+// partials: 26 us per iteration at 215k cells, 19 at 65k, where the passes' bytes take 1 us from L2.
+// Here one CTA per SM keeps its cells' p, r, diagonal and row on chip for the whole loop, and the
+// iteration has two grid-wide meetings, each a reduction and a barrier at once (GridTeam::sum).
+// Between them a cell exchanges with its neighbours only z and the last direction, through L2.
+//
+// Measured (B200, whole calls): a projection of 75 x 61 x 47 cells (260 iterations) 7.22 -> 1.97 ms, the linear
+// step of 64 x 32 x 32 (244 iterations) 5.04 -> 1.57 ms: 6 us per iteration, of which the two meetings take 4.3.
+#pragma once
+
+#include "fd3_fast.cuh"
+
+namespace fd3 {
+
+constexpr int GRID_THREADS = 512;   // one CTA per SM: the meetings cost less with fewer CTAs and warps
+constexpr int GRID_MAX_CTAS = 160;  // slots
+constexpr int GRID_MAX_CELLS = 12;  // cells of a thread (k_cg_loop's largest instance)
+constexpr size_t cg_smem(int cells) { return (size_t)cells * 7 * GRID_THREADS * sizeof(float); }
+// Polls before a CTA gives up (about a second): a meeting that never completes ends the kernel with
+// status 100 instead of hanging the GPU.
+constexpr unsigned GRID_POLLS = 1u << 20;
+
+// The CTAs of a cooperative grid as one team, meeting at a counter that is 0 at the launch and never
+// reset.  A meeting is one release-add and an acquire-poll by one thread per CTA (1.3 us on 148 CTAs); a sum
+// adds the CTAs' partials in its slots (2.1 us).  Polling the slots themselves, one number per CTA beside its
+// partial, took 5.6 us (148 x 148 polls of the same lines), and mailboxes per reader 2.6 us.  The slots
+// alternate between two sets: a CTA writes a set again only after a later meeting, which every CTA has
+// reached only after reading it.
+struct GridSlots {
+  double2 part[2][GRID_MAX_CTAS];
+  unsigned arrived;
+};
+struct GridShared {
+  double warp[GRID_THREADS / 32][2];
+  double sum[2];
+};
+struct GridTeam {
+  GridSlots* slots;
+  GridShared& sh;
+  unsigned meeting = 0;
+  __device__ __forceinline__ GridTeam(GridSlots* s, GridShared& shared) : slots(s), sh(shared) {}
+
+  // Called by every thread of every CTA; what the team wrote to global memory before is visible to all of
+  // it after.  False, for the whole CTA, when another did not arrive within GRID_POLLS.
+  __device__ __forceinline__ bool arrive_and_wait() {  // thread 0; the CTA's writes ordered before by a barrier
+    ++meeting;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&slots->arrived) : "memory");
+    const unsigned target = meeting * gridDim.x;
+    unsigned seen, polls = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&slots->arrived) : "memory");
+    } while (seen < target && ++polls < GRID_POLLS);
+    return seen >= target;
+  }
+  // Sums a (and b, when TWO) over every thread of the grid: the same totals, added in the same order, for
+  // every thread.  A meeting.
+  template <bool TWO>
+  __device__ __forceinline__ bool sum(double& a, double& b) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (TWO) b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+      sh.warp[wid][0] = a;
+      if (TWO) sh.warp[wid][1] = b;
+    }
+    __syncthreads();
+    double2* half = slots->part[meeting & 1u];
+    bool late = false;
+    if (threadIdx.x == 0) {
+      double2 p = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int q = 0; q < GRID_THREADS / 32; ++q) {
+        p.x += sh.warp[q][0];
+        if (TWO) p.y += sh.warp[q][1];
+      }
+      __stcg(half + blockIdx.x, p);
+      late = !arrive_and_wait();
+    } else {
+      ++meeting;
+    }
+    if (__syncthreads_or(late)) return false;
+    if (wid == 0) {
+      constexpr int PER = (GRID_MAX_CTAS + 31) / 32;
+      double2 v[PER];
+#pragma unroll
+      for (int e = 0; e < PER; ++e) {
+        const int q = lane + 32 * e;
+        v[e] = q < (int)gridDim.x ? __ldcg(half + q) : make_double2(0.0, 0.0);
+      }
+      a = b = 0.0;
+#pragma unroll
+      for (int e = 0; e < PER; ++e) {
+        a += v[e].x;
+        if (TWO) b += v[e].y;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (TWO) b += __shfl_xor_sync(0xffffffffu, b, o);
+      }
+      if (lane == 0) {
+        sh.sum[0] = a;
+        sh.sum[1] = b;
+      }
+    }
+    __syncthreads();
+    a = sh.sum[0];
+    b = sh.sum[1];
+    return true;
+  }
+};
+
+// The meeting counter to 0, before a launch that meets.
+__global__ void k_grid_reset(GridSlots* slots) {
+  KSTART();
+  slots->arrived = 0u;
+}
+
+// A cell's row kept on chip: per face the aperture onto a fluid neighbour, or the ghost's 1/theta (the
+// lid: twice the aperture), evaluated as apply_code does, a (pc - x) and (a pc) it.  ROW_CUT_GHOST marks the
+// rare row with a ghost face whose aperture is not 1, which reads that aperture again.
+constexpr unsigned ROW_CUT_GHOST = 1u << 14;
+__device__ __forceinline__ unsigned kept_row(const Geo& g, unsigned code, int i, int j, int k, float (&w)[6]) {
+  const bool unit = code & RC_UNIT;
+  const int axis[6] = {0, 0, 1, 1, 2, 2};
+  const int fi[6] = {fu(g, i, j, k), fu(g, i + 1, j, k), fv(g, i, j, k), fv(g, i, j + 1, k), fw(g, i, j, k),
+                     fw(g, i, j, k + 1)};
+  const int xs[4] = {i - 1, i + 1, i, i}, ys[4] = {j, j, j - 1, j + 1};
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const unsigned st = face_state(code, f);
+    w[f] = 0.f;
+    if (!st) continue;
+    const float a = unit ? 1.f : aper3(g, axis[f], fi[f]);
+    if (st == 1) w[f] = a;
+    else if (f == 5 && g.linear) w[f] = 2.f * a;
+    else {
+      w[f] = f == 5 ? ghost_it_up(g, i, j, k) : ghost_it_side(g, i, j, k, xs[f < 4 ? f : 0], ys[f < 4 ? f : 0]);
+      if (a != 1.f) code |= ROW_CUT_GHOST;
+    }
+  }
+  return code;
+}
+__device__ __noinline__ float face_aperture(const Geo& g, int c, int f) {
+  int i, j, k;
+  cell_ijk(g, c, i, j, k);
+  if (f < 2) return aper3(g, 0, fu(g, i + f, j, k));
+  if (f < 4) return aper3(g, 1, fv(g, i, j + f - 2, k));
+  return aper3(g, 2, fw(g, i, j, k + f - 4));
+}
+// W(f): the kept coefficient of face f; v: the operand at the six neighbours (any value where the face has
+// no fluid neighbour).
+template <class W>
+__device__ __forceinline__ float apply_kept(const Geo& g, unsigned code, int c, float pc, W w, const float (&v)[6]) {
+  float acc = 0.f;
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const unsigned st = face_state(code, f);
+    float ghost = pc * w(f);
+    if ((code & ROW_CUT_GHOST) && st == 2u && !(f == 5 && g.linear)) ghost = face_aperture(g, c, f) * pc * w(f);
+    acc += st == 1u ? w(f) * (pc - v[f]) : (st == 2u ? ghost : 0.f);
+  }
+  return acc * g.inv;
+}
+
+// The Jacobi-PCG loop (delta3d_mobile.rs:515-545 with z = prec r): its prime, then iterations until
+// S->active drops, with the scalar steps of apply_op (f64 reductions).  Thread t of the T threads of the
+// grid owns the cells t, t + T, ...: CELLS of them, each with r, prec, its code and direction in registers
+// and p and its row's coefficients in shared memory (14 KB per cell of a thread).
+// Per iteration: d = z + beta d at the cell and, recomputed from z and the previous d, at its neighbours;
+// q = A d; d.q | p += alpha d, r -= alpha q, z = prec r; r.r and r.z together.  z and the two
+// alternating direction buffers live in global memory, read past L1 (other SMs write them).
+template <int CELLS>
+__global__ void __launch_bounds__(GRID_THREADS, 1)
+    k_cg_loop(const __grid_constant__ Geo g, const unsigned short* __restrict__ codes, const float* __restrict__ prec, float* p,
+              float* r, float* d0, float* d1, float* z, Scalars* S, GridSlots* slots) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // no early start of the next kernel: its CTAs find no room
+  if (!S->active) return;
+  extern __shared__ float kept[];  // [CELLS][7][GRID_THREADS]: six coefficients and p
+  __shared__ GridShared sh;
+  GridTeam team(slots, sh);
+  auto K = [&](int s, int f) -> float& { return kept[(s * 7 + f) * GRID_THREADS + threadIdx.x]; };
+  constexpr int PAIR = CELLS < 2 ? 1 : 2;
+  const int nxny = g.nx * g.ny;
+  const int T = gridDim.x * GRID_THREADS, t0 = blockIdx.x * GRID_THREADS + threadIdx.x;
+  float rc[CELLS], mc[CELLS], dc[CELLS], qc[CELLS];
+  unsigned code[CELLS];
+  double acc = 0.0, acc2 = 0.0;
+#pragma unroll
+  for (int s = 0; s < CELLS; ++s) {
+    const int c = t0 + s * T;
+    rc[s] = mc[s] = dc[s] = qc[s] = 0.f;
+    code[s] = 0u;
+    if (c < g.n) {
+      K(s, 6) = p[c];
+      rc[s] = r[c];
+      mc[s] = prec[c];
+      const unsigned rc16 = codes[c];
+      if (rc16 & RC_WET) {
+        int i, j, k;
+        cell_ijk(g, c, i, j, k);
+        float w[6];
+        code[s] = kept_row(g, rc16, i, j, k, w);
+#pragma unroll
+        for (int f = 0; f < 6; ++f) K(s, f) = w[f];
+      }
+      z[c] = mc[s] * rc[s];
+      acc += (double)rc[s] * (double)mc[s] * (double)rc[s];
+    }
+  }
+  double rz, rr = S->rr;
+  const double tolb2 = S->tolb2, phys = S->phys;
+  unsigned it = S->it;
+  const unsigned max_iters = S->max_iters;
+  int status = 0, brk = 0;
+  float beta = 0.f;
+  float* din = d0;
+  float* dout = d1;
+  if (!team.sum<false>(acc, acc2)) status = 100;
+  rz = acc;
+  if (!status && !isfinite(rz)) status = 2;
+  while (!status) {
+    acc = 0.0;
+    acc2 = 0.0;
+    // PAIR cells' twelve loads each go out together; the stores of the direction come after them all
+#pragma unroll
+    for (int s0 = 0; s0 < CELLS; s0 += PAIR) {
+      float v[PAIR][6];
+#pragma unroll
+      for (int e = 0; e < PAIR; ++e) {
+        const int s = s0 + e, c = t0 + s * T;
+        if (s >= CELLS) continue;
+        const int nb[6] = {c - 1, c + 1, c - g.nx, c + g.nx, c - nxny, c + nxny};
+        float zn[6], dn[6];
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+          const bool on = face_state(code[s], f) == 1u;
+          zn[f] = on ? __ldcg(z + nb[f]) : 0.f;
+          dn[f] = on && beta != 0.f ? __ldcg(din + nb[f]) : 0.f;
+        }
+#pragma unroll
+        for (int f = 0; f < 6; ++f) v[e][f] = beta == 0.f ? zn[f] : zn[f] + beta * dn[f];
+      }
+#pragma unroll
+      for (int e = 0; e < PAIR; ++e) {
+        const int s = s0 + e, c = t0 + s * T;
+        if (s >= CELLS) continue;
+        const float zc = mc[s] * rc[s];
+        const float d = beta == 0.f ? zc : zc + beta * dc[s];
+        qc[s] = (code[s] & RC_WET) ? apply_kept(g, code[s], c, d, [&](int f) { return K(s, f); }, v[e]) : 0.f;
+        dc[s] = d;
+        acc += (double)d * (double)qc[s];
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < CELLS; ++s) {
+      const int c = t0 + s * T;
+      if (c < g.n) dout[c] = dc[s];
+    }
+    if (!team.sum<false>(acc, acc2)) { status = 100; break; }
+    if (!(acc > 0.0)) { brk = 1; break; }  // FIN_DQ
+    const float alpha = (float)(rz / acc);
+    acc = 0.0;
+    acc2 = 0.0;
+#pragma unroll
+    for (int s = 0; s < CELLS; ++s) {
+      const int c = t0 + s * T;
+      if (c < g.n) {
+        K(s, 6) += alpha * dc[s];
+        const float rn = rc[s] - alpha * qc[s];
+        rc[s] = rn;
+        z[c] = mc[s] * rn;
+        acc += (double)rn * (double)rn;
+        acc2 += (double)rn * (double)mc[s] * (double)rn;
+      }
+    }
+    if (!team.sum<true>(acc, acc2)) { status = 100; break; }
+    if (!isfinite(acc)) { status = 2; break; }  // FIN_RN
+    ++it;
+    rr = acc;
+    if (!((acc > tolb2 || acc > phys) && it < max_iters)) break;
+    if (!isfinite(acc2)) { status = 2; break; }  // FIN_RZ_ITER
+    beta = (float)(acc2 / rz);
+    rz = acc2;
+    float* t = din;
+    din = dout;
+    dout = t;
+  }
+#pragma unroll
+  for (int s = 0; s < CELLS; ++s) {
+    const int c = t0 + s * T;
+    if (c < g.n) { p[c] = K(s, 6); r[c] = rc[s]; }
+  }
+  // every CTA has met for the last time here, but one that gave up says so whichever it is
+  if (threadIdx.x == 0 && (blockIdx.x == 0 || status == 100)) {
+    S->rr = rr;
+    S->rz = rz;
+    S->it = it;
+    S->brk = brk;
+    if (status) S->status = status;
+    S->active = 0;
+  }
+}
+
+}  // namespace fd3

@@ -29,6 +29,7 @@
 #include "fd3_tmarch.cuh"
 #include "fd3_batch.cuh"
 #include "fd3_linear.cuh"
+#include "fd3_persist.cuh"
 #include "fd3_levels.cuh"
 
 using namespace fd3;
@@ -148,6 +149,8 @@ struct fd3_volume {
   int p64_cap = 0;  // f64 partial slots
   float* p32 = nullptr;
   unsigned* count = nullptr;
+  GridSlots* slots = nullptr;  // the meetings of k_cg_loop
+  int grid_ctas = 0;          // CTAs of a cooperative launch of GRID_THREADS threads (one per SM)
   Scalars* dS = nullptr;
   Scalars* hS = nullptr;  // pinned
   int* dflag = nullptr;
@@ -226,6 +229,12 @@ struct fd3_volume {
     return opt.kernels == 4 || (opt.kernels == 0 && (long long)n >= kQuadMinCells);
   }
   bool mg_on() const { return has_mg && !linear; }  // the linear path has no multigrid
+  // Without the multigrid, the inner loop in one cooperative launch (k_cg_loop), up to the cells its
+  // threads hold in registers; larger volumes, the ordered mode and use_graphs = 0 keep the four
+  // kernels per iteration.
+  bool cg_loop() const {
+    return !ord() && !mg_on() && opt.use_graphs && (long long)n <= (long long)grid_ctas * GRID_THREADS * GRID_MAX_CELLS;
+  }
   // FP16 storage of the V-cycle vectors (fd3_set_options accepts it only with the paired kernels)
   bool half() const { return opt.storage == FD3_STORAGE_F16 && paired() && mg_on(); }
   int loop_key() const {
@@ -819,16 +828,61 @@ int build_loop_graph(fd3_volume* V) {
   return FD3_OK;
 }
 
+// The inner loop without the multigrid, prime included, as one cooperative launch.
+template <int CELLS>
+void launch_cg_loop(fd3_volume* V, int ctas) {
+  cudaEvent_t a = nullptr, b = nullptr;
+  if (V->prof) { a = next_event(V); cudaEventRecord(a, V->stream); }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(GRID_THREADS);
+  cfg.dynamicSmemBytes = cg_smem(CELLS);
+  cfg.stream = V->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_cg_loop<CELLS>, V->geo(), (const unsigned short*)V->codes, (const float*)V->prec, V->p,
+                     V->res, V->dir, V->dir2, V->tmp, V->dS, V->slots);
+  if (V->prof) { b = next_event(V); cudaEventRecord(b, V->stream); V->pending.push_back({"k_cg_loop", a, b}); }
+  V->launches++;
+}
+void run_cg_loop(fd3_volume* V) {
+  LAUNCH_G(V, k_grid_reset, 1, 1, V->slots);
+  const int ctas = std::min(V->grid_ctas, (V->n + GRID_THREADS - 1) / GRID_THREADS);
+  const int cells = (V->n + ctas * GRID_THREADS - 1) / (ctas * GRID_THREADS);
+  if (cells <= 1) launch_cg_loop<1>(V, ctas);
+  else if (cells <= 2) launch_cg_loop<2>(V, ctas);
+  else if (cells <= 3) launch_cg_loop<3>(V, ctas);
+  else if (cells <= 4) launch_cg_loop<4>(V, ctas);
+  else if (cells <= 8) launch_cg_loop<8>(V, ctas);
+  else launch_cg_loop<GRID_MAX_CELLS>(V, ctas);
+}
+
+// The whole inner loop enqueued, without a synchronisation: the cooperative launch, or the loop graph.
+int enqueue_loop(fd3_volume* V) {
+  if (V->cg_loop()) {
+    run_cg_loop(V);
+    return FD3_OK;
+  }
+  const int mode = V->loop_key();
+  if (!V->loop_exec || V->loop_mode != mode || V->loop_stream != V->stream) TRY(build_loop_graph(V));
+  CK(cudaGraphLaunch(V->loop_exec, V->stream));
+  return FD3_OK;
+}
+// The launches of `ran` iterations of the loop graph (the cooperative launch counts itself).
+void count_loop(fd3_volume* V, unsigned ran) {
+  if (!V->cg_loop()) V->launches += (unsigned long long)((ran + 1) / 2) * V->body_nodes;
+}
+
 // Run the inner loop until S->active drops.
 int run_inner(fd3_volume* V, uint32_t it_before) {
-  const bool graphs = V->opt.use_graphs && !V->prof;
+  const bool graphs = V->cg_loop() || (V->opt.use_graphs && !V->prof);
   if (graphs) {
-    int mode = V->loop_key();
-    if (!V->loop_exec || V->loop_mode != mode || V->loop_stream != V->stream) TRY(build_loop_graph(V));
-    CK(cudaGraphLaunch(V->loop_exec, V->stream));
+    TRY(enqueue_loop(V));
     TRY(pull(V));
-    unsigned ran = V->hS->it > it_before ? V->hS->it - it_before : 1;
-    V->launches += (unsigned long long)((ran + 1) / 2) * V->body_nodes;
+    count_loop(V, V->hS->it > it_before ? V->hS->it - it_before : 1);
     return FD3_OK;
   }
   // The device clears S->active within max_iters iterations (FIN_RN); the host bound is a guard.
@@ -971,18 +1025,17 @@ int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd
   // would not have started it) and the outer checks, with one synchronisation at their end.  A
   // prime that turns out unneeded changes nothing the checks or the report read; a non-finite
   // set-up stops the loop on the device and is reported after the checks, as before them.
-  const bool speculate = !ord && V->mg_on() && V->opt.use_graphs && !V->prof;
+  const bool cg = V->cg_loop();  // its loop primes itself
+  const bool speculate = !ord && (V->mg_on() || cg) && V->opt.use_graphs && !V->prof;
   Checks ck{};
   bool have_checks = false;
   if (speculate) {
-    prime(V);
+    if (!cg) prime(V);
     LAUNCH_G(V, k_loop_start_dev, 1, 1, V->dS, max_iters);
-    const int mode = V->loop_key();
-    if (!V->loop_exec || V->loop_mode != mode || V->loop_stream != V->stream) TRY(build_loop_graph(V));
-    CK(cudaGraphLaunch(V->loop_exec, V->stream));
+    TRY(enqueue_loop(V));
     TRY(outer_checks(V, k1, &ck));
     if (V->hS->status) return V->hS->status;
-    V->launches += (unsigned long long)((std::max(V->hS->it, 1u) + 1) / 2) * V->body_nodes;
+    count_loop(V, std::max(V->hS->it, 1u));
     have_checks = true;
   } else {
     TRY(pull(V));
@@ -1014,19 +1067,16 @@ int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd
     } else {
     if (b2 > 0 && above(rr) && it < max_iters) {
       if (!primed) {
-        prime(V);
+        if (!cg) prime(V);
         primed = true;
       }
       LAUNCH_G(V, k_loop_start, 1, 1, V->dS, rr, tolb2, phys, it, max_iters);
       V->hS->max_iters = max_iters;
       if (speculate) {  // the loop and the checks behind it, one synchronisation (the checks keep it and rr)
-        const int mode = V->loop_key();
-        if (!V->loop_exec || V->loop_mode != mode || V->loop_stream != V->stream) TRY(build_loop_graph(V));
-        CK(cudaGraphLaunch(V->loop_exec, V->stream));
+        TRY(enqueue_loop(V));
         TRY(outer_checks(V, k1, &ck));
         if (V->hS->status) return V->hS->status;
-        const unsigned ran = V->hS->it > it ? V->hS->it - it : 1;
-        V->launches += (unsigned long long)((ran + 1) / 2) * V->body_nodes;
+        count_loop(V, V->hS->it > it ? V->hS->it - it : 1);
         it = V->hS->it;
         rr = V->hS->rr;
       } else {
@@ -1078,7 +1128,7 @@ int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd
       since = 0;
     }
     rr = actual;
-    prime(V);
+    if (!cg) prime(V);
   }
   double residual;
   if (ord) residual = b2 > 0 ? (double)std::sqrt((float)actual_rr / (float)b2) : 0.0;
@@ -1273,6 +1323,18 @@ int alloc_state(fd3_volume* V) {
   TRY(dalloc(V, &V->p32, (size_t)(V->n + CHUNK - 1) / CHUNK + 64));
   TRY(dalloc(V, &q, sizeof(Scalars) / sizeof(float) + 16)); V->dS = (Scalars*)q;
   TRY(dalloc(V, &q, 16)); V->dflag = (int*)q;
+  TRY(dalloc(V, &q, (sizeof(GridSlots) + 3) / 4)); V->slots = (GridSlots*)q;
+  int sms = 0, coop = 0, resident = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, V->device));
+  CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, V->device));
+  // the attribute is per function, shared by every volume: the size each instance always asks for
+  CK(cudaFuncSetAttribute(k_cg_loop<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(4)));
+  CK(cudaFuncSetAttribute(k_cg_loop<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(8)));
+  CK(cudaFuncSetAttribute(k_cg_loop<GRID_MAX_CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)cg_smem(GRID_MAX_CELLS)));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_cg_loop<GRID_MAX_CELLS>, GRID_THREADS,
+                                                   cg_smem(GRID_MAX_CELLS)));
+  V->grid_ctas = coop && resident >= 1 ? std::min(sms, GRID_MAX_CTAS) : 0;
   CK(cudaMallocHost((void**)&V->hS, sizeof(Scalars)));
   CK(cudaMallocHost((void**)&V->hflag, sizeof(int)));
   TRY(dalloc(V, &q, 32)); V->fsc = (double*)q;
