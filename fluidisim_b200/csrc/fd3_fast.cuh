@@ -20,7 +20,9 @@ namespace fd3 {
 // apertures and six wet tests.  Apertures of cut faces and ghost coefficients are recomputed with
 // the reference's own expressions, so an encoded row evaluates to the same bits.
 constexpr unsigned RC_WET = 1u;
+//   bit 14       a surface ghost's face has an aperture other than 1
 constexpr unsigned RC_UNIT = 1u << 13;
+constexpr unsigned RC_CUT_GHOST = 1u << 14;
 
 __device__ __forceinline__ unsigned face_state(unsigned code, int f) { return (code >> (1 + 2 * f)) & 3u; }
 
@@ -33,11 +35,11 @@ __device__ __forceinline__ unsigned row_code_of(const RowE (&row)[6]) {
     unsigned st = row[f].n >= 0 ? 1u : (row[f].a > 0.f ? 2u : 0u);
     code |= st << (1 + 2 * f);
     if (st && row[f].a != 1.f) unit = false;
+    if (st == 2u && row[f].a != 1.f) code |= RC_CUT_GHOST;
   }
   if (unit) code |= RC_UNIT;
   return code;
 }
-
 
 // 1/max(theta, 1e-3) of ghost_side3 and ghost_up3 (delta3d_mobile.rs:126-147).
 __device__ __forceinline__ float ghost_it_side(const Geo& g, int i, int j, int k, int x, int y) {
@@ -65,10 +67,73 @@ constexpr unsigned RC_GHOSTS = (2u << 1) | (2u << 3) | (2u << 5) | (2u << 7) | (
 // the bits of the reference's sum over the live faces in the same order.
 __device__ __forceinline__ bool rc_plain(unsigned code) { return (code & (RC_UNIT | RC_GHOSTS)) == RC_UNIT; }
 
+// A row that is not plain, given the six neighbours' values (used only on a face onto a fluid neighbour):
+// apply_mobile3's terms a (pc - x) and (a pc) it, the lid's (2 a) pc, in its face order.  From its record
+// (Geo::rec) the row is two loads and a sum with selects: a kept ghost's a is 1, so (a pc) it is pc it, and a
+// missing face adds +0 (rc_plain).  Rebuilt face by face, a surface row is up to five chains of dependent
+// loads and two divisions in series, and nearly every chunk under a wavy surface, or at an obstacle, waits for a
+// warp with such rows: whole 128^3 basin projections 3.11 ms rebuilt, 2.81 from records (2.92 with the ghosts
+// alone kept, per column; 3.16 rebuilt with all divisions side by side), 256^3 waves 10.3 and 9.8 ms.
+__device__ __forceinline__ bool rec_kept(const Geo& g, unsigned code) { return g.rec && !(code & RC_CUT_GHOST); }
+__device__ __forceinline__ void rec_store(const Geo& g, int c, const float (&w)[6]) {
+  float4* R = g.rec + 2 * (size_t)c;
+  R[0] = make_float4(w[0], w[1], w[2], w[3]);
+  R[1] = make_float4(w[4], w[5], 0.f, 0.f);
+}
+__device__ __forceinline__ float row_general(const Geo& g, unsigned code, int i, int j, int k, float pc, float xm,
+                                             float xp, float ym, float yp, float zm, float zp) {
+  float acc = 0.f;
+  if (rec_kept(g, code)) {
+    const float4* R = g.rec + 2 * (size_t)((k * g.ny + j) * g.nx + i);
+    const float4 a = __ldg(R);
+    const float2 b = __ldg(reinterpret_cast<const float2*>(R + 1));
+    const float w[6] = {a.x, a.y, a.z, a.w, b.x, b.y}, v[6] = {xm, xp, ym, yp, zm, zp};
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      const unsigned st = face_state(code, f);
+      acc += st == 1u ? w[f] * (pc - v[f]) : (st == 2u ? pc * w[f] : 0.f);
+    }
+    return acc * g.inv;
+  }
+  const bool unit = code & RC_UNIT;
+  unsigned st = face_state(code, 0);
+  if (st) {
+    float a = unit ? 1.f : aper3(g, 0, fu(g, i, j, k));
+    if (st == 1) acc += a * (pc - xm); else acc += a * pc * ghost_it_side(g, i, j, k, i - 1, j);
+  }
+  st = face_state(code, 1);
+  if (st) {
+    float a = unit ? 1.f : aper3(g, 0, fu(g, i + 1, j, k));
+    if (st == 1) acc += a * (pc - xp); else acc += a * pc * ghost_it_side(g, i, j, k, i + 1, j);
+  }
+  st = face_state(code, 2);
+  if (st) {
+    float a = unit ? 1.f : aper3(g, 1, fv(g, i, j, k));
+    if (st == 1) acc += a * (pc - ym); else acc += a * pc * ghost_it_side(g, i, j, k, i, j - 1);
+  }
+  st = face_state(code, 3);
+  if (st) {
+    float a = unit ? 1.f : aper3(g, 1, fv(g, i, j + 1, k));
+    if (st == 1) acc += a * (pc - yp); else acc += a * pc * ghost_it_side(g, i, j, k, i, j + 1);
+  }
+  st = face_state(code, 4);  // the face below is never a ghost
+  if (st) {
+    float a = unit ? 1.f : aper3(g, 2, fw(g, i, j, k));
+    acc += a * (pc - zm);
+  }
+  st = face_state(code, 5);
+  if (st) {
+    float a = unit ? 1.f : aper3(g, 2, fw(g, i, j, k + 1));
+    if (st == 1) acc += a * (pc - zp);
+    else if (g.linear) acc += 2.f * a * pc;  // the lid of apply / apply_cut (delta3d.rs:741, 797)
+    else acc += a * pc * ghost_it_up(g, i, j, k);
+  }
+  return acc * g.inv;
+}
+
 template <class P>
 __device__ __forceinline__ float apply_code(const Geo& g, unsigned code, int i, int j, int k, int c, P p) {
   const float pc = p(c);
-  const bool unit = code & RC_UNIT;
   const int nxny = g.nx * g.ny;
   float acc = 0.f;
   if (rc_plain(code)) {  // a = 1 on every live face, no ghost: the masked sum, without the decoding
@@ -80,39 +145,10 @@ __device__ __forceinline__ float apply_code(const Geo& g, unsigned code, int i, 
     acc += (code & (1u << 11)) ? pc - p(c + nxny) : 0.f;
     return acc * g.inv;
   }
-  unsigned st = face_state(code, 0);
-  if (st) {
-    float a = unit ? 1.f : aper3(g, 0, fu(g, i, j, k));
-    if (st == 1) acc += a * (pc - p(c - 1)); else acc += a * pc * ghost_it_side(g, i, j, k, i - 1, j);
-  }
-  st = face_state(code, 1);
-  if (st) {
-    float a = unit ? 1.f : aper3(g, 0, fu(g, i + 1, j, k));
-    if (st == 1) acc += a * (pc - p(c + 1)); else acc += a * pc * ghost_it_side(g, i, j, k, i + 1, j);
-  }
-  st = face_state(code, 2);
-  if (st) {
-    float a = unit ? 1.f : aper3(g, 1, fv(g, i, j, k));
-    if (st == 1) acc += a * (pc - p(c - g.nx)); else acc += a * pc * ghost_it_side(g, i, j, k, i, j - 1);
-  }
-  st = face_state(code, 3);
-  if (st) {
-    float a = unit ? 1.f : aper3(g, 1, fv(g, i, j + 1, k));
-    if (st == 1) acc += a * (pc - p(c + g.nx)); else acc += a * pc * ghost_it_side(g, i, j, k, i, j + 1);
-  }
-  st = face_state(code, 4);  // the face below is never a ghost
-  if (st) {
-    float a = unit ? 1.f : aper3(g, 2, fw(g, i, j, k));
-    acc += a * (pc - p(c - nxny));
-  }
-  st = face_state(code, 5);
-  if (st) {
-    float a = unit ? 1.f : aper3(g, 2, fw(g, i, j, k + 1));
-    if (st == 1) acc += a * (pc - p(c + nxny));
-    else if (g.linear) acc += 2.f * a * pc;  // the lid of apply / apply_cut (delta3d.rs:741, 797)
-    else acc += a * pc * ghost_it_up(g, i, j, k);
-  }
-  return acc * g.inv;
+  return row_general(g, code, i, j, k, pc, face_state(code, 0) == 1u ? p(c - 1) : 0.f,
+                     face_state(code, 1) == 1u ? p(c + 1) : 0.f, face_state(code, 2) == 1u ? p(c - g.nx) : 0.f,
+                     face_state(code, 3) == 1u ? p(c + g.nx) : 0.f, face_state(code, 4) == 1u ? p(c - nxny) : 0.f,
+                     face_state(code, 5) == 1u ? p(c + nxny) : 0.f);
 }
 
 struct Load {
@@ -124,6 +160,44 @@ struct LoadT {
   const T* __restrict__ x;
   __device__ __forceinline__ float operator()(int n) const { return Store<T>::ld(x, n); }
 };
+
+// ------------------------------------------------------------------------------------------------
+// Geo::ztop from the surface: one CTA per 32 x 8 tile, one thread per column.  wet3's height test is
+// monotone in k, so a column's wet cells end where it first fails (solids below only make the bound loose).
+__global__ void __launch_bounds__(TILE_X * TILE_Y) k_tile_tops(Geo g, int* __restrict__ ztop) {
+  KSTART();
+  const int ntx = (g.nx + TILE_X - 1) / TILE_X;
+  const int i = (int)(blockIdx.x % ntx) * TILE_X + (int)threadIdx.x % TILE_X;
+  const int j = (int)(blockIdx.x / ntx) * TILE_Y + (int)threadIdx.x / TILE_X;
+  int top = 0;
+  if (i < g.nx && j < g.ny && col_active(g, i, j)) {
+    const float h = g.eta[j * g.nx + i];
+    int lo = 0, hi = g.nz;  // the first k in [0, nz] that is not below the surface
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (((float)mid + 0.5f) * g.dx < h) lo = mid + 1; else hi = mid;
+    }
+    top = lo;
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  __shared__ int warp[TILE_Y];
+  if (threadIdx.x % 32 == 0) warp[threadIdx.x / 32] = top;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < TILE_Y; ++w) top = max(top, warp[w]);
+    ztop[blockIdx.x] = (top + 1) & ~1;
+  }
+}
+// The same bound for a coarse level, 2^sh fine cells to a side of its cells: the cell (i, j, k) lies in
+// the air.  Only up to sh = 3, where a cell's columns lie in one tile (ztop is null above).
+struct Air {
+  const int* ztop;
+  int sh, ntx;
+};
+__device__ __forceinline__ bool in_air(const Air& a, int i, int j, int k) {
+  return a.ztop && (k << a.sh) >= a.ztop[((j << a.sh) / TILE_Y) * a.ntx + (i << a.sh) / TILE_X];
+}
 
 // ------------------------------------------------------------------------------------------------
 // The outer loop's metrics from the projection's row codes (the surface is the one the codes were
@@ -798,18 +872,26 @@ __global__ void k_level_prepare_a(Geo g, Lev F, Lev C, int fine) {
   if (fine) coarsen_open_at(g.nx, g.ny, g.ou, g.ov, g.ow, g.act, C, q);
   else coarsen_open_at(F.nx, F.ny, F.ou, F.ov, F.ow, nullptr, C, q);
 }
-__global__ void k_level_prepare_b(Lev C) {
+// An inactive cell's vectors are zeroed (Geo::ztop), in the storage they are kept in.
+__device__ __forceinline__ void level_zero_inactive(const Lev& C, int c, int half) {
+  if (C.kind[c] > 0.f) return;
+  for (float* f : {C.x, C.x2, C.r, C.t}) {
+    if (half) as<__half>(f)[c] = __float2half_rn(0.f); else f[c] = 0.f;
+  }
+}
+__global__ void k_level_prepare_b(Lev C, int half) {
   KSTART();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C.n) return;
   C.diag[c] = level_diag_at(C, c);
   C.code[c] = (unsigned short)level_codes_at(C, c);
+  level_zero_inactive(C, c, half);
 }
 // The same for levels first .. last (first >= 1, every one small) in one CTA: the kinds and
 // apertures level by level, a barrier after each, then every level's diagonal and codes.
 constexpr int PREP_SMALL_THREADS = 1024;
 __global__ void __launch_bounds__(PREP_SMALL_THREADS) k_levels_prepare_small(const Lev* __restrict__ levs, int first,
-                                                                          int last) {
+                                                                          int last, int half) {
   KSTART();
   for (int l = first; l <= last; ++l) {
     const Lev F = levs[l - 1], C = levs[l];
@@ -825,6 +907,7 @@ __global__ void __launch_bounds__(PREP_SMALL_THREADS) k_levels_prepare_small(con
     for (int c = threadIdx.x; c < C.n; c += blockDim.x) {
       C.diag[c] = level_diag_at(C, c);
       C.code[c] = (unsigned short)level_codes_at(C, c);
+      level_zero_inactive(C, c, half);
     }
   }
 }
@@ -943,7 +1026,7 @@ __device__ __forceinline__ void level_ijk(const Lev& L, int c, int& i, int& j, i
 
 // The two pre-sweeps of a coarse level from x = 0, written to L.x (smooth3 twice after fill(0)).
 template <class T, bool SPEC>
-__global__ void __launch_bounds__(TPB) k_level_pre(Lev L, const Scalars* S, int gate) {
+__global__ void __launch_bounds__(TPB) k_level_pre(Lev L, Air air, const Scalars* S, int gate) {
   KSTART();
   if (!SPEC && gate && !S->active) return;
   int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -952,6 +1035,7 @@ __global__ void __launch_bounds__(TPB) k_level_pre(Lev L, const Scalars* S, int 
   auto X1c = [&](int n, int, int, int) { return level_x1<T>(L, n); };
   int i, j, k;
   level_ijk(L, c, i, j, k);
+  if (in_air(air, i, j, k)) return;
   const unsigned code = L.code[c];
   const float dg = L.diag[c];
   const float rc = Store<T>::ld(as<T>(L.r), c);
@@ -969,7 +1053,7 @@ __global__ void __launch_bounds__(TPB) k_level_pre(Lev L, const Scalars* S, int 
 
 // t = r - L x on every cell of a coarse level (0 on inactive rows), the restriction's operand.
 template <class T, bool SPEC>
-__global__ void __launch_bounds__(TPB) k_level_resid(Lev L, const Scalars* S, int gate) {
+__global__ void __launch_bounds__(TPB) k_level_resid(Lev L, Air air, const Scalars* S, int gate) {
   KSTART();
   if (!SPEC && gate && !S->active) return;
   int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -978,6 +1062,7 @@ __global__ void __launch_bounds__(TPB) k_level_resid(Lev L, const Scalars* S, in
   auto Xc = [&](int n, int, int, int) { return X(n); };
   int i, j, k;
   level_ijk(L, c, i, j, k);
+  if (in_air(air, i, j, k)) return;
   const unsigned code = L.code[c];
   const float rc = Store<T>::ld(as<T>(L.r), c);
   const float pc = X(c);
@@ -995,11 +1080,12 @@ __global__ void __launch_bounds__(TPB) k_level_resid(Lev L, const Scalars* S, in
 
 // C.r = mean of the 8 children of F.t, in the reference's CHILDREN order (restrict3).
 template <class T>
-__global__ void __launch_bounds__(TPB) k_level_sum8(Lev F, Lev C, const Scalars* S, int gate) {
+__global__ void __launch_bounds__(TPB) k_level_sum8(Lev F, Lev C, Air air, const Scalars* S, int gate) {
   KSTART();
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= C.n) return;
   int ci = q % C.nx, t = q / C.nx, cj = t % C.ny, ck = t / C.ny;
+  if (in_air(air, ci, cj, ck)) return;
   float v[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
@@ -1018,12 +1104,14 @@ __global__ void __launch_bounds__(TPB) k_level_sum8(Lev F, Lev C, const Scalars*
 // CHILDREN order) each evaluate one child's t = r - L x, rounded through the storage type as the
 // stored t would be, and the first of them sums the eight in order (restrict3).
 template <class T, bool SPEC>
-__global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, const Scalars* S, int gate) {
+__global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, Air air, const Scalars* S, int gate) {
   KSTART();
   if (!SPEC && gate && !S->active) return;
   const int q8 = blockIdx.x * blockDim.x + threadIdx.x;
   const int q = q8 >> 3, e = q8 & 7;
-  const bool own = q < C.n;
+  bool own = q < C.n;
+  if (own) own = !in_air(air, q % C.nx, q / C.nx % C.ny, q / (C.nx * C.ny));
+  if (!__any_sync(0xffffffffu, own)) return;
   float tv = 0.f;
   unsigned code = 0u;
   int i = 0, j = 0, k = 0, c = 0;
@@ -1060,7 +1148,7 @@ __global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, const Sca
 
 // Prolongation from C (x += parent) fused with the first post-sweep, L.x -> L.x2.
 template <class T, bool SPEC>
-__global__ void __launch_bounds__(TPB) k_level_post1(Lev L, Lev C, const Scalars* S, int gate) {
+__global__ void __launch_bounds__(TPB) k_level_post1(Lev L, Lev C, Air air, const Scalars* S, int gate) {
   KSTART();
   if (!SPEC && gate && !S->active) return;
   int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1075,6 +1163,7 @@ __global__ void __launch_bounds__(TPB) k_level_post1(Lev L, Lev C, const Scalars
   };
   int i, j, k;
   level_ijk(L, c, i, j, k);
+  if (in_air(air, i, j, k)) return;
   const unsigned code = L.code[c];
   const float dg = L.diag[c];
   const float rc = Store<T>::ld(as<T>(L.r), c);
@@ -1092,7 +1181,7 @@ __global__ void __launch_bounds__(TPB) k_level_post1(Lev L, Lev C, const Scalars
 
 // The second post-sweep, L.x2 -> L.x.
 template <class T, bool SPEC>
-__global__ void __launch_bounds__(TPB) k_level_post2(Lev L, const Scalars* S, int gate) {
+__global__ void __launch_bounds__(TPB) k_level_post2(Lev L, Air air, const Scalars* S, int gate) {
   KSTART();
   if (!SPEC && gate && !S->active) return;
   int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1101,6 +1190,7 @@ __global__ void __launch_bounds__(TPB) k_level_post2(Lev L, const Scalars* S, in
   auto Xc = [&](int n, int, int, int) { return X(n); };
   int i, j, k;
   level_ijk(L, c, i, j, k);
+  if (in_air(air, i, j, k)) return;
   const unsigned code = L.code[c];
   const float dg = L.diag[c];
   const float rc = Store<T>::ld(as<T>(L.r), c);
@@ -1123,12 +1213,14 @@ __global__ void __launch_bounds__(TPB) k_level_post2(Lev L, const Scalars* S, in
 // C.x would be; the warp shares the seven values; each child then sweeps its own row with
 // k_level_post1's expression.  C.x is never stored: only this pass would read it.
 template <class T>
-__global__ void __launch_bounds__(TPB) k_level_post21(Lev L, Lev C, const Scalars* S, int gate) {
+__global__ void __launch_bounds__(TPB) k_level_post21(Lev L, Lev C, Air air, const Scalars* S, int gate) {
   KSTART();
   const int q8 = blockIdx.x * blockDim.x + threadIdx.x;
   const int q = q8 >> 3, e = q8 & 7;
-  const bool own = q < C.n;
+  bool own = q < C.n;
   const int ci = own ? q % C.nx : 0, cj = own ? (q / C.nx) % C.ny : 0, ck = own ? q / (C.nx * C.ny) : 0;
+  if (own) own = !in_air(air, ci, cj, ck);
+  if (!__any_sync(0xffffffffu, own)) return;
   // the C cell this lane sweeps: 0 the parent, 1..6 its x-, x+, y-, y+, z-, z+ neighbours
   int pi = ci, pj = cj, pk = ck;
   if (e == 1) pi -= 1; else if (e == 2) pi += 1; else if (e == 3) pj -= 1;
@@ -1566,9 +1658,23 @@ __device__ __forceinline__ float rhs_b2_at(const Geo& g, float scale, float* __r
   }
   rhs[c] = b;
   prec[c] = diag > 0.f ? 1.f / (diag * g.inv) : 0.f;
-  if (codes) codes[c] = (unsigned short)row_code_of(row);
+  if (codes) {
+    const unsigned code = row_code_of(row);
+    codes[c] = (unsigned short)code;
+    if (rec_kept(g, code) && !rc_plain(code)) {
+      float w[6];
+#pragma unroll
+      for (int f = 0; f < 6; ++f) w[f] = row[f].n >= 0 ? row[f].a : row[f].it;
+      rec_store(g, c, w);
+    }
+  }
   return b;
 }
+
+// The loop's r, d (two buffers) and q: zeroed where there is no row (Geo::ztop).  Null: left alone.
+struct WorkVectors {
+  float* v[4];
+};
 
 // rhs_mobile3 (delta3d_mobile.rs:215-241) with b.b (FIN_B2) when `reduce`.
 // With `codes` not null, the same pass also writes each cell's row code (row_code_of the same
@@ -1576,10 +1682,14 @@ __device__ __forceinline__ float rhs_b2_at(const Geo& g, float scale, float* __r
 template <int MODE>
 __global__ void __launch_bounds__(TPB, FD3_SETUP_MINB) k_rhs_b2(Geo g, float scale, float* __restrict__ rhs, float* __restrict__ prec,
                                                 Red red, Scalars* S, int reduce, unsigned short* __restrict__ codes,
-                                                float* __restrict__ pdry) {
+                                                float* __restrict__ pdry, WorkVectors work) {
   KSTART();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   const float b = c < g.n ? rhs_b2_at(g, scale, rhs, prec, codes, pdry, c) : 0.f;
+  if (work.v[0] && c < g.n && prec[c] == 0.f) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) work.v[q][c] = 0.f;
+  }
   if (!reduce) return;
   if (__syncthreads_or(c < g.n && b != 0.f) && threadIdx.x == 0) atomicOr(&S->any_nonzero, 1);
   reduce_finish<MODE>(Acc<MODE>::prod(b, b), c, g.n, red, S, FIN_B2);

@@ -69,6 +69,15 @@ struct Geo {
   // projection writes is 0 there (the set change zeroes them), and a skipped tile adds exactly 0 to
   // each reduction, so skipping changes no bit.
   const unsigned char* tiles;
+  // per 32 x 8 tile of columns, the layers from the bottom up to the tile's highest wet cell, rounded up to
+  // even (k_tile_tops; null: every layer).  The air above holds no row: during a projection the blocked
+  // fine kernels and the level kernels leave it alone.  The assembly zeroes p and the loop's work vectors in
+  // every dry cell and the level vectors in every inactive coarse cell, so what the passes would have
+  // written there is there already, and a skipped cell adds exactly 0 to each reduction.
+  const int* ztop;
+  // eight floats per cell, written with the row codes for the rows that are not plain (null: not kept):
+  // per face its aperture onto a fluid neighbour, or the ghost's 1/theta (the lid: twice the aperture).
+  float4* rec;
   // A solid set in motion by set_solid_rigid: wall = 1 in translation, 2 in rotation, 0 at rest or
   // without a solid.  The divergence then adds the flux of the parts of the faces the solid covers
   // (base apertures bou/bov/bow, the bottom-only cut, minus the apertures).
@@ -79,6 +88,14 @@ struct Geo {
   const float* bow;
 };
 constexpr int TILE_X = 32, TILE_Y = 8;
+
+// The layers to process of the columns [x0, x0 + 64) x [y0, y0 + 8) (two tiles), and of one column.
+__device__ __forceinline__ int tops64(const Geo& g, int x0, int y0) {
+  if (!g.ztop) return g.nz;
+  const int ntx = (g.nx + TILE_X - 1) / TILE_X, a = x0 / TILE_X, row = (y0 / TILE_Y) * ntx;
+  const int t0 = g.ztop[row + a], t1 = a + 1 < ntx ? g.ztop[row + a + 1] : 0;
+  return min(max(t0, t1), g.nz);
+}
 
 // A coarse level (Level3, delta3d_multigrid.rs:37-52).
 struct Lev {

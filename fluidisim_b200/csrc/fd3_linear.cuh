@@ -40,6 +40,12 @@ __global__ void k_row_codes_linear(Geo g, unsigned short* __restrict__ codes) {
       if (st && a[f] != 1.f) unit = false;
     }
     if (unit) code |= RC_UNIT;
+    if (rec_kept(g, code) && !rc_plain(code)) {
+      float w[6];
+#pragma unroll
+      for (int f = 0; f < 6; ++f) w[f] = face_state(code, f) == 2u ? 2.f * a[f] : a[f];
+      rec_store(g, c, w);
+    }
   }
   codes[c] = (unsigned short)code;
 }

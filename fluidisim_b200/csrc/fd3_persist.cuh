@@ -123,11 +123,10 @@ __global__ void k_grid_reset(GridSlots* slots) {
   slots->arrived = 0u;
 }
 
-// A cell's row kept on chip: per face the aperture onto a fluid neighbour, or the ghost's 1/theta (the
-// lid: twice the aperture), evaluated as apply_code does, a (pc - x) and (a pc) it.  ROW_CUT_GHOST marks the
-// rare row with a ghost face whose aperture is not 1, which reads that aperture again.
-constexpr unsigned ROW_CUT_GHOST = 1u << 14;
-__device__ __forceinline__ unsigned kept_row(const Geo& g, unsigned code, int i, int j, int k, float (&w)[6]) {
+// A cell's row kept on chip, as Geo::rec keeps it: per face the aperture onto a fluid neighbour, or the ghost's
+// 1/theta (the lid: twice the aperture).  A ghost face with an aperture other than 1 (RC_CUT_GHOST) reads that
+// aperture again.
+__device__ __forceinline__ void kept_row(const Geo& g, unsigned code, int i, int j, int k, float (&w)[6]) {
   const bool unit = code & RC_UNIT;
   const int axis[6] = {0, 0, 1, 1, 2, 2};
   const int fi[6] = {fu(g, i, j, k), fu(g, i + 1, j, k), fv(g, i, j, k), fv(g, i, j + 1, k), fw(g, i, j, k),
@@ -138,15 +137,13 @@ __device__ __forceinline__ unsigned kept_row(const Geo& g, unsigned code, int i,
     const unsigned st = face_state(code, f);
     w[f] = 0.f;
     if (!st) continue;
-    const float a = unit ? 1.f : aper3(g, axis[f], fi[f]);
-    if (st == 1) w[f] = a;
-    else if (f == 5 && g.linear) w[f] = 2.f * a;
-    else {
+    if (st == 1 || g.linear) {
+      const float a = unit ? 1.f : aper3(g, axis[f], fi[f]);
+      w[f] = st == 1 ? a : 2.f * a;
+    } else {
       w[f] = f == 5 ? ghost_it_up(g, i, j, k) : ghost_it_side(g, i, j, k, xs[f < 4 ? f : 0], ys[f < 4 ? f : 0]);
-      if (a != 1.f) code |= ROW_CUT_GHOST;
     }
   }
-  return code;
 }
 __device__ __noinline__ float face_aperture(const Geo& g, int c, int f) {
   int i, j, k;
@@ -164,7 +161,7 @@ __device__ __forceinline__ float apply_kept(const Geo& g, unsigned code, int c, 
   for (int f = 0; f < 6; ++f) {
     const unsigned st = face_state(code, f);
     float ghost = pc * w(f);
-    if ((code & ROW_CUT_GHOST) && st == 2u && !(f == 5 && g.linear)) ghost = face_aperture(g, c, f) * pc * w(f);
+    if ((code & RC_CUT_GHOST) && st == 2u) ghost = face_aperture(g, c, f) * pc * w(f);
     acc += st == 1u ? w(f) * (pc - v[f]) : (st == 2u ? ghost : 0.f);
   }
   return acc * g.inv;
@@ -207,7 +204,8 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
         int i, j, k;
         cell_ijk(g, c, i, j, k);
         float w[6];
-        code[s] = kept_row(g, rc16, i, j, k, w);
+        code[s] = rc16;
+        kept_row(g, rc16, i, j, k, w);
 #pragma unroll
         for (int f = 0; f < 6; ++f) K(s, f) = w[f];
       }

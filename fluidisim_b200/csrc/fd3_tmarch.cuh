@@ -198,14 +198,14 @@ __global__ void __launch_bounds__(TQ<Q>::NT, MINB)
   int b = blockIdx.x;
   const int bx = b % ntx; b /= ntx;
   const int by = b % nty; b /= nty;
-  const int x0 = bx * TMX, y0 = by * TMY, k0 = b * K, k1 = min(k0 + K, g.nz);
+  const int x0 = bx * TMX, y0 = by * TMY, k0 = b * K, k1 = min(min(k0 + K, g.nz), tops64(g, x0, y0));
   const int i0 = x0 + Q * tx, j = y0 + ty;
   const bool inside = i0 < g.nx && j < g.ny;  // nx % 8 == 0: the thread's Q cells are all inside or all out
   double acc = 0.0;
-  bool skip = false;
+  bool skip = k0 >= k1;  // the chunk lies in the air
   if (g.tiles) {  // a 64 x 8 tile is two 32 x 8 tiles of the set's tile flags
     const int ntt = (g.nx + TILE_X - 1) / TILE_X, row = (y0 / TILE_Y) * ntt, t0 = x0 / TILE_X;
-    skip = !g.tiles[row + t0] && (t0 + 1 >= ntt || !g.tiles[row + t0 + 1]);  // no column of the set
+    skip = skip || (!g.tiles[row + t0] && (t0 + 1 >= ntt || !g.tiles[row + t0 + 1]));  // no column of the set
   }
   if (!skip) {
     const int dmode = PASS == TP_DIR ? S->dir_mode : 0;

@@ -83,6 +83,10 @@ struct ScopedDevice {
 #endif
 constexpr int SPEC_MAX_CELLS = FD3_SPEC_MAX;
 
+// Volumes of at most this many cells keep their rows (Geo::rec, 32 bytes per cell: 4.3 GB here); larger ones
+// rebuild them, so that the largest volume a GPU holds stays what it was.
+constexpr int kRecMaxCells = 1 << 27;
+
 // Volumes from this many cells run the four-cells-per-thread fine kernels by default (kernels = 0).
 constexpr long long kQuadMinCells = 1LL << 23;
 
@@ -113,6 +117,7 @@ struct fd3_volume {
   float *us = nullptr, *vs = nullptr, *ws = nullptr, *p = nullptr, *rhs = nullptr, *res = nullptr;
   float *dir = nullptr, *dir2 = nullptr, *tmp = nullptr, *prec = nullptr;
   unsigned short* codes = nullptr;  // row codes of the current projection
+  float4* rec = nullptr;            // its rows that are not plain (Geo::rec); none above kRecMaxCells
   float *sv_u = nullptr, *sv_v = nullptr, *sv_w = nullptr, *sv_p = nullptr, *sv_eta = nullptr, *sv_rof = nullptr;
   float *flux_x = nullptr, *flux_y = nullptr;
   // a volume configured with a solid: its node SDF buffer and the bottom-only base geometry the
@@ -129,6 +134,8 @@ struct fd3_volume {
   bool sparse = false;
   unsigned char *act = nullptr, *act_next = nullptr;
   std::vector<unsigned char> hact;
+  int* ztop = nullptr;       // per 32 x 8 tile of columns: the layers below its highest wet cell (Geo::ztop)
+  bool skip_air = false;     // project_mobile3 is running with ztop and the zeroed dry cells of its assembly
   unsigned char* tiles = nullptr;  // per 32 x 8 tile of columns: any column in the set (Geo::tiles)
   // multigrid
   bool has_mg = false;
@@ -201,6 +208,8 @@ struct fd3_volume {
     G.frac = frac; G.ou = ou; G.ov = ov; G.ow = ow;
     G.act = sparse ? act : nullptr;
     G.tiles = sparse && !opt.no_tile_skip ? tiles : nullptr;
+    G.ztop = skip_air ? ztop : nullptr;
+    G.rec = rec;
     G.wall = wall;
     G.rig = motion;
     G.bou = bou; G.bov = bov; G.bow = bow;
@@ -240,7 +249,7 @@ struct fd3_volume {
   int loop_key() const {
     return (ord() ? 1 : 0) | (mg_on() ? 2 : 0) | (blocked() ? 4 : 0) | (opt.no_overlap ? 8 : 0) | (linear ? 16 : 0) |
            (paired() ? 32 : 0) | (half() ? 64 : 0) | (sparse ? 128 : 0) |  // the captured Geo holds the set's mask
-           (opt.no_tile_skip ? 256 : 0) | (quad() ? 512 : 0) | (tmaf() ? 1024 : 0);
+           (opt.no_tile_skip ? 256 : 0) | (skip_air ? 2048 : 0) | (quad() ? 512 : 0) | (tmaf() ? 1024 : 0);
   }
   Red red() const { return Red{p64, p32, count}; }
 };
@@ -369,13 +378,13 @@ void prepare_multigrid(fd3_volume* V) {
   for (int l = 0; l < nl; ++l) {
     const Lev& C = V->levels[l];
     if (l > 0 && C.n <= PREP_SMALL_CELLS) {
-      LAUNCH_G(V, k_levels_prepare_small, 1, PREP_SMALL_THREADS, (const Lev*)V->dlev, l, nl - 1);
+      LAUNCH_G(V, k_levels_prepare_small, 1, PREP_SMALL_THREADS, (const Lev*)V->dlev, l, nl - 1, V->half() ? 1 : 0);
       return;
     }
     const long long nfaces = (long long)(C.nx + 1) * C.ny * C.nz + (long long)C.nx * (C.ny + 1) * C.nz +
                              (long long)C.nx * C.ny * (C.nz + 1);
     LAUNCH(V, k_level_prepare_a, C.n + nfaces, G, l > 0 ? V->levels[l - 1] : Lev{}, C, l == 0 ? 1 : 0);
-    LAUNCH(V, k_level_prepare_b, C.n, C);
+    LAUNCH(V, k_level_prepare_b, C.n, C, V->half() ? 1 : 0);
   }
 }
 
@@ -390,6 +399,7 @@ void coarse_cycle_t(fd3_volume* V, int gate) {
   const bool half = Store<T>::half;
   const int first_tail = (half && !V->tail_reg) ? (int)Ls.size() : V->tail_first;
   const Scalars* S = V->dS;
+  auto air = [&](int l) { return Air{V->skip_air && l < 3 ? V->ztop : nullptr, l + 1, (V->nx + TILE_X - 1) / TILE_X}; };
   for (int l = 0; l < first_tail && l <= last; ++l) {
     Lev& L = Ls[l];
     if (l == last) {  // a large coarsest level: its 8 sweeps one by one
@@ -399,12 +409,12 @@ void coarse_cycle_t(fd3_volume* V, int gate) {
     } else {
       const long long n8 = 8LL * Ls[l + 1].n;  // one thread per child of each next-level cell
       if (L.n <= SPEC_MAX_CELLS) {
-        launch_grid(V, "k_level_pre", blocks_for(L.n), TPB, k_level_pre<T, true>, L, S, gate);
-        launch_grid(V, "k_level_restrict8", blocks_for(n8), TPB, k_level_restrict8<T, true>, L, Ls[l + 1], S, gate);
+        launch_grid(V, "k_level_pre", blocks_for(L.n), TPB, k_level_pre<T, true>, L, air(l), S, gate);
+        launch_grid(V, "k_level_restrict8", blocks_for(n8), TPB, k_level_restrict8<T, true>, L, Ls[l + 1], air(l + 1), S, gate);
       } else {
-        launch_grid(V, "k_level_pre", blocks_for(L.n), TPB, k_level_pre<T, false>, L, S, gate);
-        launch_grid(V, "k_level_resid", blocks_for(L.n), TPB, k_level_resid<T, false>, L, S, gate);
-        LAUNCH(V, k_level_sum8<T>, Ls[l + 1].n, L, Ls[l + 1], S, gate);
+        launch_grid(V, "k_level_pre", blocks_for(L.n), TPB, k_level_pre<T, false>, L, air(l), S, gate);
+        launch_grid(V, "k_level_resid", blocks_for(L.n), TPB, k_level_resid<T, false>, L, air(l), S, gate);
+        LAUNCH(V, k_level_sum8<T>, Ls[l + 1].n, L, Ls[l + 1], air(l + 1), S, gate);
       }
     }
   }
@@ -427,15 +437,15 @@ void coarse_cycle_t(fd3_volume* V, int gate) {
   for (int l = top; l >= 0; --l) {
     if (Ls[l].n <= SPEC_MAX_CELLS) {
       if (fused(l))
-        launch_grid(V, "k_level_post21", blocks_for(8LL * Ls[l + 1].n), TPB, k_level_post21<T>, Ls[l], Ls[l + 1], S,
+        launch_grid(V, "k_level_post21", blocks_for(8LL * Ls[l + 1].n), TPB, k_level_post21<T>, Ls[l], Ls[l + 1], air(l + 1), S,
                     gate);
       else
-        launch_grid(V, "k_level_post1", blocks_for(Ls[l].n), TPB, k_level_post1<T, true>, Ls[l], Ls[l + 1], S, gate);
+        launch_grid(V, "k_level_post1", blocks_for(Ls[l].n), TPB, k_level_post1<T, true>, Ls[l], Ls[l + 1], air(l), S, gate);
       if (!fused(l - 1))
-        launch_grid(V, "k_level_post2", blocks_for(Ls[l].n), TPB, k_level_post2<T, true>, Ls[l], S, gate);
+        launch_grid(V, "k_level_post2", blocks_for(Ls[l].n), TPB, k_level_post2<T, true>, Ls[l], air(l), S, gate);
     } else {
-      launch_grid(V, "k_level_post1", blocks_for(Ls[l].n), TPB, k_level_post1<T, false>, Ls[l], Ls[l + 1], S, gate);
-      launch_grid(V, "k_level_post2", blocks_for(Ls[l].n), TPB, k_level_post2<T, false>, Ls[l], S, gate);
+      launch_grid(V, "k_level_post1", blocks_for(Ls[l].n), TPB, k_level_post1<T, false>, Ls[l], Ls[l + 1], air(l), S, gate);
+      launch_grid(V, "k_level_post2", blocks_for(Ls[l].n), TPB, k_level_post2<T, false>, Ls[l], air(l), S, gate);
     }
   }
 }
@@ -723,6 +733,18 @@ void prime(fd3_volume* V) {
   }
 }
 
+// The update of the loops on the paired march and the TMA-staged passes (the same tiles).
+void paired_update(fd3_volume* V, const float* d) {
+  const int k2 = pick_k2(V->nx, V->ny, V->nz);
+  const int zb = zblocks2(V->nx, V->ny, V->nz, k2);
+  if (k2 == 8)
+    launch_grid(V, "kx_update_rn", zb, Z2T, kx_update_rn<8>, V->geo(), V->p, V->res, d, (const float*)V->tmp,
+                V->red(), V->dS);
+  else
+    launch_grid(V, "kx_update_rn", zb, Z2T, kx_update_rn<4>, V->geo(), V->p, V->res, d, (const float*)V->tmp,
+                V->red(), V->dS);
+}
+
 // One inner PCG iteration (delta3d_mobile.rs:515-545), every kernel gated on S->active.  With the
 // multigrid, the direction alternates between dir and dir2 (parity) because it is recomputed at
 // the stencil points of the operator.
@@ -733,8 +755,7 @@ void iteration(fd3_volume* V, int parity) {
     float* dout = parity ? V->dir : V->dir2;
     if (V->tmaf() && tma_ready(V)) {
       tma_dir(V, parity);
-      LAUNCH_G(V, kv_update_rn, update_blocks(V->n), TPB, V->n, V->p, V->res, (const float*)dout,
-               (const float*)V->tmp, V->red(), V->dS, update_mask(V), V->ncol);
+      paired_update(V, dout);
     } else if (V->quad()) {
       quad_dispatch(V, [&](auto qx, auto k4) {
         constexpr int QX = decltype(qx)::value, K4 = decltype(k4)::value;
@@ -765,8 +786,7 @@ void iteration(fd3_volume* V, int parity) {
           launch_grid(V, "kx_dir_apply_dot<4>", zb, Z2T, kx_dir_apply_dot<4, float>, G, codes, z, (const float*)din,
                       dout, V->tmp, V->red(), V->dS);
       }
-      LAUNCH_G(V, kv_update_rn, update_blocks(V->n), TPB, V->n, V->p, V->res, (const float*)dout,
-               (const float*)V->tmp, V->red(), V->dS, update_mask(V), V->ncol);
+      paired_update(V, dout);
     } else if (V->blocked()) {
       if (zfull(V->nx, V->ny, V->nz))
         LAUNCH_G(V, kz_dir_apply_dot<true>, zblocks(V->nx, V->ny, V->nz), ZT, G, (const unsigned short*)V->codes,
@@ -1003,7 +1023,7 @@ float vscale_k(const fd3_volume* V) {
 
 // project_mobile3 (delta3d_mobile.rs:465-609), or, with V->linear, project (delta3d.rs:1060-1196):
 // the same loop and outer logic on the linear rows, CG or Jacobi-PCG, from p = 0 everywhere.
-int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_report* rep) {
+int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_report* rep) {
   const bool ord = V->ord();
   Geo G = V->geo();
   LAUNCH_G(V, k_reset_scalars, 1, 1, V->dS, vscale_k(V));
@@ -1015,7 +1035,11 @@ int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd
     CK(cudaMemsetAsync(V->p, 0, (size_t)V->n * sizeof(float), V->stream));
   } else {
     // the assembly also zeroes p on the dry cells (delta3d_mobile.rs:486-495)
-    DISPATCH(V, k_rhs_b2, V->n, G, scale, V->rhs, V->prec, V->red(), V->dS, 1, V->codes, V->p);
+    DISPATCH(V, k_rhs_b2, V->n, G, scale, V->rhs, V->prec, V->red(), V->dS, 1, V->codes, V->p,
+             V->skip_air ? WorkVectors{{V->res, V->dir, V->dir2, V->tmp}} : WorkVectors{});
+    if (V->skip_air)
+      LAUNCH_G(V, k_tile_tops, ((V->nx + TILE_X - 1) / TILE_X) * ((V->ny + TILE_Y - 1) / TILE_Y), TILE_X * TILE_Y, G,
+               V->ztop);
     if (V->has_mg) prepare_multigrid(V);
   }
   residual(V, (int)FIN_RR0);
@@ -1148,6 +1172,15 @@ int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd
   rep->backward_error = (double)ck.be;
   rep->divergence_plain = div_plain;
   return FD3_OK;
+}
+
+// With f64 reductions, an even nx and the multigrid, the passes leave the air above the surface alone
+// (Geo::ztop); fd3_options.no_tile_skip switches that off with the tiles'.
+int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_report* rep) {
+  V->skip_air = V->mg_on() && V->paired() && !V->opt.no_tile_skip;
+  const int e = project_rows(V, scale, k1, max_iters, rep);
+  V->skip_air = false;
+  return e;
 }
 
 // ---------------------------------------------------------------------------- input validation
@@ -1311,6 +1344,10 @@ int alloc_state(fd3_volume* V) {
   float* cq;
   TRY(dalloc(V, &cq, (size_t)(V->n + 1) / 2)); V->codes = (unsigned short*)cq;
   TRY(dalloc(V, &cq, 4)); V->count = (unsigned*)cq;
+  if (V->n <= kRecMaxCells) {
+    TRY(dalloc(V, &cq, (size_t)V->n * 8));
+    V->rec = (float4*)cq;
+  }
   TRY(dalloc(V, &V->sv_u, V->nu)); TRY(dalloc(V, &V->sv_v, V->nv)); TRY(dalloc(V, &V->sv_w, V->nw));
   TRY(dalloc(V, &V->sv_p, V->n)); TRY(dalloc(V, &V->sv_eta, V->ncol)); TRY(dalloc(V, &V->sv_rof, V->ncol));
   TRY(dalloc(V, &V->flux_x, (size_t)(V->nx + 1) * V->ny)); TRY(dalloc(V, &V->flux_y, (size_t)V->nx * (V->ny + 1)));
@@ -1323,6 +1360,7 @@ int alloc_state(fd3_volume* V) {
   TRY(dalloc(V, &V->p32, (size_t)(V->n + CHUNK - 1) / CHUNK + 64));
   TRY(dalloc(V, &q, sizeof(Scalars) / sizeof(float) + 16)); V->dS = (Scalars*)q;
   TRY(dalloc(V, &q, 16)); V->dflag = (int*)q;
+  TRY(dalloc(V, &q, (size_t)((V->nx + TILE_X - 1) / TILE_X) * ((V->ny + TILE_Y - 1) / TILE_Y))); V->ztop = (int*)q;
   TRY(dalloc(V, &q, (sizeof(GridSlots) + 3) / 4)); V->slots = (GridSlots*)q;
   int sms = 0, coop = 0, resident = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, V->device));
@@ -2480,7 +2518,7 @@ int fd3_assemble_pressure_problem_for_trials(fd3_volume* V, const float* diverge
   if (!ok) return FD3_ERR_NOT_FINITE;
   CK(cudaMemcpyAsync(V->rhs, V->tmp, len * 4, cudaMemcpyDeviceToDevice, V->stream));
   DISPATCH(V, k_rhs_b2, V->n, V->geo(), scale, V->rhs, V->prec, V->red(), V->dS, 0, (unsigned short*)nullptr,
-           (float*)nullptr);
+           (float*)nullptr, WorkVectors{});
   CK(cudaMemcpyAsync(rhs, V->rhs, len * 4, cudaMemcpyDeviceToHost, V->stream));
   CK(cudaMemcpyAsync(prec, V->prec, len * 4, cudaMemcpyDeviceToHost, V->stream));
   return sync(V);
@@ -2492,7 +2530,8 @@ int fd3_vcycle_for_tests(fd3_volume* V, const float* x, float* z, size_t len) {
   if (!V->has_mg) return FD3_ERR_DOMAIN;
   if (len != (size_t)V->n) return FD3_ERR_SHAPE;
   CK(cudaMemsetAsync(V->rhs, 0, len * 4, V->stream));
-  DISPATCH(V, k_rhs_b2, V->n, V->geo(), 1.f, V->rhs, V->prec, V->red(), V->dS, 0, V->codes, (float*)nullptr);
+  DISPATCH(V, k_rhs_b2, V->n, V->geo(), 1.f, V->rhs, V->prec, V->red(), V->dS, 0, V->codes, (float*)nullptr,
+           WorkVectors{});
   prepare_multigrid(V);
   CK(cudaMemcpyAsync(V->res, x, len * 4, cudaMemcpyHostToDevice, V->stream));
   if (V->half()) LAUNCH_G(V, k_reset_scalars, 1, 1, V->dS, 0.f);  // FP16 storage, r unscaled (vinv = 1)
