@@ -1,0 +1,229 @@
+// The multigrid PCG loop in one cooperative launch, for volumes whose passes are latency.
+//
+// In the loop graph an iteration of a 128^3 volume is seventeen kernels, and 4 us of each is its launch boundary, the
+// gate, and the chain of loads before its first sum: 150 us per iteration, when the passes' work is a third of
+// that.  Here one CTA per SM stays for the whole loop, the passes are separated by grid meetings (GridTeam: 1.3 us, 2.1
+// with a sum), and the scalars are on chip.  The fine passes are the paired march's (fd3_zmarch2.cuh) with three teams
+// of 256 threads per CTA, each taking chunks of a tile in turn; the levels run one cell per thread, their warps
+// spread over the SMs; the levels of at most TAIL_REG_THREADS cells run in the first CTA, its rows kept in shared
+// memory for the whole loop.
+//
+// Every cell value is that of the separate kernels; the f64 sums are added in the order of the chunks here.  Whole
+// projections, separate kernels and one launch (B200): 64^3 basin 1.49 and 1.27 ms, a 12288-cell time step 0.90 and
+// 0.79, 96^3 1.89 and 1.85; above 2^20 cells the separate kernels, whose chunks the hardware deals as SMs free up,
+// are faster (a team's chunk takes 9 us, the slowest 15, at 128^3).
+#pragma once
+
+#include "fd3_persist.cuh"
+#include "fd3_zmarch2.cuh"
+
+namespace fd3 {
+
+constexpr int MG_TEAMS = 3;
+constexpr int MG_THREADS = MG_TEAMS * Z2T;  // one CTA per SM, 80 registers
+constexpr int MG_LEVELS = 8;                // levels above the tail
+
+struct MgLoop {
+  Geo g;
+  const unsigned short* codes;
+  const float* prec;
+  float *p, *r, *dir[2], *q;
+  void *z, *z2;
+  Lev lev[MG_LEVELS];
+  int nlev;    // levels above the tail
+  Lev tail[TAIL_REG_LEVELS];
+  int ntail;
+  Air air;     // of level 0 (sh = 1)
+  Scalars* S;
+  GridSlots* slots;
+};
+
+struct MgShared {
+  ZPlanes2 sbuf[MG_TEAMS][2];
+  ZResid2 tr[MG_TEAMS][2];
+  TailShared tail;
+  GridShared grid;
+  int chunk;  // layers of a chunk
+};
+
+struct TeamSync {
+  int id;
+  __device__ __forceinline__ void operator()() const {
+    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(Z2T) : "memory");
+  }
+};
+
+// Layers of a chunk: the even number that makes the longest team's march shortest, a chunk of K layers counting K + 2
+// (its halo layers) and the teams taking the chunks that hold water in turn.
+__device__ __forceinline__ int mg_pick_chunk(const Geo& g, int teams, int* cost) {
+  const int ntx = (g.nx + Z2X - 1) / Z2X, nty = (g.ny + Z2Y - 1) / Z2Y;
+  if (threadIdx.x < 8) cost[threadIdx.x] = 0;
+  __syncthreads();
+  for (int q = threadIdx.x; q < 8 * ntx * nty; q += MG_THREADS) {
+    const int k = 2 + 2 * (q & 7), t = q >> 3;
+    const int top = ztile2_at(g, t % ntx, t / ntx, 0, g.nz, 0, 0).k1;
+    if (top > 0) atomicAdd(cost + (q & 7), (top + k - 1) / k);
+  }
+  __syncthreads();
+  int best = 2, least = 0x7fffffff;
+  for (int q = 0; q < 8; ++q) {
+    const int k = 2 + 2 * q, c = (cost[q] + teams - 1) / teams * (k + 2);
+    if (c < least) { least = c; best = k; }
+  }
+  return best;
+}
+
+template <class T>
+__global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant__ MgLoop a) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // no early start of the next kernel: its CTAs find no room
+  Scalars* S = a.S;
+  if (!S->active) return;
+  extern __shared__ float4 mg_smem4[];
+  MgShared& sh = *reinterpret_cast<MgShared*>(mg_smem4);
+  const Geo& g = a.g;
+  GridTeam<MG_THREADS> grid(a.slots, sh.grid);
+  const int tid = threadIdx.x, team = tid / Z2T, tx = tid & 31, ty = (tid >> 5) & 7, teams = gridDim.x * MG_TEAMS;
+  const int ntx = (g.nx + Z2X - 1) / Z2X, nty = (g.ny + Z2Y - 1) / Z2Y, tiles = ntx * nty;
+  const int K = mg_pick_chunk(g, teams, reinterpret_cast<int*>(sh.grid.warp));
+  __syncthreads();
+  const int chunks = tiles * ((g.nz + K - 1) / K);
+  const bool first_cta = blockIdx.x == 0;
+  if (first_cta && a.ntail > 0) tail_rows(a.tail, a.ntail, sh.tail);
+  T* z = static_cast<T*>(a.z);
+  T* z2 = static_cast<T*>(a.z2);
+  const TeamSync sync{6 + team};
+  // f(march) over the chunks of this thread's team: the chunks in order of height, dealt to the CTAs first
+  auto each_chunk = [&](auto f) {
+    for (int q = team * gridDim.x + blockIdx.x; q < chunks; q += teams) {
+      const int tile = q % tiles;
+      const March2<TeamSync> march{g,  a.codes,       ztile2_at(g, tile % ntx, tile / ntx, q / tiles * K, K, tx, ty), tx,
+                                   ty, sh.sbuf[team], sh.tr[team], sync};
+      f(march);
+      sync();  // the planes are free for the next chunk
+    }
+  };
+  // f(i) for i = 0 .. n - 1 (a multiple of 32 rounded up), whole warps, spread over the SMs warp by warp
+  auto each_warp = [&](int n, auto f) {
+    for (int w = (tid >> 5) * gridDim.x + blockIdx.x; 32 * w < n; w += gridDim.x * (MG_THREADS / 32)) f(32 * w + (tid & 31));
+  };
+  auto air = [&](int l) { return Air{l < 3 ? a.air.ztop : nullptr, l + 1, a.air.ntx}; };
+  float vinv = S->vinv;
+
+  // z = M^-1 r with r.z in rz (v_cycle3); false when a meeting failed
+  auto vcycle = [&](double& rz) -> bool {
+    const float rs = Store<T>::half ? vinv : 1.f;
+    const bool levels = a.nlev + a.ntail > 0;
+    each_chunk([&](const auto& m) { march_pre(m, a.prec, a.r, z, rs); });
+    if (!grid.meet()) return false;
+    const Lev& L0 = a.nlev > 0 ? a.lev[0] : a.tail[0];
+    if (levels) {
+      each_chunk([&](const auto& m) { march_restrict(m, a.r, (const T*)z, L0, rs); });
+      if (!grid.meet()) return false;
+      const int last = a.nlev - 1;
+#pragma unroll 1
+      for (int l = 0; l < a.nlev; ++l) {
+        const Lev& L = a.lev[l];
+        if (l == last && a.ntail == 0) {  // a large coarsest level: its eight sweeps
+#pragma unroll 1
+          for (int s = 0; s < 8; ++s) {
+            each_warp(L.n, [&](int c) {
+              if (c < L.n) level_sweep_at<T>(L, (s & 1) ? L.x2 : L.x, (s & 1) ? L.x : L.x2, s == 0, c);
+            });
+            if (!grid.meet()) return false;
+          }
+        } else {
+          const Lev& C = l < last ? a.lev[l + 1] : a.tail[0];
+          each_warp(L.n, [&](int c) {
+            if (c < L.n) level_pre_at<T>(L, air(l), c);
+          });
+          if (!grid.meet()) return false;
+          each_warp(8 * C.n, [&](int q8) { level_restrict8_at<T>(L, C, air(l + 1), q8); });
+          if (!grid.meet()) return false;
+        }
+      }
+      if (a.ntail > 0) {
+        if (first_cta) {
+          const Lev& L = a.tail[0];
+          if (tid < L.n) sh.tail.R[tid] = Store<T>::ld(as<T>(L.r), tid);
+          __syncthreads();
+          tail_cycle(a.tail, a.ntail, sh.tail);
+          if (tid < L.n) Store<T>::st(as<T>(L.x), tid, sh.tail.XF[tid]);
+        }
+        if (!grid.meet()) return false;
+      }
+      // up: level l's second post-sweep is part of level l - 1's first (level_post21_at)
+      const int top = a.ntail > 0 ? last : last - 1;
+#pragma unroll 1
+      for (int l = top; l >= 0; --l) {
+        const Lev& L = a.lev[l];
+        const Lev& C = l < last ? a.lev[l + 1] : a.tail[0];
+        if (l < top) each_warp(8 * C.n, [&](int q8) { level_post21_at<T>(L, C, air(l + 1), q8); });
+        else each_warp(L.n, [&](int c) {
+          if (c < L.n) level_post1_at<T>(L, C, air(l), c);
+        });
+        if (!grid.meet()) return false;
+      }
+      if (top >= 0) {
+        const Lev& L = a.lev[0];
+        each_warp(L.n, [&](int c) {
+          if (c < L.n) level_post2_at<T>(L, air(0), c);
+        });
+        if (!grid.meet()) return false;
+      }
+    }
+    each_chunk([&](const auto& m) { march_post1(m, a.prec, a.r, (const T*)z, L0, levels ? 1 : 0, z2, rs); });
+    if (!grid.meet()) return false;
+    double acc = 0.0, none = 0.0;
+    each_chunk([&](const auto& m) { march_post2(m, a.prec, a.r, (const T*)z2, z, rs, acc); });
+    if (!grid.template sum<false>(acc, none)) return false;
+    rz = acc;
+    return true;
+  };
+
+  const double tolb2 = S->tolb2, phys = S->phys;
+  const unsigned max_iters = S->max_iters;
+  const float vk = S->vk;
+  double rr = S->rr, rn = rr, rz = 0.0, none = 0.0;
+  unsigned it = S->it;
+  int status = 0, brk = 0, mode = 0;
+  float beta = 0.f;
+  // the prime (mode 0), then iterations: each ends with a V-cycle
+#pragma unroll 1
+  for (;;) {
+    double zn = 0.0;
+    if (!vcycle(zn)) { status = 100; break; }
+    if (!isfinite(zn)) { status = 2; break; }
+    if (mode) {  // FIN_RZ_ITER
+      beta = (float)(zn / rz);
+      rr = rn;
+      ++it;
+    }
+    rz = zn;
+    const float* din = a.dir[it & 1];
+    float* dout = a.dir[(it & 1) ^ 1];
+    double dq = 0.0;
+    each_chunk([&](const auto& m) { march_dir(m, (const T*)z, din, dout, a.q, mode, beta, dq); });
+    if (!grid.template sum<false>(dq, none)) { status = 100; break; }
+    if (!(dq > 0.0)) { brk = 1; break; }  // FIN_DQ
+    const float alpha = (float)(rz / dq);
+    double acc = 0.0;
+    each_chunk([&](const auto& m) { chunk_update(g, m.t, alpha, a.p, a.r, dout, a.q, acc); });
+    if (!grid.template sum<false>(acc, none)) { status = 100; break; }
+    rn = acc;
+    if (!isfinite(rn)) { status = 2; break; }  // FIN_RN
+    if (vk > 0.f && rn > 0.0) vinv = (float)((double)vk / sqrt(rn));
+    if (!((rn > tolb2 || rn > phys) && it + 1 < max_iters)) { rr = rn; ++it; break; }
+    mode = 1;
+  }
+  if (tid == 0 && (first_cta || status == 100)) {
+    S->rr = rr;
+    S->rz = rz;
+    S->it = it;
+    S->brk = brk;
+    S->vinv = vinv;
+    if (status) S->status = status;
+    S->active = 0;
+  }
+}
+
+}  // namespace fd3

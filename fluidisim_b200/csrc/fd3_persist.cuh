@@ -35,16 +35,17 @@ struct GridSlots {
   unsigned arrived;
 };
 struct GridShared {
-  double warp[GRID_THREADS / 32][2];
+  double warp[32][2];
   double sum[2];
 };
+template <int THREADS>
 struct GridTeam {
   GridSlots* slots;
   GridShared& sh;
   unsigned meeting = 0;
   __device__ __forceinline__ GridTeam(GridSlots* s, GridShared& shared) : slots(s), sh(shared) {}
 
-  // Called by every thread of every CTA; what the team wrote to global memory before is visible to all of
+  // What the team wrote to global memory before is visible to all of
   // it after.  False, for the whole CTA, when another did not arrive within GRID_POLLS.
   __device__ __forceinline__ bool arrive_and_wait() {  // thread 0; the CTA's writes ordered before by a barrier
     ++meeting;
@@ -55,6 +56,14 @@ struct GridTeam {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&slots->arrived) : "memory");
     } while (seen < target && ++polls < GRID_POLLS);
     return seen >= target;
+  }
+  // A meeting without a sum.
+  __device__ __forceinline__ bool meet() {
+    __syncthreads();
+    bool late = false;
+    if (threadIdx.x == 0) late = !arrive_and_wait();
+    else ++meeting;
+    return !__syncthreads_or(late);
   }
   // Sums a (and b, when TWO) over every thread of the grid: the same totals, added in the same order, for
   // every thread.  A meeting.
@@ -76,7 +85,7 @@ struct GridTeam {
     if (threadIdx.x == 0) {
       double2 p = make_double2(0.0, 0.0);
 #pragma unroll
-      for (int q = 0; q < GRID_THREADS / 32; ++q) {
+      for (int q = 0; q < THREADS / 32; ++q) {
         p.x += sh.warp[q][0];
         if (TWO) p.y += sh.warp[q][1];
       }
@@ -182,7 +191,7 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
   if (!S->active) return;
   extern __shared__ float kept[];  // [CELLS][7][GRID_THREADS]: six coefficients and p
   __shared__ GridShared sh;
-  GridTeam team(slots, sh);
+  GridTeam<GRID_THREADS> team(slots, sh);
   auto K = [&](int s, int f) -> float& { return kept[(s * 7 + f) * GRID_THREADS + threadIdx.x]; };
   constexpr int PAIR = CELLS < 2 ? 1 : 2;
   const int nxny = g.nx * g.ny;

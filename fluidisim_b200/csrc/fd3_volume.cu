@@ -30,6 +30,7 @@
 #include "fd3_batch.cuh"
 #include "fd3_linear.cuh"
 #include "fd3_persist.cuh"
+#include "fd3_mgloop.cuh"
 #include "fd3_levels.cuh"
 
 using namespace fd3;
@@ -89,6 +90,13 @@ constexpr int kRecMaxCells = 1 << 27;
 
 // Volumes from this many cells run the four-cells-per-thread fine kernels by default (kernels = 0).
 constexpr long long kQuadMinCells = 1LL << 23;
+// The TMA-staged kernels by default from this many cells (projections, ms, paired / TMA-staged: 112^3 basin 2.25 / 2.33;
+// 160 x 80 x 120 tank 4.26 / 4.08; 128^3 basin 2.60 / 2.53; 160^3 3.94 / 3.61; 256^3 wave 10.25 / 9.38).
+constexpr long long kTmaMinCells = 1500000;
+// The loop in one launch (k_mg_loop) up to this many cells (ms, separate kernels / one launch: 64^3 basin 1.49 / 1.27,
+// 80^3 1.63 / 1.51, 128 x 64 x 96 tank 1.84 / 1.78, 96^3 1.89 / 1.85, 112^3 2.25 / 2.22, 128^3 2.60 / 2.87, 160 x 80 x 120
+// tank 4.26 / 4.82): above, its slowest team's chunks cost more than the launches it saves.
+constexpr long long kLoopMaxCells = 1LL << 20;
 
 // Coarse levels of at most this many cells are solved together by one CTA (k_coarse_tail).
 constexpr int TAIL_MAX_CELLS = 512;
@@ -157,7 +165,7 @@ struct fd3_volume {
   float* p32 = nullptr;
   unsigned* count = nullptr;
   GridSlots* slots = nullptr;  // the meetings of k_cg_loop
-  int grid_ctas = 0;          // CTAs of a cooperative launch of GRID_THREADS threads (one per SM)
+  int grid_ctas = 0;          // CTAs of the cooperative launches (one per SM; 0: not to be had)
   Scalars* dS = nullptr;
   Scalars* hS = nullptr;  // pinned
   int* dflag = nullptr;
@@ -222,12 +230,10 @@ struct fd3_volume {
   }
   // TMA-staged fine kernels (fd3_tmarch.cuh) for the V-cycle's and the direction's passes: f32 storage,
   // nx % 8 == 0 and the multigrid, chosen explicitly (kernels = 5) or by default on volumes of at least
-  // kQuadMinCells, where the passes stream from HBM (measured on the 256^3 wave: 19.3 against 20.0 ms
-  // per projection with four cells per thread; on the 128^3 basin, which sits in L2, 3.07 against
-  // 3.03 ms with two cells per thread, which stays the default there)
+  // kTmaMinCells
   bool tmaf() const {
     if (!blocked() || nx % 8 != 0 || opt.storage == FD3_STORAGE_F16 || !mg_on() || tma_state < 0) return false;
-    return opt.kernels == 5 || (opt.kernels == 0 && (long long)n >= kQuadMinCells);
+    return opt.kernels == 5 || (opt.kernels == 0 && (long long)n >= kTmaMinCells);
   }
   // four cells per thread: with f32 storage and nx % 4 == 0, chosen explicitly (kernels = 4) or by
   // default on volumes of at least kQuadMinCells, where the passes stream from HBM (measured: 256^3
@@ -251,6 +257,13 @@ struct fd3_volume {
            (paired() ? 32 : 0) | (half() ? 64 : 0) | (sparse ? 128 : 0) |  // the captured Geo holds the set's mask
            (opt.no_tile_skip ? 256 : 0) | (skip_air ? 2048 : 0) | (quad() ? 512 : 0) | (tmaf() ? 1024 : 0);
   }
+  // With the multigrid, the inner loop in one cooperative launch (k_mg_loop): the default on the paired march up to
+  // kLoopMaxCells.  Profiling, use_graphs = 0 and kernels = 3 keep the separate kernels.
+  bool mg_loop() const {
+    return opt.kernels == 0 && paired() && mg_on() && (long long)n <= kLoopMaxCells && opt.use_graphs && !prof &&
+           grid_ctas > 0 && tail_reg && tail_first <= MG_LEVELS;
+  }
+  bool one_launch() const { return cg_loop() || mg_loop(); }
   Red red() const { return Red{p64, p32, count}; }
 };
 
@@ -880,10 +893,46 @@ void run_cg_loop(fd3_volume* V) {
   else launch_cg_loop<GRID_MAX_CELLS>(V, ctas);
 }
 
-// The whole inner loop enqueued, without a synchronisation: the cooperative launch, or the loop graph.
+// The multigrid PCG loop, prime included, as one cooperative launch.
+template <class T>
+void launch_mg_loop(fd3_volume* V) {
+  MgLoop a{};
+  a.g = V->geo();
+  a.codes = V->codes;
+  a.prec = V->prec;
+  a.p = V->p; a.r = V->res; a.dir[0] = V->dir; a.dir[1] = V->dir2; a.q = V->tmp;
+  a.z = V->z; a.z2 = V->z2;
+  a.nlev = V->tail_first;
+  a.ntail = (int)V->levels.size() - V->tail_first;
+  for (int l = 0; l < a.nlev; ++l) a.lev[l] = V->levels[l];
+  for (int l = 0; l < a.ntail; ++l) a.tail[l] = V->levels[a.nlev + l];
+  a.air = Air{V->skip_air ? V->ztop : nullptr, 1, (V->nx + TILE_X - 1) / TILE_X};
+  a.S = V->dS;
+  a.slots = V->slots;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(V->grid_ctas);
+  cfg.blockDim = dim3(MG_THREADS);
+  cfg.dynamicSmemBytes = sizeof(MgShared);
+  cfg.stream = V->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_mg_loop<T>, a);
+  V->launches++;
+}
+
+// The whole inner loop enqueued, without a synchronisation: a cooperative launch, or the loop graph.
 int enqueue_loop(fd3_volume* V) {
   if (V->cg_loop()) {
     run_cg_loop(V);
+    return FD3_OK;
+  }
+  if (V->mg_loop()) {
+    LAUNCH_G(V, k_grid_reset, 1, 1, V->slots);
+    if (V->half()) launch_mg_loop<__half>(V);
+    else launch_mg_loop<float>(V);
     return FD3_OK;
   }
   const int mode = V->loop_key();
@@ -893,7 +942,7 @@ int enqueue_loop(fd3_volume* V) {
 }
 // The launches of `ran` iterations of the loop graph (the cooperative launch counts itself).
 void count_loop(fd3_volume* V, unsigned ran) {
-  if (!V->cg_loop()) V->launches += (unsigned long long)((ran + 1) / 2) * V->body_nodes;
+  if (!V->one_launch()) V->launches += (unsigned long long)((ran + 1) / 2) * V->body_nodes;
 }
 
 // Run the inner loop until S->active drops.
@@ -1049,12 +1098,12 @@ int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_r
   // would not have started it) and the outer checks, with one synchronisation at their end.  A
   // prime that turns out unneeded changes nothing the checks or the report read; a non-finite
   // set-up stops the loop on the device and is reported after the checks, as before them.
-  const bool cg = V->cg_loop();  // its loop primes itself
-  const bool speculate = !ord && (V->mg_on() || cg) && V->opt.use_graphs && !V->prof;
+  const bool self = V->one_launch();  // its loop primes itself
+  const bool speculate = !ord && (V->mg_on() || self) && V->opt.use_graphs && !V->prof;
   Checks ck{};
   bool have_checks = false;
   if (speculate) {
-    if (!cg) prime(V);
+    if (!self) prime(V);
     LAUNCH_G(V, k_loop_start_dev, 1, 1, V->dS, max_iters);
     TRY(enqueue_loop(V));
     TRY(outer_checks(V, k1, &ck));
@@ -1091,7 +1140,7 @@ int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_r
     } else {
     if (b2 > 0 && above(rr) && it < max_iters) {
       if (!primed) {
-        if (!cg) prime(V);
+        if (!self) prime(V);
         primed = true;
       }
       LAUNCH_G(V, k_loop_start, 1, 1, V->dS, rr, tolb2, phys, it, max_iters);
@@ -1152,7 +1201,7 @@ int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_r
       since = 0;
     }
     rr = actual;
-    if (!cg) prime(V);
+    if (!self) prime(V);
   }
   double residual;
   if (ord) residual = b2 > 0 ? (double)std::sqrt((float)actual_rr / (float)b2) : 0.0;
@@ -1373,6 +1422,11 @@ int alloc_state(fd3_volume* V) {
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_cg_loop<GRID_MAX_CELLS>, GRID_THREADS,
                                                    cg_smem(GRID_MAX_CELLS)));
   V->grid_ctas = coop && resident >= 1 ? std::min(sms, GRID_MAX_CTAS) : 0;
+  for (auto k : {k_mg_loop<float>, k_mg_loop<__half>}) {
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MgShared)));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k, MG_THREADS, sizeof(MgShared)));
+    if (resident < 1) V->grid_ctas = 0;
+  }
   CK(cudaMallocHost((void**)&V->hS, sizeof(Scalars)));
   CK(cudaMallocHost((void**)&V->hflag, sizeof(int)));
   TRY(dalloc(V, &q, 32)); V->fsc = (double*)q;

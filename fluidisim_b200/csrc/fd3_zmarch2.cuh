@@ -42,21 +42,28 @@ struct ZTile2 {
   int i0, j, k0, k1, x0;
   bool inside;
 };
-template <int K2>
-__device__ __forceinline__ ZTile2 ztile2(const Geo& g) {
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int ntx = (g.nx + Z2X - 1) / Z2X, nty = (g.ny + Z2Y - 1) / Z2Y;
-  int b = blockIdx.x;
-  const int bx = b % ntx; b /= ntx;
-  const int by = b % nty; b /= nty;
+// The chunk of layers [k0, k0 + k2) of the tile (bx, by), less the air above it, for the thread (tx, ty) of its team.
+__device__ __forceinline__ ZTile2 ztile2_at(const Geo& g, int bx, int by, int k0, int k2, int tx, int ty) {
   ZTile2 t;
   t.x0 = bx * Z2X;
   t.i0 = t.x0 + 2 * tx;
   t.j = by * Z2Y + ty;
-  t.k0 = b * K2;
-  t.k1 = min(t.k0 + K2, g.nz);
+  t.k0 = k0;
+  t.k1 = min(min(k0 + k2, g.nz), tops64(g, t.x0, by * Z2Y));
   t.inside = t.i0 < g.nx && t.j < g.ny;  // nx even: i0 + 1 < nx too
+  if (g.tiles) {  // a 64 x 8 tile is two 32 x 8 tiles of the set's tile flags
+    const int ntx = (g.nx + TILE_X - 1) / TILE_X, row = by * ntx, q = t.x0 / TILE_X;
+    if (!g.tiles[row + q] && (q + 1 >= ntx || !g.tiles[row + q + 1])) t.k1 = t.k0;  // no column of the set
+  }
   return t;
+}
+template <int K2>
+__device__ __forceinline__ ZTile2 ztile2(const Geo& g) {
+  const int ntx = (g.nx + Z2X - 1) / Z2X, nty = (g.ny + Z2Y - 1) / Z2Y;
+  int b = blockIdx.x;
+  const int bx = b % ntx; b /= ntx;
+  const int by = b % nty; b /= nty;
+  return ztile2_at(g, bx, by, b * K2, K2, threadIdx.x & 31, threadIdx.x >> 5);
 }
 
 __device__ __forceinline__ float2 ld2(const float* __restrict__ p, int c) {
@@ -73,78 +80,116 @@ __device__ __forceinline__ void st2(float* __restrict__ p, int c, float a, float
 //   L.halo(i, j, k, c) -> Halo / L.hv: the operand of one cell (x halo)
 // E(c, Raw2, pc, ax0, ax1) consumes A.P at the pair (ax = 0 at a dry cell); A(k) runs after each
 // layer (all threads).
-template <int K2, class L, class E, class A = NoAfter>
-__device__ __forceinline__ void zmarch2(const Geo& g, const unsigned short* __restrict__ codes, const L& ld, E epi,
-                                        A after = A()) {
-  typedef typename L::Raw2 Raw2;
-  typedef typename L::Halo Halo;
-  typedef typename L::Halo2 Halo2;
-  __shared__ __align__(16) float sbuf[2][Z2Y + 2][Z2ROW];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  ZTile2 t = ztile2<K2>(g);
-  t.k1 = min(t.k1, tops64(g, t.x0, t.j - ty));
-  if (t.k0 >= t.k1) return;  // the chunk lies in the air
-  if (g.tiles) {  // a 64 x 8 tile is two 32 x 8 tiles of the set's tile flags
-    const int ntx = (g.nx + TILE_X - 1) / TILE_X, row = (t.j / TILE_Y) * ntx, a = t.x0 / TILE_X;
-    if (!g.tiles[row + a] && (a + 1 >= ntx || !g.tiles[row + a + 1])) return;  // no column of the set
-  }
-  const int nxny = g.nx * g.ny;
-  const int base = t.j * g.nx + t.i0;
-  // x halo: lane 0 the cell left of the tile, lane 31 the cell right of it
-  const int hxi = tx == 0 ? t.x0 - 1 : (tx == 31 ? t.x0 + Z2X : -1);
-  const bool hx_on = hxi >= 0 && hxi < g.nx && t.j < g.ny;
-  const int hxs = tx == 0 ? 1 : Z2X + 2;
-  // y halo: row 0 the pairs below the tile, row 7 the pairs above
-  const int hyj = ty == 0 ? t.j - 1 : (ty == Z2Y - 1 ? t.j + 1 : -1);
-  const bool hy_on = hyj >= 0 && hyj < g.ny && t.i0 < g.nx;
-  const int hys = ty == 0 ? 0 : Z2Y + 1;
-  auto fetch_full = [&](int k) { return (t.inside && k < g.nz && k >= 0) ? ld.full2(t.i0, t.j, k, base + k * nxny) : Raw2(); };
-  auto fetch_hx = [&](int k) { return (hx_on && k < t.k1) ? ld.halo(hxi, t.j, k, t.j * g.nx + hxi + k * nxny) : Halo(); };
-  auto fetch_hy = [&](int k) { return (hy_on && k < t.k1) ? ld.halo2(t.i0, hyj, k, hyj * g.nx + t.i0 + k * nxny) : Halo2(); };
-  auto fetch_code = [&](int k) {
-    return (t.inside && k < t.k1) ? *reinterpret_cast<const unsigned*>(codes + base + k * nxny) : 0u;
-  };
-
-  float2 pprev = make_float2(0.f, 0.f);
-  if (t.k0 > 0 && t.inside) pprev = ld.pv2(fetch_full(t.k0 - 1));
-  Raw2 rc = fetch_full(t.k0);
-  Raw2 rn = fetch_full(t.k0 + 1);
-  Halo hx = fetch_hx(t.k0);
-  Halo2 hy = fetch_hy(t.k0);
-  unsigned code = fetch_code(t.k0);
-  for (int k = t.k0; k < t.k1; ++k) {
-    const int c = base + k * nxny;
-    Raw2 rnn = fetch_full(k + 2 <= t.k1 ? k + 2 : g.nz);
-    Halo hx2 = fetch_hx(k + 1);
-    Halo2 hy2 = fetch_hy(k + 1);
-    const unsigned code2 = fetch_code(k + 1);
-    const float2 pc = t.inside ? ld.pv2(rc) : make_float2(0.f, 0.f);
-    const float2 pn = (t.inside && k + 1 < g.nz) ? ld.pv2(rn) : make_float2(0.f, 0.f);
-    float (*s)[Z2ROW] = sbuf[(k - t.k0) & 1];
-    *reinterpret_cast<float2*>(&s[ty + 1][2 + 2 * tx]) = pc;
-    if (hxi >= 0 || tx == 0 || tx == 31) s[ty + 1][hxs] = hx_on ? ld.hv(hx) : 0.f;
-    if (hyj >= 0 || ty == 0 || ty == Z2Y - 1)
-      *reinterpret_cast<float2*>(&s[hys][2 + 2 * tx]) = hy_on ? ld.hv2(hy) : make_float2(0.f, 0.f);
-    __syncthreads();
-    if (t.inside) {
-      const unsigned c0 = code & 0xffffu, c1 = code >> 16;
-      const float xm0 = s[ty + 1][1 + 2 * tx], xp1 = s[ty + 1][4 + 2 * tx];
-      const float2 ym = *reinterpret_cast<const float2*>(&s[ty][2 + 2 * tx]);
-      const float2 yp = *reinterpret_cast<const float2*>(&s[ty + 2][2 + 2 * tx]);
-      float ax0 = 0.f, ax1 = 0.f;
-      if (c0 & RC_WET) ax0 = apply_code_nb(g, c0, t.i0, t.j, k, pc.x, xm0, pc.y, ym.x, yp.x, pprev.x, pn.x);
-      if (c1 & RC_WET) ax1 = apply_code_nb(g, c1, t.i0 + 1, t.j, k, pc.y, pc.x, xp1, ym.y, yp.y, pprev.y, pn.y);
-      epi(c, rc, pc, ax0, ax1);
-    }
-    after(k);
-    pprev = pc;
-    rc = rn;
-    rn = rnn;
-    hx = hx2;
-    hy = hy2;
-    code = code2;
-  }
+// A row whose six faces all open onto water with aperture 1 (apply_code_nb's masked sum, no face missing).
+__device__ __forceinline__ float interior_row(const Geo& g, float pc, float xm, float xp, float ym, float yp, float zm,
+                                              float zp) {
+  float acc = 0.f;
+  acc += pc - xm;
+  acc += pc - xp;
+  acc += pc - ym;
+  acc += pc - yp;
+  acc += pc - zm;
+  acc += pc - zp;
+  return acc * g.inv;
 }
+// The team is 256 threads, tx in 0..31 and ty in 0..7, that meet at sync(): a CTA, or a part of one.
+struct BlockSync {
+  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+};
+typedef float ZPlanes2[Z2Y + 2][Z2ROW];
+typedef float ZResid2[Z2Y][Z2X];
+template <class Sync>
+struct March2 {
+  const Geo& g;
+  const unsigned short* codes;
+  ZTile2 t;
+  int tx, ty;
+  ZPlanes2* sbuf;  // two
+  ZResid2* tr;     // two, of the restriction
+  Sync sync;
+
+  __device__ __forceinline__ bool any() const { return t.k0 < t.k1; }
+
+  template <class L, class E, class A = NoAfter>
+  __device__ __forceinline__ void operator()(const L& ld, E epi, A after = A()) const {
+    typedef typename L::Raw2 Raw2;
+    typedef typename L::Halo Halo;
+    typedef typename L::Halo2 Halo2;
+    if (!any()) return;
+    const int nxny = g.nx * g.ny;
+    const int base = t.j * g.nx + t.i0;
+    // x halo: lane 0 the cell left of the tile, lane 31 the cell right of it
+    const int hxi = tx == 0 ? t.x0 - 1 : (tx == 31 ? t.x0 + Z2X : -1);
+    const bool hx_on = hxi >= 0 && hxi < g.nx && t.j < g.ny;
+    const int hxs = tx == 0 ? 1 : Z2X + 2;
+    // y halo: row 0 the pairs below the tile, row 7 the pairs above
+    const int hyj = ty == 0 ? t.j - 1 : (ty == Z2Y - 1 ? t.j + 1 : -1);
+    const bool hy_on = hyj >= 0 && hyj < g.ny && t.i0 < g.nx;
+    const int hys = ty == 0 ? 0 : Z2Y + 1;
+    auto fetch_full = [&](int k) { return (t.inside && k < g.nz && k >= 0) ? ld.full2(t.i0, t.j, k, base + k * nxny) : Raw2(); };
+    auto fetch_hx = [&](int k) { return (hx_on && k < t.k1) ? ld.halo(hxi, t.j, k, t.j * g.nx + hxi + k * nxny) : Halo(); };
+    auto fetch_hy = [&](int k) { return (hy_on && k < t.k1) ? ld.halo2(t.i0, hyj, k, hyj * g.nx + t.i0 + k * nxny) : Halo2(); };
+    auto fetch_code = [&](int k) {
+      return (t.inside && k < t.k1) ? *reinterpret_cast<const unsigned*>(codes + base + k * nxny) : 0u;
+    };
+
+    // every load two layers ahead: a layer's work covers half an L2 round trip
+    float2 pprev = make_float2(0.f, 0.f);
+    const Raw2 rp = fetch_full(t.k0 > 0 ? t.k0 - 1 : g.nz);
+    Raw2 rc = fetch_full(t.k0);
+    Raw2 rn = fetch_full(t.k0 + 1);
+    Halo hx = fetch_hx(t.k0), hxn = fetch_hx(t.k0 + 1);
+    Halo2 hy = fetch_hy(t.k0), hyn = fetch_hy(t.k0 + 1);
+    unsigned code = fetch_code(t.k0), coden = fetch_code(t.k0 + 1);
+    if (t.k0 > 0 && t.inside) pprev = ld.pv2(rp);
+    float2 pc = t.inside ? ld.pv2(rc) : make_float2(0.f, 0.f);
+    int c = base + t.k0 * nxny;
+    for (int k = t.k0; k < t.k1; ++k, c += nxny) {
+      const Raw2 rnn = fetch_full(k + 2 <= t.k1 ? k + 2 : g.nz);
+      const Halo hx2 = fetch_hx(k + 2);
+      const Halo2 hy2 = fetch_hy(k + 2);
+      const unsigned code2 = fetch_code(k + 2);
+      float (*s)[Z2ROW] = sbuf[(k - t.k0) & 1];
+      *reinterpret_cast<float2*>(&s[ty + 1][2 + 2 * tx]) = pc;
+      if (hxi >= 0 || tx == 0 || tx == 31) s[ty + 1][hxs] = hx_on ? ld.hv(hx) : 0.f;
+      if (hyj >= 0 || ty == 0 || ty == Z2Y - 1)
+        *reinterpret_cast<float2*>(&s[hys][2 + 2 * tx]) = hy_on ? ld.hv2(hy) : make_float2(0.f, 0.f);
+      sync();
+      const float2 pn = (t.inside && k + 1 < g.nz) ? ld.pv2(rn) : make_float2(0.f, 0.f);
+      if (t.inside) {
+        const float xm0 = s[ty + 1][1 + 2 * tx], xp1 = s[ty + 1][4 + 2 * tx];
+        const float2 ym = *reinterpret_cast<const float2*>(&s[ty][2 + 2 * tx]);
+        const float2 yp = *reinterpret_cast<const float2*>(&s[ty + 2][2 + 2 * tx]);
+        float ax0 = 0.f, ax1 = 0.f;
+        if (code == (RC_INTERIOR | RC_INTERIOR << 16)) {  // the bulk: every face open onto water, no decoding
+          ax0 = interior_row(g, pc.x, xm0, pc.y, ym.x, yp.x, pprev.x, pn.x);
+          ax1 = interior_row(g, pc.y, pc.x, xp1, ym.y, yp.y, pprev.y, pn.y);
+        } else {
+          const unsigned c0 = code & 0xffffu, c1 = code >> 16;
+          if (c0 & RC_WET) ax0 = apply_code_nb(g, c0, t.i0, t.j, k, pc.x, xm0, pc.y, ym.x, yp.x, pprev.x, pn.x);
+          if (c1 & RC_WET) ax1 = apply_code_nb(g, c1, t.i0 + 1, t.j, k, pc.y, pc.x, xp1, ym.y, yp.y, pprev.y, pn.y);
+        }
+        epi(c, rc, pc, ax0, ax1);
+      }
+      after(k);
+      pprev = pc;
+      pc = pn;
+      rc = rn;
+      rn = rnn;
+      hx = hxn;
+      hxn = hx2;
+      hy = hyn;
+      hyn = hy2;
+      code = coden;
+      coden = code2;
+    }
+  }
+};
+// The march of a kernel whose CTAs are the chunks.
+#define MARCH2(K2)                                                              \
+  __shared__ __align__(16) ZPlanes2 sbuf_[2];                                   \
+  const March2<BlockSync> march{g,    codes,   ztile2<K2>(g), (int)(threadIdx.x & 31), (int)(threadIdx.x >> 5), \
+                                sbuf_, nullptr, BlockSync()}
 
 // Loaders.  T is the storage of the V-cycle vectors (z, z2, the coarse x): f32, or FP16 in the
 // mixed-precision mode, where the V-cycle also sees r scaled by rs (Scalars::vinv).
@@ -253,40 +298,125 @@ struct L2LoadR {  // operand x, with r carried for the epilogue
   __device__ __forceinline__ float hv(const Halo& h) const { return h.v; }
 };
 
-// p += alpha d, r -= alpha q, with r.r (FIN_RN) over the chunks of the march: K2 layers of a 64 x 8 tile,
-// the loads of all of them in flight together, the air left alone.  kv_update_rn streams the whole volume
-// instead (402 MB of a 256^3 wave, 69 us; 50 us here, where 45% of the layers are water).
+// The passes on a march, for the kernels below and the one-launch loop.
+// p += alpha d, r -= alpha q over a chunk, the loads of four layers in flight together; r.r added to acc.
+__device__ __forceinline__ void chunk_update(const Geo& g, const ZTile2& t, float alpha, float* p, float* r, const float* d,
+                                             const float* q, double& acc) {
+  if (!t.inside) return;
+  const int nxny = g.nx * g.ny, base = t.j * g.nx + t.i0;
+  for (int k0 = t.k0; k0 < t.k1; k0 += 4) {
+    float2 P[4], R[4], D[4], Q[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (k0 + e >= t.k1) continue;
+      const int c = base + (k0 + e) * nxny;
+      P[e] = ld2(p, c);
+      R[e] = ld2(r, c);
+      D[e] = ld2(d, c);
+      Q[e] = ld2(q, c);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (k0 + e >= t.k1) continue;
+      const int c = base + (k0 + e) * nxny;
+      const float r0 = R[e].x - alpha * Q[e].x, r1 = R[e].y - alpha * Q[e].y;
+      st2(p, c, P[e].x + alpha * D[e].x, P[e].y + alpha * D[e].y);
+      st2(r, c, r0, r1);
+      acc += (double)r0 * (double)r0;
+      acc += (double)r1 * (double)r1;
+    }
+  }
+}
+// d = z (+ beta d) into dout, q = A d; d.q added to acc.
+template <class T, class M>
+__device__ __forceinline__ void march_dir(const M& march, const T* z, const float* din, float* dout, float* q, int mode,
+                                          float beta, double& acc) {
+  march(L2Dir<T>{z, din, mode, beta}, [&](int c, const typename L2Dir<T>::Raw2&, float2 pc, float a0, float a1) {
+    st2(dout, c, pc.x, pc.y);
+    st2(q, c, a0, a1);
+    acc += (double)pc.x * (double)a0;
+    acc += (double)pc.y * (double)a1;
+  });
+}
+// The two pre-sweeps from z = 0.
+template <class T, class M>
+__device__ __forceinline__ void march_pre(const M& march, const float* prec, const float* r, T* z2, float rs) {
+  march(L2Z1<T>{prec, r, rs}, [&](int c, const typename L2Z1<T>::Raw2& o, float2 pc, float a0, float a1) {
+    float z0 = pc.x, z1 = pc.y;
+    if (o.m.x > 0.f) z0 += OMEGA * o.m.x * (rsc<T>(o.r.x, rs) - a0);
+    if (o.m.y > 0.f) z1 += OMEGA * o.m.y * (rsc<T>(o.r.y, rs) - a1);
+    Store<T>::st2(z2, c, z0, z1);
+  });
+}
+// Prolongation + zeroing + first post-sweep (or the plain third sweep without coarse levels).
+template <class T, class M>
+__device__ __forceinline__ void march_post1(const M& march, const float* prec, const float* r, const T* zin, const Lev& L,
+                                            int prolong, T* zout, float rs) {
+  march(L2Prolong<T>{zin, prec, r, as<T>(L.x), L.nx, L.ny, prolong},
+        [&](int c, const typename L2Prolong<T>::Raw2& o, float2 pc, float a0, float a1) {
+          float z0 = pc.x, z1 = pc.y;
+          if (o.m.x > 0.f) z0 += OMEGA * o.m.x * (rsc<T>(o.r.x, rs) - a0);
+          if (o.m.y > 0.f) z1 += OMEGA * o.m.y * (rsc<T>(o.r.y, rs) - a1);
+          Store<T>::st2(zout, c, z0, z1);
+        });
+}
+// Second post-sweep; r.z added to acc.  The dot takes the z that is stored (the value the direction update reads
+// back) and the unscaled r.
+template <class T, class M>
+__device__ __forceinline__ void march_post2(const M& march, const float* prec, const float* r, const T* zin, T* zout,
+                                            float rs, double& acc) {
+  march(L2Sweep<T>{zin, prec, r}, [&](int c, const typename L2Sweep<T>::Raw2& o, float2 pc, float a0, float a1) {
+    float z0 = pc.x, z1 = pc.y;
+    if (o.m.x > 0.f) z0 += OMEGA * o.m.x * (rsc<T>(o.r.x, rs) - a0);
+    if (o.m.y > 0.f) z1 += OMEGA * o.m.y * (rsc<T>(o.r.y, rs) - a1);
+    Store<T>::st2(zout, c, z0, z1);
+    acc += (double)o.r.x * (double)Store<T>::rt(z0);
+    acc += (double)o.r.y * (double)Store<T>::rt(z1);
+  });
+}
+// Residual r - A z at every fine cell and its 8-child mean (restrict3, delta3d_multigrid.rs:258-272):
+// each thread's pair is one coarse cell's x children; the even rows sum the eight children, in the
+// reference's CHILDREN order, from the two layers kept in shared memory.
+template <class T, class M>
+__device__ __forceinline__ void march_restrict(const M& march, const float* r, const T* z, const Lev& L, float rs) {
+  const ZTile2& t = march.t;
+  ZResid2* tr = march.tr;
+  const int tx = march.tx, ty = march.ty, nxny = march.g.nx * march.g.ny;
+  march(
+      L2LoadR<T>{z, r},
+      [&](int c, const typename L2LoadR<T>::Raw2& o, float2, float a0, float a1) {
+        *reinterpret_cast<float2*>(&tr[(c / nxny) & 1][ty][2 * tx]) =
+            make_float2(rsc<T>(o.r.x, rs) - a0, rsc<T>(o.r.y, rs) - a1);
+      },
+      [&](int k) {
+        if (k & 1) {
+          march.sync();  // the epilogue's tr writes before the reads below
+          if (t.inside && !(ty & 1)) {
+            float sum = 0.f;
+            sum += tr[0][ty][2 * tx];
+            sum += tr[0][ty][2 * tx + 1];
+            sum += tr[0][ty + 1][2 * tx];
+            sum += tr[0][ty + 1][2 * tx + 1];
+            sum += tr[1][ty][2 * tx];
+            sum += tr[1][ty][2 * tx + 1];
+            sum += tr[1][ty + 1][2 * tx];
+            sum += tr[1][ty + 1][2 * tx + 1];
+            Store<T>::st(as<T>(L.r), ((k >> 1) * L.ny + (t.j >> 1)) * L.nx + (t.i0 >> 1), 0.125f * sum);
+          }
+        }
+      });
+}
+
+// p += alpha d, r -= alpha q, with r.r (FIN_RN) over the chunks of the march, the air left alone.  kv_update_rn streams
+// the whole volume instead (402 MB of a 256^3 wave, 69 us; 50 us here, where 45% of the layers are water).
 template <int K2>
 __global__ void __launch_bounds__(Z2T) kx_update_rn(Geo g, float* __restrict__ p, float* __restrict__ r,
                                                     const float* __restrict__ d, const float* __restrict__ q, Red red,
                                                     Scalars* S) {
   KSTART();
   if (!S->active) return;
-  const float alpha = S->alpha;
-  ZTile2 t = ztile2<K2>(g);
-  t.k1 = min(t.k1, tops64(g, t.x0, t.j - (int)(threadIdx.x >> 5)));
-  const int nxny = g.nx * g.ny, base = t.j * g.nx + t.i0 + t.k0 * nxny;
   double acc = 0.0;
-  float2 P[K2], R[K2], D[K2], Q[K2];
-#pragma unroll
-  for (int e = 0; e < K2; ++e) {
-    if (!t.inside || t.k0 + e >= t.k1) continue;
-    const int c = base + e * nxny;
-    P[e] = ld2(p, c);
-    R[e] = ld2(r, c);
-    D[e] = ld2(d, c);
-    Q[e] = ld2(q, c);
-  }
-#pragma unroll
-  for (int e = 0; e < K2; ++e) {
-    if (!t.inside || t.k0 + e >= t.k1) continue;
-    const int c = base + e * nxny;
-    const float r0 = R[e].x - alpha * Q[e].x, r1 = R[e].y - alpha * Q[e].y;
-    st2(p, c, P[e].x + alpha * D[e].x, P[e].y + alpha * D[e].y);
-    st2(r, c, r0, r1);
-    acc += (double)r0 * (double)r0;
-    acc += (double)r1 * (double)r1;
-  }
+  chunk_update(g, ztile2<K2>(g), S->alpha, p, r, d, q, acc);
   zreduce_finish(acc, red, S, FIN_RN);
 }
 
@@ -296,9 +426,9 @@ __global__ void __launch_bounds__(Z2T, FD3_ZMINB2) kx_residual(Geo g, const unsi
                                                              const float* __restrict__ p, const float* __restrict__ rhs,
                                                              float* __restrict__ res, Red red, Scalars* S, int op) {
   KSTART();
-  L2LoadR<float> ld{p, rhs};
+  MARCH2(K2);
   double acc = 0.0;
-  zmarch2<K2>(g, codes, ld, [&](int c, const L2LoadR<float>::Raw2& o, float2, float a0, float a1) {
+  march(L2LoadR<float>{p, rhs}, [&](int c, const L2LoadR<float>::Raw2& o, float2, float a0, float a1) {
     const float r0 = o.r.x - a0, r1 = o.r.y - a1;
     st2(res, c, r0, r1);
     acc += (double)r0 * (double)r0;
@@ -315,35 +445,22 @@ __global__ void __launch_bounds__(Z2T, FD3_ZMINB2_LIGHT) kx_dir_apply_dot(Geo g,
                                                                   float* __restrict__ q, Red red, Scalars* S) {
   KSTART();
   if (!S->active) return;
-  L2Dir<T> ld{z, din, S->dir_mode, S->beta};
+  MARCH2(K2);
   double acc = 0.0;
-  zmarch2<K2>(g, codes, ld, [&](int c, const typename L2Dir<T>::Raw2&, float2 pc, float a0, float a1) {
-    st2(dout, c, pc.x, pc.y);
-    st2(q, c, a0, a1);
-    acc += (double)pc.x * (double)a0;
-    acc += (double)pc.y * (double)a1;
-  });
+  march_dir(march, z, din, dout, q, S->dir_mode, S->beta, acc);
   zreduce_finish(acc, red, S, FIN_DQ);
 }
 
-// The two pre-sweeps from z = 0.
 template <int K2, class T>
 __global__ void __launch_bounds__(Z2T, FD3_ZMINB2) kx_fine_pre(Geo g, const unsigned short* __restrict__ codes,
                                                              const float* __restrict__ prec, const float* __restrict__ r,
                                                              T* __restrict__ z2, const Scalars* S, int gate) {
   KSTART();
   if (gate && !S->active) return;
-  const float rs = vscale<T>(S);
-  L2Z1<T> ld{prec, r, rs};
-  zmarch2<K2>(g, codes, ld, [&](int c, const typename L2Z1<T>::Raw2& o, float2 pc, float a0, float a1) {
-    float z0 = pc.x, z1 = pc.y;
-    if (o.m.x > 0.f) z0 += OMEGA * o.m.x * (rsc<T>(o.r.x, rs) - a0);
-    if (o.m.y > 0.f) z1 += OMEGA * o.m.y * (rsc<T>(o.r.y, rs) - a1);
-    Store<T>::st2(z2, c, z0, z1);
-  });
+  MARCH2(K2);
+  march_pre(march, prec, r, z2, vscale<T>(S));
 }
 
-// Prolongation + zeroing + first post-sweep (or the plain third sweep without coarse levels).
 template <int K2, class T>
 __global__ void __launch_bounds__(Z2T, FD3_ZMINB2) kx_fine_post1(Geo g, const unsigned short* __restrict__ codes,
                                                                const float* __restrict__ prec, const float* __restrict__ r,
@@ -351,18 +468,11 @@ __global__ void __launch_bounds__(Z2T, FD3_ZMINB2) kx_fine_post1(Geo g, const un
                                                                T* __restrict__ zout, const Scalars* S, int gate) {
   KSTART();
   if (gate && !S->active) return;
-  const float rs = vscale<T>(S);
-  L2Prolong<T> ld{zin, prec, r, as<T>(L.x), L.nx, L.ny, prolong};
-  zmarch2<K2>(g, codes, ld, [&](int c, const typename L2Prolong<T>::Raw2& o, float2 pc, float a0, float a1) {
-    float z0 = pc.x, z1 = pc.y;
-    if (o.m.x > 0.f) z0 += OMEGA * o.m.x * (rsc<T>(o.r.x, rs) - a0);
-    if (o.m.y > 0.f) z1 += OMEGA * o.m.y * (rsc<T>(o.r.y, rs) - a1);
-    Store<T>::st2(zout, c, z0, z1);
-  });
+  MARCH2(K2);
+  march_post1(march, prec, r, zin, L, prolong, zout, vscale<T>(S));
 }
 
-// Second post-sweep with r.z (FIN_RZ_PRIME or FIN_RZ_ITER).  The dot takes the z that is stored
-// (the value the direction update reads back) and the unscaled r.
+// Second post-sweep with r.z (FIN_RZ_PRIME or FIN_RZ_ITER).
 template <int K2, class T>
 __global__ void __launch_bounds__(Z2T, FD3_ZMINB2) kx_fine_post2_rz(Geo g, const unsigned short* __restrict__ codes,
                                                                   const float* __restrict__ prec,
@@ -371,23 +481,12 @@ __global__ void __launch_bounds__(Z2T, FD3_ZMINB2) kx_fine_post2_rz(Geo g, const
                                                                   Red red, Scalars* S, int gate, int op) {
   KSTART();
   if (gate && !S->active) return;
-  const float rs = vscale<T>(S);
-  L2Sweep<T> ld{zin, prec, r};
+  MARCH2(K2);
   double acc = 0.0;
-  zmarch2<K2>(g, codes, ld, [&](int c, const typename L2Sweep<T>::Raw2& o, float2 pc, float a0, float a1) {
-    float z0 = pc.x, z1 = pc.y;
-    if (o.m.x > 0.f) z0 += OMEGA * o.m.x * (rsc<T>(o.r.x, rs) - a0);
-    if (o.m.y > 0.f) z1 += OMEGA * o.m.y * (rsc<T>(o.r.y, rs) - a1);
-    Store<T>::st2(zout, c, z0, z1);
-    acc += (double)o.r.x * (double)Store<T>::rt(z0);
-    acc += (double)o.r.y * (double)Store<T>::rt(z1);
-  });
+  march_post2(march, prec, r, zin, zout, vscale<T>(S), acc);
   zreduce_finish(acc, red, S, op);
 }
 
-// Residual r - A z at every fine cell and its 8-child mean (restrict3, delta3d_multigrid.rs:258-272):
-// each thread's pair is one coarse cell's x children; the even rows sum the eight children, in the
-// reference's CHILDREN order, from the two layers kept in shared memory.
 template <int K2, class T>
 __global__ void __launch_bounds__(Z2T, FD3_ZMINB2_LIGHT) kx_fine_restrict(Geo g, const unsigned short* __restrict__ codes,
                                                                   const float* __restrict__ r,
@@ -395,35 +494,10 @@ __global__ void __launch_bounds__(Z2T, FD3_ZMINB2_LIGHT) kx_fine_restrict(Geo g,
                                                                   int gate) {
   KSTART();
   if (gate && !S->active) return;
-  __shared__ __align__(8) float tr[2][Z2Y][Z2X];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const ZTile2 t = ztile2<K2>(g);
-  const int nxny = g.nx * g.ny;
-  const float rs = vscale<T>(S);
-  L2LoadR<T> ld{z, r};
-  zmarch2<K2>(
-      g, codes, ld,
-      [&](int c, const typename L2LoadR<T>::Raw2& o, float2, float a0, float a1) {
-        *reinterpret_cast<float2*>(&tr[(c / nxny) & 1][ty][2 * tx]) =
-            make_float2(rsc<T>(o.r.x, rs) - a0, rsc<T>(o.r.y, rs) - a1);
-      },
-      [&](int k) {
-        if (k & 1) {
-          __syncthreads();  // the epilogue's tr writes before the reads below
-          if (t.inside && !(ty & 1)) {
-            float sum = 0.f;
-            sum += tr[0][ty][2 * tx];
-            sum += tr[0][ty][2 * tx + 1];
-            sum += tr[0][ty + 1][2 * tx];
-            sum += tr[0][ty + 1][2 * tx + 1];
-            sum += tr[1][ty][2 * tx];
-            sum += tr[1][ty][2 * tx + 1];
-            sum += tr[1][ty + 1][2 * tx];
-            sum += tr[1][ty + 1][2 * tx + 1];
-            Store<T>::st(as<T>(L.r), ((k >> 1) * L.ny + (t.j >> 1)) * L.nx + (t.i0 >> 1), 0.125f * sum);
-          }
-        }
-      });
+  MARCH2(K2);
+  __shared__ __align__(8) ZResid2 tr_[2];
+  march_restrict(March2<BlockSync>{g, codes, march.t, march.tx, march.ty, march.sbuf, tr_, BlockSync()}, r, z, L,
+                 vscale<T>(S));
 }
 
 }  // namespace fd3
