@@ -73,6 +73,20 @@ struct ClusterTeam {
   __device__ __forceinline__ void sync() const { cooperative_groups::this_cluster().sync(); }
 };
 
+// Division by a number known for a whole patch: the quotient from the high product, one too small at most.
+struct FastDiv {
+  unsigned d, m;
+  __device__ __forceinline__ void set(int by) {
+    d = (unsigned)by;
+    m = by > 1 ? (unsigned)(0x100000000ull / d) : 0xffffffffu;
+  }
+  __device__ __forceinline__ int div(int c) const {
+    const unsigned q = __umulhi((unsigned)c, m);
+    return (int)(q + ((unsigned)c - q * d >= d ? 1u : 0u));
+  }
+};
+constexpr int BATCH_LEVELS = 16;
+
 // Shared state of one CTA.
 struct BatchShared {
   Scalars S;                     // this CTA's copy of the patch's scalars
@@ -81,6 +95,12 @@ struct BatchShared {
   double warp[32][6];
   unsigned long long hwarp[32];
   BatchPatch P;
+  int ktop;                             // layers of the patch up to its highest wet cell
+  FastDiv nx[BATCH_LEVELS + 1], ny[BATCH_LEVELS + 1];  // of the patch, then of its levels
+  Lev lev[BATCH_LEVELS];
+  int tail_first, ntail;                // the levels the first CTA solves in shared memory (ntail = 0: none)
+  Lev tail_levs[TAIL_REG_LEVELS];
+  TailShared tail;
 };
 
 // The cluster-wide reduction of K per-thread values (sums, or maxima where `mx` has bit k set)
@@ -169,121 +189,219 @@ __device__ __forceinline__ void strided_cells(const ClusterTeam& tm, int n, F f)
 // barriers instead of cluster barriers (the single-volume path's coarse tail does the same).
 constexpr int BATCH_CTA_LEVEL_CELLS = 4096;
 
-// v_cycle3 (delta3d_multigrid.rs:393-429) of P.res into P.z with res.z at its end (op), the
-// one-cell-per-thread passes of the library and the coarse tail over every level.
+// A.P at wet cell c: P(n, f) yields the operand at its neighbour n across face f.  A plain row (the bulk, walls and
+// obstacles' flat sides) needs neither the cell's coordinates nor any coefficient; the others find theirs.
+// (The others are a call: inlined in every phase they would take the registers of the plain ones, and a spilled
+// register is read from L2 after each cluster barrier.)
+__device__ __noinline__ float batch_row_general(const BatchShared& sh, unsigned code, int c, float pc, float xm, float xp,
+                                                float ym, float yp, float zm, float zp) {
+  const Geo& g = sh.P.g;
+  const int t = sh.nx[0].div(c), k = sh.ny[0].div(t);
+  return row_general(g, code, c - t * g.nx, t - k * g.ny, k, pc, xm, xp, ym, yp, zm, zp);
+}
+template <class P>
+__device__ __forceinline__ float batch_row(const BatchShared& sh, unsigned code, int c, float pc, P p) {
+  const Geo& g = sh.P.g;
+  const int nx = g.nx, nxny = nx * g.ny;
+  if (rc_plain(code)) {
+    float acc = 0.f;
+    acc += (code & (1u << 1)) ? pc - p(c - 1, 0) : 0.f;
+    acc += (code & (1u << 3)) ? pc - p(c + 1, 1) : 0.f;
+    acc += (code & (1u << 5)) ? pc - p(c - nx, 2) : 0.f;
+    acc += (code & (1u << 7)) ? pc - p(c + nx, 3) : 0.f;
+    acc += (code & (1u << 9)) ? pc - p(c - nxny, 4) : 0.f;
+    acc += (code & (1u << 11)) ? pc - p(c + nxny, 5) : 0.f;
+    return acc * g.inv;
+  }
+  return batch_row_general(sh, code, c, pc, face_state(code, 0) == 1u ? p(c - 1, 0) : 0.f,
+                           face_state(code, 1) == 1u ? p(c + 1, 1) : 0.f, face_state(code, 2) == 1u ? p(c - nx, 2) : 0.f,
+                           face_state(code, 3) == 1u ? p(c + nx, 3) : 0.f, face_state(code, 4) == 1u ? p(c - nxny, 4) : 0.f,
+                           face_state(code, 5) == 1u ? p(c + nxny, 5) : 0.f);
+}
+// The cells of a level below the air, and row_sums of its active cell c with values x (level_row_code).
+__device__ __forceinline__ int batch_level_cells(const BatchShared& sh, int l, const Lev& L) {
+  return L.nx * L.ny * min(L.nz, (sh.ktop + (2 << l) - 1) >> (l + 1));
+}
+__device__ __noinline__ float batch_level_row_general(const BatchShared& sh, int l, const Lev& L, unsigned code, int c,
+                                                      const float* x) {
+  const int t = sh.nx[l + 1].div(c), k = sh.ny[l + 1].div(t);
+  return level_row_code(L, code, c - t * L.nx, t - k * L.ny, k, c, Load{x});
+}
+__device__ __forceinline__ float batch_level_row(const BatchShared& sh, int l, const Lev& L, unsigned code, int c,
+                                                 const float* x) {
+  if (!rc_plain(code)) return batch_level_row_general(sh, l, L, code, c, x);
+  return level_row_code(L, code, 0, 0, 0, c, Load{x});  // a plain row needs no coordinates
+}
+
+// coarse_cycle3's way down over levels first .. stop - 1 and up again (tail_down_t, tail_up_t), from the row codes.
+template <class Team>
+__device__ __forceinline__ void batch_sweep(const Team& tm, const BatchShared& sh, int l, const Lev& L, const float* xin,
+                                            float* xout, bool zero_in) {
+  const int n = batch_level_cells(sh, l, L);
+  for (int c = tm.rank(); c < n; c += tm.size()) {
+    const float dg = L.diag[c], r = L.r[c];
+    float x = 0.f;
+    if (zero_in) {
+      if (dg > 0.f) x = 0.f + OMEGA * (r - 0.f) / dg;
+    } else {
+      x = xin[c];
+      if (dg > 0.f) x += OMEGA * (r - batch_level_row(sh, l, L, L.code[c], c, xin)) / dg;
+    }
+    xout[c] = x;
+  }
+  tm.sync();
+}
+template <class Team>
+__device__ __forceinline__ void batch_down(const Team& tm, const BatchShared& sh, int first, int stop, int last) {
+  for (int l = first; l < stop; ++l) {
+    const Lev& L = sh.lev[l];
+    const int sweeps = l == last ? 8 : 2;  // COARSE_SWEEPS_3D, PRE_SWEEPS_3D
+    for (int s = 0; s < sweeps; ++s) batch_sweep(tm, sh, l, L, (s & 1) ? L.x2 : L.x, (s & 1) ? L.x : L.x2, s == 0);
+    if (l < last) {
+      const Lev& C = sh.lev[l + 1];
+      const int n = batch_level_cells(sh, l + 1, C);
+      for (int q = tm.rank(); q < n; q += tm.size()) {
+        const int t = sh.nx[l + 2].div(q), ck = sh.ny[l + 2].div(t), ci = q - t * C.nx, cj = t - ck * C.ny;
+        float s = 0.f;
+#pragma unroll 1
+        for (int e = 0; e < 8; ++e) {
+          const int c = ((2 * ck + (e >> 2)) * L.ny + 2 * cj + ((e >> 1) & 1)) * L.nx + 2 * ci + (e & 1);
+          const unsigned code = L.code[c];
+          s += L.r[c] - ((code & RC_WET) ? batch_level_row(sh, l, L, code, c, L.x) : 0.f);
+        }
+        C.r[q] = 0.125f * s;
+      }
+      tm.sync();
+    }
+  }
+}
+template <class Team>
+__device__ __forceinline__ void batch_up(const Team& tm, const BatchShared& sh, int first, int from) {
+  for (int l = from; l >= first; --l) {
+    const Lev &L = sh.lev[l], &C = sh.lev[l + 1];
+    const int n = batch_level_cells(sh, l, L);
+    for (int c = tm.rank(); c < n; c += tm.size()) {
+      const int t = sh.nx[l + 1].div(c), k = sh.ny[l + 1].div(t), i = c - t * L.nx, j = t - k * L.ny;
+      L.x[c] += C.x[((k >> 1) * C.ny + (j >> 1)) * C.nx + (i >> 1)];
+    }
+    tm.sync();
+    batch_sweep(tm, sh, l, L, L.x, L.x2, false);
+    batch_sweep(tm, sh, l, L, L.x2, L.x, false);
+  }
+}
+
+// v_cycle3 (delta3d_multigrid.rs:393-429) of P.res into P.z with res.z at its end (op).  z2 holds the first pre-sweep
+// w prec r of every cell (batch_first_sweep, or the update, writes it).
 __device__ __forceinline__ void batch_vcycle(const ClusterTeam& tm, BatchShared& sh, int& ph, int op) {
   const BatchPatch& P = sh.P;
   const Geo& g = P.g;
-  const float* __restrict__ prec = P.prec;
-  const float* __restrict__ r = P.res;
-  const unsigned short* __restrict__ codes = P.codes;
-  float* __restrict__ z = P.z;
-  float* __restrict__ z2 = P.z2;
-  // the two pre-sweeps from z = 0 (k_fine_pre): z1 = w prec r recomputed at the stencil points
-  {
-    auto Z1 = [&](int n) {
-      float m = prec[n];
-      return m > 0.f ? 0.f + OMEGA * m * (r[n] - 0.f) : 0.f;
-    };
-    strided_cells(tm, g.n, [&](int c) {
-      float m = prec[c];
-      float zc = Z1(c);
-      if (m > 0.f) {
-        int i, j, k; cell_ijk(g, c, i, j, k);
-        zc += OMEGA * m * (r[c] - apply_code(g, (unsigned)codes[c], i, j, k, c, Z1));
-      }
-      z[c] = zc;
+  const float* prec = P.prec;
+  const float* r = P.res;
+  const unsigned short* codes = P.codes;
+  float* z = P.z;
+  float* z2 = P.z2;
+  const int ntop = g.nx * g.ny * sh.ktop;
+  // a sweep from `in` into `out` (k_fine_pre's second, k_fine_post2_rz's)
+  auto sweep = [&](const float* in, float* out, auto done) {
+    strided_cells(tm, ntop, [&](int c) {
+      const float m = prec[c], rc = r[c];
+      const unsigned code = codes[c];
+      float zc = in[c];
+      if (m > 0.f) zc += OMEGA * m * (rc - batch_row(sh, code, c, zc, [&](int n, int) { return in[n]; }));
+      out[c] = zc;
+      done(rc, zc);
     });
-    tm.sync();
-  }
+  };
+  sweep(z2, z, [](float, float) {});
+  tm.sync();
   const bool levels = P.nlev > 0;
+  const int last = P.nlev - 1;
   if (levels) {  // restrict3 of r - A z (k_fine_restrict_c), then the coarse levels
-    const Lev L = P.lev[0];
-    Load Z{z};
-    float* __restrict__ lr = L.r;
-    strided_cells(tm, L.n, [&](int qi) {
-      int ci = qi % L.nx, t = qi / L.nx, cj = t % L.ny, ck = t / L.ny;
+    const Lev& L = sh.lev[0];
+    const int n = batch_level_cells(sh, 0, L);
+    strided_cells(tm, n, [&](int qi) {
+      const int t = sh.nx[1].div(qi), ck = sh.ny[1].div(t), ci = qi - t * L.nx, cj = t - ck * L.ny;
       float s = 0.f;
-#pragma unroll
+#pragma unroll 1
       for (int e = 0; e < 8; ++e) {
-        int i = 2 * ci + (e & 1), j = 2 * cj + ((e >> 1) & 1), k = 2 * ck + (e >> 2);
-        int c = (k * g.ny + j) * g.nx + i;
-        unsigned code = codes[c];
-        float az = (code & RC_WET) ? apply_code(g, code, i, j, k, c, Z) : 0.f;
-        s += r[c] - az;
+        const int c = ((2 * ck + (e >> 2)) * g.ny + 2 * cj + ((e >> 1) & 1)) * g.nx + 2 * ci + (e & 1);
+        const unsigned code = codes[c];
+        s += r[c] - ((code & RC_WET) ? batch_row(sh, code, c, z[c], [&](int m, int) { return z[m]; }) : 0.f);
       }
-      lr[qi] = 0.125f * s;
+      L.r[qi] = 0.125f * s;
     });
     tm.sync();
-    // the small levels from `t` down are solved by the first CTA alone
-    const int last = P.nlev - 1;
+    // the small levels from `t` down are solved by the first CTA alone, the smallest in its shared memory
     int t = P.nlev;
-    while (t > 0 && P.lev[t - 1].n <= BATCH_CTA_LEVEL_CELLS) --t;
-    if (t >= P.nlev) {
-      tail_run_t(tm, P.lev, 0, last);
-    } else {
-      tail_down_t(tm, P.lev, 0, t, last);
-      if (cooperative_groups::this_cluster().block_rank() == 0) tail_run_t(BlockTeam{}, P.lev, t, last);
+    while (t > 0 && sh.lev[t - 1].n <= BATCH_CTA_LEVEL_CELLS) --t;
+    batch_down(tm, sh, 0, t, last);
+    if (t < P.nlev) {
+      if (cooperative_groups::this_cluster().block_rank() == 0) {
+        const int tf = sh.ntail > 0 ? sh.tail_first : P.nlev;
+        batch_down(BlockTeam{}, sh, t, tf, last);
+        if (sh.ntail > 0) {
+          const Lev& T = sh.tail_levs[0];
+          if ((int)threadIdx.x < T.n) sh.tail.R[threadIdx.x] = T.r[threadIdx.x];
+          __syncthreads();
+          tail_cycle(sh.tail_levs, sh.ntail, sh.tail);
+          if ((int)threadIdx.x < T.n) T.x[threadIdx.x] = sh.tail.XF[threadIdx.x];
+          __syncthreads();
+        }
+        batch_up(BlockTeam{}, sh, t, min(tf, last) - 1);
+      }
       tm.sync();
-      tail_up_t(tm, P.lev, 0, t - 1);
     }
+    batch_up(tm, sh, 0, min(t, last) - 1);
   }
-  // prolongation, dry cells zeroed, first post-sweep (k_fine_post1)
-  {
-    const Lev L = levels ? P.lev[0] : Lev{};
-    const float* __restrict__ zin = z;
-    const float* __restrict__ lx = L.x;
-    auto ZP = [&](int n) {
-      if (!levels) return zin[n];
-      int i = n % g.nx, t = n / g.nx, j = t % g.ny, k = t / g.ny;
-      float v = zin[n] + lx[((k >> 1) * L.ny + (j >> 1)) * L.nx + (i >> 1)];
-      return prec[n] == 0.f ? 0.f : v;
-    };
-    strided_cells(tm, g.n, [&](int c) {
-      float m = prec[c];
-      float zc = ZP(c);
+  // prolongation, dry cells zeroed, first post-sweep (k_fine_post1); a neighbour that the row reads is never dry
+  if (levels) {
+    const Lev& L = sh.lev[0];
+    const float* lx = L.x;
+    strided_cells(tm, ntop, [&](int c) {
+      const float m = prec[c], rc = r[c];
+      const unsigned code = codes[c];
+      float zc = 0.f;
       if (m > 0.f) {
-        int i, j, k; cell_ijk(g, c, i, j, k);
-        zc += OMEGA * m * (r[c] - apply_code(g, (unsigned)codes[c], i, j, k, c, ZP));
+        const int t = sh.nx[0].div(c), k = sh.ny[0].div(t), i = c - t * g.nx, j = t - k * g.ny;
+        const int at = ((k >> 1) * L.ny + (j >> 1)) * L.nx + (i >> 1);
+        const int step[6] = {(i & 1) ? 0 : -1, (i & 1) ? 1 : 0, (j & 1) ? 0 : -L.nx, (j & 1) ? L.nx : 0,
+                             (k & 1) ? 0 : -L.nx * L.ny, (k & 1) ? L.nx * L.ny : 0};
+        zc = z[c] + lx[at];
+        zc += OMEGA * m * (rc - batch_row(sh, code, c, zc, [&](int n, int f) { return z[n] + lx[at + step[f]]; }));
       }
       z2[c] = zc;
     });
-    tm.sync();
+  } else {
+    sweep(z, z2, [](float, float) {});
   }
+  tm.sync();
   // the last post-sweep with r.z (k_fine_post2_rz)
   double acc[1] = {0.0};
-  {
-    Load Z{z2};
-    strided_cells(tm, g.n, [&](int c) {
-      float m = prec[c];
-      float rc = r[c];
-      float zc = z2[c];
-      if (m > 0.f) {
-        int i, j, k; cell_ijk(g, c, i, j, k);
-        zc += OMEGA * m * (rc - apply_code(g, (unsigned)codes[c], i, j, k, c, Z));
-      }
-      z[c] = zc;
-      acc[0] += (double)rc * (double)zc;
-    });
-  }
+  sweep(z2, z, [&](float rc, float zc) { acc[0] += (double)rc * (double)zc; });
   crew_reduce<1>(sh, ph, acc, 0u, nullptr);
   crew_apply(sh, acc[0], op);
+}
+// The first pre-sweep from z = 0, into z2, of the prime; an iteration's update writes its own.
+__device__ __forceinline__ float batch_z1(float m, float r) { return m > 0.f ? 0.f + OMEGA * m * (r - 0.f) : 0.f; }
+__device__ __forceinline__ void batch_first_sweep(const ClusterTeam& tm, const BatchShared& sh) {
+  const BatchPatch& P = sh.P;
+  const int ntop = P.g.nx * P.g.ny * sh.ktop;
+  for (int c = tm.rank(); c < ntop; c += tm.size()) P.z2[c] = batch_z1(P.prec[c], P.res[c]);
+  tm.sync();
 }
 
 // res = rhs - A p with res.res (FIN_RR0 or FIN_ACTUAL).
 __device__ __forceinline__ void batch_residual(const ClusterTeam& tm, BatchShared& sh, int& ph, int op) {
   const BatchPatch& P = sh.P;
   const Geo& g = P.g;
-  const unsigned short* __restrict__ codes = P.codes;
-  const float* __restrict__ rhs = P.rhs;
-  float* __restrict__ res = P.res;
-  Load Pl{P.p};
+  const unsigned short* codes = P.codes;
+  const float* rhs = P.rhs;
+  const float* p = P.p;
+  float* res = P.res;
   double acc[1] = {0.0};
-  strided_cells(tm, g.n, [&](int c) {
-    unsigned code = codes[c];
-    float ap = 0.f;
-    if (code & RC_WET) { int i, j, k; cell_ijk(g, c, i, j, k); ap = apply_code(g, code, i, j, k, c, Pl); }
-    const float rv = rhs[c] - ap;
+  strided_cells(tm, g.nx * g.ny * sh.ktop, [&](int c) {
+    const unsigned code = codes[c];
+    const float rv = rhs[c] - ((code & RC_WET) ? batch_row(sh, code, c, p[c], [&](int n, int) { return p[n]; }) : 0.f);
     res[c] = rv;
     acc[0] += (double)rv * (double)rv;
   });
@@ -296,21 +414,21 @@ __device__ __forceinline__ void batch_residual(const ClusterTeam& tm, BatchShare
 __device__ __forceinline__ void batch_iteration(const ClusterTeam& tm, BatchShared& sh, int& ph, int parity) {
   const BatchPatch& P = sh.P;
   const Geo& g = P.g;
-  const float* __restrict__ din = parity ? P.dir2 : P.dir;
-  float* __restrict__ dout = parity ? P.dir : P.dir2;
-  const unsigned short* __restrict__ codes = P.codes;
-  float* __restrict__ q = P.q;
+  const float* din = parity ? P.dir2 : P.dir;
+  float* dout = parity ? P.dir : P.dir2;
+  const unsigned short* codes = P.codes;
+  float* q = P.q;
+  const int ntop = g.nx * g.ny * sh.ktop;
   {  // d = z (+ beta d), q = A d, d.q, alpha (k_dir_apply_dot)
     const int mode = sh.S.dir_mode;
     const float beta = sh.S.beta;
-    const float* __restrict__ z = P.z;
-    auto D = [&](int n) { return mode ? z[n] + beta * din[n] : z[n]; };
+    const float* z = P.z;
+    auto D = [&](int n, int) { return mode ? z[n] + beta * din[n] : z[n]; };
     double acc[1] = {0.0};
-    strided_cells(tm, g.n, [&](int c) {
-      const float dc = D(c);
+    strided_cells(tm, ntop, [&](int c) {
       const unsigned code = codes[c];
-      float qc = 0.f;
-      if (code & RC_WET) { int i, j, k; cell_ijk(g, c, i, j, k); qc = apply_code(g, code, i, j, k, c, D); }
+      const float dc = (code & RC_WET) ? D(c, 0) : 0.f;
+      const float qc = (code & RC_WET) ? batch_row(sh, code, c, dc, D) : 0.f;
       dout[c] = dc;
       q[c] = qc;
       acc[0] += (double)dc * (double)qc;
@@ -319,15 +437,18 @@ __device__ __forceinline__ void batch_iteration(const ClusterTeam& tm, BatchShar
     crew_apply(sh, acc[0], FIN_DQ);
   }
   if (!sh.S.active) return;
-  {  // p += alpha d, r -= alpha q, r.r (k_update_rn)
+  {  // p += alpha d, r -= alpha q, r.r (k_update_rn), and the next V-cycle's first sweep
     const float alpha = sh.S.alpha;
-    float* __restrict__ p = P.p;
-    float* __restrict__ res = P.res;
+    float* p = P.p;
+    float* res = P.res;
+    const float* prec = P.prec;
+    float* z2 = P.z2;
     double acc[1] = {0.0};
-    strided_cells(tm, g.n, [&](int c) {
+    strided_cells(tm, ntop, [&](int c) {
       p[c] += alpha * dout[c];
       const float rn = res[c] - alpha * q[c];
       res[c] = rn;
+      z2[c] = batch_z1(prec[c], rn);
       acc[0] += (double)rn * (double)rn;
     });
     crew_reduce<1>(sh, ph, acc, 0u, nullptr);
@@ -413,6 +534,33 @@ __device__ __forceinline__ void batch_project_one(const ClusterTeam& tm, BatchSh
     if (P.reset_p) P.p[c] = 0.f;
   }
   crew_reduce<1>(sh, ph, bad, 1u, nullptr);
+  // the layers below the air (the columns' highest wet cells, by wet3's height test), the divisors, the tail's levels
+  double top[1] = {0.0};
+  for (int c = tm.rank(); c < g.nx * g.ny; c += tm.size()) {
+    if (!col_active(g, c % g.nx, c / g.nx)) continue;
+    int lo = 0, hi = g.nz;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (((float)mid + 0.5f) * g.dx < g.eta[c]) lo = mid + 1; else hi = mid;
+    }
+    top[0] = fmax(top[0], (double)lo);
+  }
+  crew_reduce<1>(sh, ph, top, 1u, nullptr);
+  if (threadIdx.x == 0) {
+    sh.ktop = min(((int)top[0] + 1) & ~1, g.nz);
+    int t = P.nlev;
+    while (t > 0 && P.lev[t - 1].n <= TAIL_REG_THREADS) --t;
+    sh.tail_first = t;
+    sh.ntail = P.nlev - t <= TAIL_REG_LEVELS ? P.nlev - t : 0;
+  }
+  if ((int)threadIdx.x <= P.nlev) {
+    sh.nx[threadIdx.x].set(threadIdx.x == 0 ? g.nx : P.lev[threadIdx.x - 1].nx);
+    sh.ny[threadIdx.x].set(threadIdx.x == 0 ? g.ny : P.lev[threadIdx.x - 1].ny);
+    if (threadIdx.x > 0) sh.lev[threadIdx.x - 1] = P.lev[threadIdx.x - 1];
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < sh.ntail) sh.tail_levs[threadIdx.x] = P.lev[sh.tail_first + threadIdx.x];
+  __syncthreads();
   BatchResult res{};
   if (bad[0] > 0.0) {
     res.status = FD3_ERR_NOT_FINITE;
@@ -444,9 +592,11 @@ __device__ __forceinline__ void batch_project_one(const ClusterTeam& tm, BatchSh
       for (int c = tm.rank(); c < C.n; c += tm.size()) {
         C.diag[c] = level_diag_at(C, c);
         C.code[c] = (unsigned short)level_codes_at(C, c);
+        level_zero_inactive(C, c, 0);
       }
       tm.sync();
     }
+    if (sh.ntail > 0 && cooperative_groups::this_cluster().block_rank() == 0) tail_rows(sh.tail_levs, sh.ntail, sh.tail);
     batch_residual(tm, sh, ph, FIN_RR0);
     res.status = sh.S.status;
   }
@@ -470,6 +620,7 @@ __device__ __forceinline__ void batch_project_one(const ClusterTeam& tm, BatchSh
       const unsigned before = it;
       if (b2 > 0 && (rr > tolb2 || rr > phys) && it < P.max_iters) {
         if (!primed) {
+          batch_first_sweep(tm, sh);
           batch_vcycle(tm, sh, ph, FIN_RZ_PRIME);
           primed = true;
         }
@@ -527,6 +678,7 @@ __device__ __forceinline__ void batch_project_one(const ClusterTeam& tm, BatchSh
         since = 0;
       }
       rr = actual;
+      batch_first_sweep(tm, sh);
       batch_vcycle(tm, sh, ph, FIN_RZ_PRIME);
     }
     if (!res.status) {
