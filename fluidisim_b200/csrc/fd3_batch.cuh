@@ -565,13 +565,11 @@ __device__ __forceinline__ void batch_project_one(const ClusterTeam& tm, BatchSh
   if (bad[0] > 0.0) {
     res.status = FD3_ERR_NOT_FINITE;
   } else {
-    // divergence of us (k_divergence)
-    for (int c = tm.rank(); c < g.n; c += tm.size()) P.rhs[c] = divergence_at(g, P.us, P.vs, P.ws, c);
-    tm.sync();
-    // rhs_mobile3 with b.b, the row codes, p = 0 on the dry cells (k_rhs_b2)
+    // the divergence of us and rhs_mobile3 with b.b, the row codes, p = 0 on the dry cells (k_rhs_b2)
     double b2v[1] = {0.0};
     for (int c = tm.rank(); c < g.n; c += tm.size()) {
-      const float b = rhs_b2_at(g, P.scale, P.rhs, P.prec, P.codes, P.p, c);
+      const float b = rhs_b2_at(g, P.scale, [&] { return divergence_at(g, P.us, P.vs, P.ws, c); }, P.rhs, P.prec, P.codes,
+                                P.p, c);
       b2v[0] += (double)b * (double)b;
     }
     crew_reduce<1>(sh, ph, b2v, 0u, nullptr);

@@ -364,6 +364,10 @@ __device__ __forceinline__ void block_fmax3_atomic(float a, float b, float c, fl
 #ifndef FD3_SETUP_MINB
 #define FD3_SETUP_MINB 8
 #endif
+// The assembly forms the divergence as well, which takes more registers (40 at six CTAs per SM).
+#ifndef FD3_RHS_MINB
+#define FD3_RHS_MINB 6
+#endif
 constexpr int CM_X = 32, CM_Y = 8, CM_K = 8;
 inline int cm_blocks(int nx, int ny, int nz) {
   return ((nx + CM_X - 1) / CM_X) * ((ny + CM_Y - 1) / CM_Y) * ((nz + CM_K - 1) / CM_K);
@@ -1744,11 +1748,12 @@ __global__ void k_loop_cond(cudaGraphConditionalHandle handle, Scalars* S) {
 // ------------------------------------------------------------------------------------------------
 // Set-up reductions with the in-kernel finish.
 
-// One row of rhs_mobile3 (delta3d_mobile.rs:215-241): rhs and prec of cell c (the divergence in
-// rhs is replaced by the right-hand side), its row code into codes and p = 0 on a dry cell when
-// those are not null; returns b.
-__device__ __forceinline__ float rhs_b2_at(const Geo& g, float scale, float* __restrict__ rhs, float* __restrict__ prec,
-                                           unsigned short* __restrict__ codes, float* __restrict__ pdry, int c) {
+// One row of rhs_mobile3 (delta3d_mobile.rs:215-241): rhs and prec of cell c, whose divergence is div(), its row
+// code into codes and p = 0 on a dry cell when those are not null; returns b.
+template <class Div>
+__device__ __forceinline__ float rhs_b2_at(const Geo& g, float scale, Div div, float* __restrict__ rhs,
+                                           float* __restrict__ prec, unsigned short* __restrict__ codes,
+                                           float* __restrict__ pdry, int c) {
   int i, j, k; cell_ijk(g, c, i, j, k);
   if (!wet3(g, i, j, k)) {
     rhs[c] = 0.f; prec[c] = 0.f;
@@ -1757,7 +1762,7 @@ __device__ __forceinline__ float rhs_b2_at(const Geo& g, float scale, float* __r
     return 0.f;
   }
   RowE row[6]; mobile_row(g, i, j, k, row);
-  float b = scale * rhs[c];
+  float b = scale * div();
   float diag = 0.f;
 #pragma unroll
   for (int f = 0; f < 6; ++f) {
@@ -1790,13 +1795,20 @@ struct WorkVectors {
 // rhs_mobile3 (delta3d_mobile.rs:215-241) with b.b (FIN_B2) when `reduce`.
 // With `codes` not null, the same pass also writes each cell's row code (row_code_of the same
 // row; 0 for a dry cell); with `pdry` not null it zeroes that pressure on the dry cells.
+// The divergence is the one in rhs, or, when vel.u is not null, that of those faces, formed here (a pass over the
+// volume less, and none at all for the air).
+struct Faces {
+  const float *u, *v, *w;
+};
 template <int MODE>
-__global__ void __launch_bounds__(TPB, FD3_SETUP_MINB) k_rhs_b2(Geo g, float scale, float* __restrict__ rhs, float* __restrict__ prec,
-                                                Red red, Scalars* S, int reduce, unsigned short* __restrict__ codes,
-                                                float* __restrict__ pdry, WorkVectors work) {
+__global__ void __launch_bounds__(TPB, FD3_RHS_MINB) k_rhs_b2(Geo g, float scale, Faces vel, float* __restrict__ rhs,
+                                                            float* __restrict__ prec, Red red, Scalars* S, int reduce,
+                                                            unsigned short* __restrict__ codes, float* __restrict__ pdry,
+                                                            WorkVectors work) {
   KSTART();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const float b = c < g.n ? rhs_b2_at(g, scale, rhs, prec, codes, pdry, c) : 0.f;
+  auto div = [&] { return vel.u ? divergence_at(g, vel.u, vel.v, vel.w, c) : rhs[c]; };
+  const float b = c < g.n ? rhs_b2_at(g, scale, div, rhs, prec, codes, pdry, c) : 0.f;
   if (work.v[0] && c < g.n && prec[c] == 0.f) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) work.v[q][c] = 0.f;

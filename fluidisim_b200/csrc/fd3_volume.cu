@@ -14,6 +14,7 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <limits>
 #include <mutex>
 #include <new>
@@ -178,6 +179,8 @@ struct fd3_volume {
   fd3_report refused{};
   unsigned long long launches = 0;
   std::vector<void*> allocations;
+  char* arena = nullptr;  // what is left of the last shared chunk (dalloc)
+  size_t arena_left = 0;
   // opt-in per-kernel timing: events around every launch, collected at each synchronisation
   bool prof = false;
   std::vector<cudaEvent_t> ev_pool;
@@ -269,12 +272,57 @@ struct fd3_volume {
 
 namespace {
 
+// Zeroed device memory of the volume's.  Arrays below kArenaMax share chunks of kArenaChunk bytes: a volume has some
+// fifty arrays, a cudaMalloc takes 0.2 ms and more, and a batch configures hundreds of small volumes.
+constexpr size_t kArenaMax = 1 << 20, kArenaChunk = 4 << 20;
 int dalloc(fd3_volume* V, float** ptr, size_t count) {
-  void* q = nullptr;
-  CK(cudaMalloc(&q, count * sizeof(float) + 16));
-  CK(cudaMemsetAsync(q, 0, count * sizeof(float) + 16, V->stream));
-  V->allocations.push_back(q);
-  *ptr = (float*)q;
+  const size_t bytes = (count * sizeof(float) + 16 + 255) & ~(size_t)255;
+  const bool share = bytes < kArenaMax;
+  if (!share || V->arena_left < bytes) {
+    void* q = nullptr;
+    const size_t size = share ? kArenaChunk : bytes;
+    CK(cudaMalloc(&q, size));
+    V->allocations.push_back(q);
+    CK(cudaMemsetAsync(q, 0, size, V->stream));
+    if (!share) {
+      *ptr = (float*)q;
+      return FD3_OK;
+    }
+    V->arena = (char*)q;
+    V->arena_left = size;
+  }
+  *ptr = (float*)V->arena;
+  V->arena += bytes;
+  V->arena_left -= bytes;
+  return FD3_OK;
+}
+
+// The CTAs of the cooperative launches (k_cg_loop, k_mg_loop) on a device, one per SM; 0 where they are not to be had.
+// Asked once per device (it and the kernels' shared-memory attributes belong to the device, not to a volume).
+int cooperative_ctas(int device, int* ctas) {
+  static std::mutex m;
+  static std::vector<int> known;  // -1: not asked
+  std::lock_guard<std::mutex> lock(m);
+  if ((int)known.size() <= device) known.resize(device + 1, -1);
+  if (known[device] < 0) {
+    int sms = 0, coop = 0, least = 1, resident = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+    CK(cudaFuncSetAttribute(k_cg_loop<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(4)));
+    CK(cudaFuncSetAttribute(k_cg_loop<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(8)));
+    CK(cudaFuncSetAttribute(k_cg_loop<GRID_MAX_CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)cg_smem(GRID_MAX_CELLS)));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_cg_loop<GRID_MAX_CELLS>, GRID_THREADS,
+                                                     cg_smem(GRID_MAX_CELLS)));
+    least = std::min(least, resident);
+    for (auto k : {k_mg_loop<float>, k_mg_loop<__half>}) {
+      CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MgShared)));
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k, MG_THREADS, sizeof(MgShared)));
+      least = std::min(least, resident);
+    }
+    known[device] = coop && least >= 1 ? std::min(sms, GRID_MAX_CTAS) : 0;
+  }
+  *ctas = known[device];
   return FD3_OK;
 }
 
@@ -1076,15 +1124,15 @@ int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_r
   const bool ord = V->ord();
   Geo G = V->geo();
   LAUNCH_G(V, k_reset_scalars, 1, 1, V->dS, vscale_k(V));
-  LAUNCH(V, k_divergence, V->n, G, (const float*)V->us, (const float*)V->vs, (const float*)V->ws, V->rhs);
   if (V->linear) {
+    LAUNCH(V, k_divergence, V->n, G, (const float*)V->us, (const float*)V->vs, (const float*)V->ws, V->rhs);
     const int jacobi = V->cut && V->precondition_cut && V->ny > 1;  // delta3d.rs:1091
     DISPATCH(V, k_rhs_linear, V->n, G, scale, jacobi, V->rhs, V->prec, V->red(), V->dS);
     LAUNCH(V, k_row_codes_linear, V->n, G, V->codes);
     CK(cudaMemsetAsync(V->p, 0, (size_t)V->n * sizeof(float), V->stream));
   } else {
     // the assembly also zeroes p on the dry cells (delta3d_mobile.rs:486-495)
-    DISPATCH(V, k_rhs_b2, V->n, G, scale, V->rhs, V->prec, V->red(), V->dS, 1, V->codes, V->p,
+    DISPATCH(V, k_rhs_b2, V->n, G, scale, Faces{V->us, V->vs, V->ws}, V->rhs, V->prec, V->red(), V->dS, 1, V->codes, V->p,
              V->skip_air ? WorkVectors{{V->res, V->dir, V->dir2, V->tmp}} : WorkVectors{});
     if (V->skip_air)
       LAUNCH_G(V, k_tile_tops, ((V->nx + TILE_X - 1) / TILE_X) * ((V->ny + TILE_Y - 1) / TILE_Y), TILE_X * TILE_Y, G,
@@ -1233,11 +1281,67 @@ int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd
 }
 
 // ---------------------------------------------------------------------------- input validation
-__global__ void k_check_finite(long long n, const float* __restrict__ x, int* flag) {
+// Arrays of the library's own (16-byte aligned), handled together by one launch: a step checks fourteen and saves six,
+// and as launches or copies of their own each was 2 to 6 us.
+constexpr int MAX_ARRAYS = 14;
+struct Arrays {
+  const float* x[MAX_ARRAYS];
+  float* to[MAX_ARRAYS];
+  long long n[MAX_ARRAYS];
+  int count = 0;
+  void add(const float* from, long long size, float* dst = nullptr) {
+    x[count] = from;
+    to[count] = dst;
+    n[count++] = size;
+  }
+};
+// *flag |= 1 when a value is not finite.
+__global__ void k_check_finite(const __grid_constant__ Arrays a, int* flag) {
+  KSTART();
   bool bad = false;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-    bad |= !isfinite(x[q]);
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, T = (long long)gridDim.x * blockDim.x;
+  for (int q = 0; q < a.count; ++q) {
+    const float4* x = reinterpret_cast<const float4*>(a.x[q]);
+    const long long n4 = a.n[q] / 4;
+#pragma unroll 4
+    for (long long i = t; i < n4; i += T) {
+      const float4 v = x[i];
+      bad |= !isfinite(v.x) | !isfinite(v.y) | !isfinite(v.z) | !isfinite(v.w);
+    }
+    for (long long i = 4 * n4 + t; i < a.n[q]; i += T) bad |= !isfinite(a.x[q][i]);
+  }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(flag, 1);
+}
+__global__ void k_copy_arrays(const __grid_constant__ Arrays a) {
+  KSTART();
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, T = (long long)gridDim.x * blockDim.x;
+  for (int q = 0; q < a.count; ++q) {
+    const float4* x = reinterpret_cast<const float4*>(a.x[q]);
+    float4* y = reinterpret_cast<float4*>(a.to[q]);
+    const long long n4 = a.n[q] / 4;
+#pragma unroll 4
+    for (long long i = t; i < n4; i += T) y[i] = x[i];
+    for (long long i = 4 * n4 + t; i < a.n[q]; i += T) a.to[q][i] = a.x[q][i];
+  }
+}
+void check_arrays(fd3_volume* V, const Arrays& a) {
+  long long most = 1;
+  for (int q = 0; q < a.count; ++q) most = std::max(most, a.n[q]);
+  LAUNCH_G(V, k_check_finite, (int)std::min<long long>(8 * 148, (most / 4 + TPB - 1) / TPB + 1), TPB, a, V->dflag);
+}
+void copy_arrays(fd3_volume* V, const Arrays& a) {
+  long long most = 1;
+  for (int q = 0; q < a.count; ++q) most = std::max(most, a.n[q]);
+  LAUNCH_G(V, k_copy_arrays, (int)std::min<long long>(8 * 148, (most / 4 + TPB - 1) / TPB + 1), TPB, a);
+}
+// us = u (the velocity to project), and the pressure for a refusal.
+void stage_velocity(fd3_volume* V, bool pressure) {
+  Arrays a;
+  a.add(V->u, V->nu, V->us);
+  a.add(V->v, V->nv, V->vs);
+  a.add(V->w, V->nw, V->ws);
+  if (pressure) a.add(V->p, V->n, V->sv_p);
+  copy_arrays(V, a);
 }
 
 // A face of a column whose byte in `m` equals `mark` (clear_column_faces, delta3d_sparse.rs:213-233):
@@ -1252,27 +1356,32 @@ __device__ __forceinline__ bool column_face(const unsigned char* __restrict__ m,
 // close_walls (delta3d.rs:666-690): walls, bottom, and faces the cut closes have no velocity;
 // then close_sparse_walls (delta3d_sparse.rs:236-247): nor has any face of a column outside the
 // sparse set (g.act, 0 for those columns).
-__global__ void k_close_walls(Geo g, float* __restrict__ u, float* __restrict__ v, float* __restrict__ w) {
+// The faces come from us, vs, ws (which may be u, v, w themselves); a warp takes a row of faces along x.
+__global__ void k_close_walls(Geo g, const float* us, const float* vs, const float* ws, float* u, float* v, float* w) {
   KSTART();
   const unsigned char* out = g.act;
-  int nu = (g.nx + 1) * g.ny * g.nz, nv = g.nx * (g.ny + 1) * g.nz, nw = g.nx * g.ny * (g.nz + 1);
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < nu) {
-    int i = q % (g.nx + 1), j = (q / (g.nx + 1)) % g.ny;
-    if (i == 0 || i == g.nx || (g.cut && g.ou[q] == 0.f) || (out && column_face(out, 0, g.nx, g.ny, 0, i, j))) u[q] = 0.f;
-    return;
+  const int nx = g.nx, ny = g.ny, nz = g.nz, lane = threadIdx.x & 31;
+  const int ru = ny * nz, rv = (ny + 1) * nz, rw = ny * (nz + 1);
+  const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+  if (warp >= (long long)ru + rv + rw) return;
+  const int axis = warp < ru ? 0 : (warp < (long long)ru + rv ? 1 : 2);
+  const int row = (int)(warp - (axis == 0 ? 0 : (axis == 1 ? ru : (long long)ru + rv)));
+  const int width = axis == 0 ? nx + 1 : nx, rows = axis == 1 ? ny + 1 : ny, k = row / rows, j = row - k * rows;
+  const float* from = axis == 0 ? us : (axis == 1 ? vs : ws);
+  float* to = axis == 0 ? u : (axis == 1 ? v : w);
+  const float* open = axis == 0 ? g.ou : (axis == 1 ? g.ov : g.ow);
+  const bool wall = axis == 1 ? (j == 0 || j == ny) : (axis == 2 && k == 0);
+#pragma unroll 4
+  for (int i = lane; i < width; i += 32) {
+    const int q = row * width + i;
+    const float x = from[q];
+    const bool closed = wall || (axis == 0 && (i == 0 || i == nx)) || (g.cut && open[q] == 0.f) ||
+                        (out && column_face(out, 0, nx, ny, axis, i, j));
+    to[q] = closed ? 0.f : x;
   }
-  q -= nu;
-  if (q < nv) {
-    int i = q % g.nx, j = (q / g.nx) % (g.ny + 1);
-    if (j == 0 || j == g.ny || (g.cut && g.ov[q] == 0.f) || (out && column_face(out, 0, g.nx, g.ny, 1, i, j))) v[q] = 0.f;
-    return;
-  }
-  q -= nv;
-  if (q < nw) {
-    int k = q / (g.nx * g.ny), col = q % (g.nx * g.ny);
-    if (k == 0 || (g.cut && g.ow[q] == 0.f) || (out && out[col] == 0)) w[q] = 0.f;
-  }
+}
+inline long long wall_threads(const fd3_volume* V) {
+  return 32LL * ((long long)V->ny * V->nz + (long long)(V->ny + 1) * V->nz + (long long)V->ny * (V->nz + 1));
 }
 
 // Columns leaving the sparse set go to rest (apply_sparse, delta3d_sparse.rs:181-210): surface,
@@ -1375,7 +1484,9 @@ __global__ void k_displace_columns(int ncol, float area, const float* __restrict
 
 int check_finite_device(fd3_volume* V, const float* x, long long n, bool* ok) {
   CK(cudaMemsetAsync(V->dflag, 0, sizeof(int), V->stream));
-  LAUNCH_G(V, k_check_finite, 592, TPB, n, x, V->dflag);
+  Arrays a;
+  a.add(x, n);
+  check_arrays(V, a);
   CK(cudaMemcpyAsync(V->hflag, V->dflag, sizeof(int), cudaMemcpyDeviceToHost, V->stream));
   TRY(sync(V));
   *ok = *V->hflag == 0;
@@ -1411,24 +1522,9 @@ int alloc_state(fd3_volume* V) {
   TRY(dalloc(V, &q, 16)); V->dflag = (int*)q;
   TRY(dalloc(V, &q, (size_t)((V->nx + TILE_X - 1) / TILE_X) * ((V->ny + TILE_Y - 1) / TILE_Y))); V->ztop = (int*)q;
   TRY(dalloc(V, &q, (sizeof(GridSlots) + 3) / 4)); V->slots = (GridSlots*)q;
-  int sms = 0, coop = 0, resident = 0;
-  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, V->device));
-  CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, V->device));
-  // the attribute is per function, shared by every volume: the size each instance always asks for
-  CK(cudaFuncSetAttribute(k_cg_loop<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(4)));
-  CK(cudaFuncSetAttribute(k_cg_loop<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(8)));
-  CK(cudaFuncSetAttribute(k_cg_loop<GRID_MAX_CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)cg_smem(GRID_MAX_CELLS)));
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_cg_loop<GRID_MAX_CELLS>, GRID_THREADS,
-                                                   cg_smem(GRID_MAX_CELLS)));
-  V->grid_ctas = coop && resident >= 1 ? std::min(sms, GRID_MAX_CTAS) : 0;
-  for (auto k : {k_mg_loop<float>, k_mg_loop<__half>}) {
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MgShared)));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k, MG_THREADS, sizeof(MgShared)));
-    if (resident < 1) V->grid_ctas = 0;
-  }
+  TRY(cooperative_ctas(V->device, &V->grid_ctas));
   CK(cudaMallocHost((void**)&V->hS, sizeof(Scalars)));
-  CK(cudaMallocHost((void**)&V->hflag, sizeof(int)));
+  CK(cudaMallocHost((void**)&V->hflag, 2 * sizeof(int)));
   TRY(dalloc(V, &q, 32)); V->fsc = (double*)q;
   CK(cudaMallocHost((void**)&V->hfsc, 8 * sizeof(double)));
   memset(V->hS, 0, sizeof(Scalars));
@@ -1517,12 +1613,14 @@ int in_bounds(fd3_volume* V, bool* ok) {
 }
 
 int save_state(fd3_volume* V) {
-  CK(cudaMemcpyAsync(V->sv_u, V->u, (size_t)V->nu * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->sv_v, V->v, (size_t)V->nv * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->sv_w, V->w, (size_t)V->nw * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->sv_p, V->p, (size_t)V->n * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->sv_eta, V->eta, (size_t)V->ncol * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->sv_rof, V->rof, (size_t)V->ncol * 4, cudaMemcpyDeviceToDevice, V->stream));
+  Arrays a;
+  a.add(V->u, V->nu, V->sv_u);
+  a.add(V->v, V->nv, V->sv_v);
+  a.add(V->w, V->nw, V->sv_w);
+  a.add(V->p, V->n, V->sv_p);
+  a.add(V->eta, V->ncol, V->sv_eta);
+  a.add(V->rof, V->ncol, V->sv_rof);
+  copy_arrays(V, a);
   return FD3_OK;
 }
 
@@ -1556,21 +1654,20 @@ int step_body(fd3_volume* V, float scale, float correction, float transport, flo
          (const float*)V->v, V->flux_x, V->flux_y);
   LAUNCH(V, k_transport_eta, V->ncol, G, transport, (const float*)V->flux_x, (const float*)V->flux_y, V->eta, V->rof);
   // every field finite (delta3d_mobile.rs:885-906)
-  struct { const float* x; long long n; } fields[] = {
-      {V->u, V->nu}, {V->v, V->nv}, {V->w, V->nw}, {V->p, V->n}, {V->eta, V->ncol}, {V->rof, V->ncol},
-      {V->us, V->nu}, {V->vs, V->nv}, {V->ws, V->nw}, {V->rhs, V->n}, {V->res, V->n}, {V->dir, V->n},
-      {V->tmp, V->n}, {V->prec, V->n}};
-  CK(cudaMemsetAsync(V->dflag, 0, sizeof(int), V->stream));
-  for (auto& f : fields) {
-    LAUNCH_G(V, k_check_finite, 592, TPB, f.n, f.x, V->dflag);
-  }
-  CK(cudaMemcpyAsync(V->hflag, V->dflag, sizeof(int), cudaMemcpyDeviceToHost, V->stream));
+  Arrays fields;
+  for (auto& f : std::initializer_list<std::pair<const float*, int>>{
+           {V->u, V->nu}, {V->v, V->nv}, {V->w, V->nw}, {V->p, V->n}, {V->eta, V->ncol}, {V->rof, V->ncol},
+           {V->us, V->nu}, {V->vs, V->nv}, {V->ws, V->nw}, {V->rhs, V->n}, {V->res, V->n}, {V->dir, V->n},
+           {V->tmp, V->n}, {V->prec, V->n}})
+    fields.add(f.first, f.second);
+  CK(cudaMemsetAsync(V->dflag, 0, 2 * sizeof(int), V->stream));  // not finite; out of bounds
+  check_arrays(V, fields);
+  LAUNCH(V, k_in_bounds, V->ncol, V->geo(), (const float*)V->floor_, V->dflag + 1);
+  CK(cudaMemcpyAsync(V->hflag, V->dflag, 2 * sizeof(int), cudaMemcpyDeviceToHost, V->stream));
   TRY(sync(V));
-  if (*V->hflag) return FD3_ERR_NOT_FINITE;
+  if (V->hflag[0]) return FD3_ERR_NOT_FINITE;
   if (!std::isfinite(rep->residual) || !std::isfinite(rep->divergence)) return FD3_ERR_NOT_FINITE;
-  bool ok;
-  TRY(in_bounds(V, &ok));
-  if (!ok) return FD3_ERR_DOMAIN;
+  if (V->hflag[1]) return FD3_ERR_DOMAIN;
   return FD3_OK;
 }
 
@@ -1611,20 +1708,18 @@ int linear_body(fd3_volume* V, float scale, float correction, float transport, u
     TRY(sync(V));
     if (*V->hflag) return FD3_ERR_DOMAIN;
   }
-  CK(cudaMemcpyAsync(V->us, V->u, (size_t)V->nu * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->vs, V->v, (size_t)V->nv * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->ws, V->w, (size_t)V->nw * 4, cudaMemcpyDeviceToDevice, V->stream));
+  stage_velocity(V, false);
   TRY(project_linear(V, scale, correction, max_iters, rep));
   if (rep->degraded) return FD3_ERR_CONVERGENCE;
   LAUNCH(V, k_linear_transport, V->ncol, V->geo(), transport, (const float*)V->u, (const float*)V->v, V->eta, V->rof);
   // every field finite (delta3d.rs:1347-1353)
-  struct { const float* x; long long n; } fields[] = {
-      {V->u, V->nu}, {V->v, V->nv}, {V->w, V->nw}, {V->p, V->n}, {V->eta, V->ncol}, {V->rof, V->ncol},
-      {V->rhs, V->n}, {V->res, V->n}, {V->dir, V->n}, {V->tmp, V->n}};
+  Arrays fields;
+  for (auto& f : std::initializer_list<std::pair<const float*, int>>{
+           {V->u, V->nu}, {V->v, V->nv}, {V->w, V->nw}, {V->p, V->n}, {V->eta, V->ncol}, {V->rof, V->ncol},
+           {V->rhs, V->n}, {V->res, V->n}, {V->dir, V->n}, {V->tmp, V->n}})
+    fields.add(f.first, f.second);
   CK(cudaMemsetAsync(V->dflag, 0, sizeof(int), V->stream));
-  for (auto& f : fields) {
-    LAUNCH_G(V, k_check_finite, 592, TPB, f.n, f.x, V->dflag);
-  }
+  check_arrays(V, fields);
   CK(cudaMemcpyAsync(V->hflag, V->dflag, sizeof(int), cudaMemcpyDeviceToHost, V->stream));
   TRY(sync(V));
   if (*V->hflag) return FD3_ERR_NOT_FINITE;
@@ -1925,20 +2020,19 @@ int fd3_set_surface(fd3_volume* V, const float* eta, size_t len) {
 
 // delta3d.rs:631-645: the faces are staged in us/vs/ws, checked on the device, then published.
 // The staged faces are checked with one flag and one host round trip for the three arrays, then
-// copied into u, v, w (the published fields, which fd3_device_fields exposes: the call returns once
-// they are written).
+// published closed in u, v, w (the fields fd3_device_fields exposes: the call returns once they are written).
 static int set_velocity_staged(fd3_volume* V) {
   CK(cudaMemsetAsync(V->dflag, 0, sizeof(int), V->stream));
-  LAUNCH_G(V, k_check_finite, 592, TPB, (long long)V->nu, (const float*)V->us, V->dflag);
-  LAUNCH_G(V, k_check_finite, 592, TPB, (long long)V->nv, (const float*)V->vs, V->dflag);
-  LAUNCH_G(V, k_check_finite, 592, TPB, (long long)V->nw, (const float*)V->ws, V->dflag);
+  Arrays a;
+  a.add(V->us, V->nu);
+  a.add(V->vs, V->nv);
+  a.add(V->ws, V->nw);
+  check_arrays(V, a);
   CK(cudaMemcpyAsync(V->hflag, V->dflag, sizeof(int), cudaMemcpyDeviceToHost, V->stream));
   TRY(sync(V));
   if (*V->hflag != 0) return FD3_ERR_NOT_FINITE;
-  CK(cudaMemcpyAsync(V->u, V->us, (size_t)V->nu * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->v, V->vs, (size_t)V->nv * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->w, V->ws, (size_t)V->nw * 4, cudaMemcpyDeviceToDevice, V->stream));
-  LAUNCH(V, k_close_walls, (long long)V->nu + V->nv + V->nw, V->geo(), V->u, V->v, V->w);
+  LAUNCH(V, k_close_walls, wall_threads(V), V->geo(), (const float*)V->us, (const float*)V->vs, (const float*)V->ws, V->u,
+         V->v, V->w);
   return sync(V);
 }
 
@@ -2120,7 +2214,8 @@ int fd3_resample_from(fd3_volume* V, fd3_volume* S, fd3_level_change* change) {
          (const unsigned char*)(V->sparse ? V->act : nullptr), V->eta, V->rof);
   LAUNCH(V, k_resample_faces, (long long)V->nu + V->nv + V->nw, src, V->nx, V->ny, V->nz, n, V->u, V->v, V->w);
   CK(cudaMemsetAsync(V->p, 0, (size_t)V->n * 4, V->stream));
-  LAUNCH(V, k_close_walls, (long long)V->nu + V->nv + V->nw, V->geo(), V->u, V->v, V->w);
+  LAUNCH(V, k_close_walls, wall_threads(V), V->geo(), (const float*)V->u, (const float*)V->v, (const float*)V->w, V->u, V->v,
+         V->w);
   TRY(perturbation_volume(V, &ch.volume_after));
   if (change) *change = ch;
   return FD3_OK;
@@ -2135,10 +2230,7 @@ int fd3_reset_pressure(fd3_volume* V) {
 // tests_delta3d.rs:392-395: us = u, then project_mobile3.  A refusal leaves u, v, w, p untouched.
 int fd3_project_mobile(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_report* rep) {
   if (!V || !rep) return FD3_ERR_INVALID_ARGUMENT;
-  CK(cudaMemcpyAsync(V->us, V->u, (size_t)V->nu * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->vs, V->v, (size_t)V->nv * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->ws, V->w, (size_t)V->nw * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->sv_p, V->p, (size_t)V->n * 4, cudaMemcpyDeviceToDevice, V->stream));
+  stage_velocity(V, true);
   int e = project_mobile3(V, scale, k1, max_iters, rep);
   if (e) {
     cudaMemcpyAsync(V->u, V->us, (size_t)V->nu * 4, cudaMemcpyDeviceToDevice, V->stream);
@@ -2161,10 +2253,7 @@ __global__ void k_add_into(int n, float* __restrict__ p, const float* __restrict
 // to the base.  A refusal leaves u, v, w, p untouched.
 int fd3_refine_mobile(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_report* rep) {
   if (!V || !rep) return FD3_ERR_INVALID_ARGUMENT;
-  CK(cudaMemcpyAsync(V->us, V->u, (size_t)V->nu * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->vs, V->v, (size_t)V->nv * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->ws, V->w, (size_t)V->nw * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->sv_p, V->p, (size_t)V->n * 4, cudaMemcpyDeviceToDevice, V->stream));
+  stage_velocity(V, true);
   CK(cudaMemsetAsync(V->p, 0, (size_t)V->n * 4, V->stream));
   V->homog = true;
   int e = project_mobile3(V, scale, k1, max_iters, rep);
@@ -2192,10 +2281,7 @@ int fd3_step_surface_mobile(fd3_volume* V, uint64_t duration_us, uint32_t max_it
 int fd3_project_linear(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_report* rep) {
   if (!V || !rep) return FD3_ERR_INVALID_ARGUMENT;
   if (V->sparse) return FD3_ERR_DOMAIN;  // the linear path does not carry a sparse set (delta3d.rs:1210-1211)
-  CK(cudaMemcpyAsync(V->us, V->u, (size_t)V->nu * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->vs, V->v, (size_t)V->nv * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->ws, V->w, (size_t)V->nw * 4, cudaMemcpyDeviceToDevice, V->stream));
-  CK(cudaMemcpyAsync(V->sv_p, V->p, (size_t)V->n * 4, cudaMemcpyDeviceToDevice, V->stream));
+  stage_velocity(V, true);
   int e = project_linear(V, scale, k1, max_iters, rep);
   if (e) {
     cudaMemcpyAsync(V->u, V->us, (size_t)V->nu * 4, cudaMemcpyDeviceToDevice, V->stream);
@@ -2571,7 +2657,7 @@ int fd3_assemble_pressure_problem_for_trials(fd3_volume* V, const float* diverge
   TRY(check_finite_device(V, V->tmp, V->n, &ok));
   if (!ok) return FD3_ERR_NOT_FINITE;
   CK(cudaMemcpyAsync(V->rhs, V->tmp, len * 4, cudaMemcpyDeviceToDevice, V->stream));
-  DISPATCH(V, k_rhs_b2, V->n, V->geo(), scale, V->rhs, V->prec, V->red(), V->dS, 0, (unsigned short*)nullptr,
+  DISPATCH(V, k_rhs_b2, V->n, V->geo(), scale, Faces{}, V->rhs, V->prec, V->red(), V->dS, 0, (unsigned short*)nullptr,
            (float*)nullptr, WorkVectors{});
   CK(cudaMemcpyAsync(rhs, V->rhs, len * 4, cudaMemcpyDeviceToHost, V->stream));
   CK(cudaMemcpyAsync(prec, V->prec, len * 4, cudaMemcpyDeviceToHost, V->stream));
@@ -2584,7 +2670,7 @@ int fd3_vcycle_for_tests(fd3_volume* V, const float* x, float* z, size_t len) {
   if (!V->has_mg) return FD3_ERR_DOMAIN;
   if (len != (size_t)V->n) return FD3_ERR_SHAPE;
   CK(cudaMemsetAsync(V->rhs, 0, len * 4, V->stream));
-  DISPATCH(V, k_rhs_b2, V->n, V->geo(), 1.f, V->rhs, V->prec, V->red(), V->dS, 0, V->codes, (float*)nullptr,
+  DISPATCH(V, k_rhs_b2, V->n, V->geo(), 1.f, Faces{}, V->rhs, V->prec, V->red(), V->dS, 0, V->codes, (float*)nullptr,
            WorkVectors{});
   prepare_multigrid(V);
   CK(cudaMemcpyAsync(V->res, x, len * 4, cudaMemcpyHostToDevice, V->stream));
