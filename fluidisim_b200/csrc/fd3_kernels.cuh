@@ -903,6 +903,10 @@ __global__ void k_extrapolate(Geo g, float* __restrict__ u, float* __restrict__ 
   // the cells on either side of the face: (xl, yl) and (i, j), or the one below it
   const int xl = axis == 0 ? i - 1 : i, yl = axis == 1 ? j - 1 : j;
   const float hl = __ldg(g.eta + yl * g.nx + xl), hr = __ldg(g.eta + col);
+  if (!col_active(g, xl, yl) || !col_active(g, i, j)) return;  // the sparse set closes every face here
+  const float* ap = axis == 0 ? g.ou : (axis == 1 ? g.ov : g.ow);
+  const int f0 = axis == 0 ? fu(g, i, j, 0) : (axis == 1 ? fv(g, i, j, 0) : fw(g, i, j, 0));
+  const int fs = axis == 0 ? g.ny * (g.nx + 1) : (axis == 1 ? (g.ny + 1) * g.nx : g.nx * g.ny), nxny = g.nx * g.ny;
   // The walk's only chain is `last`: the loads of AHEAD layers go out together (one layer at a time, a 96-layer
   // column took 111 us of dependent loads).
   constexpr int AHEAD = 8;
@@ -916,11 +920,15 @@ __global__ void k_extrapolate(Geo g, float* __restrict__ u, float* __restrict__ 
       val[e] = 0.f;
       solid[e] = true;
       if (k >= end) continue;
-      const int f = axis == 0 ? fu(g, i, j, k) : (axis == 1 ? fv(g, i, j, k) : fw(g, i, j, k));
-      open[e] = open3(g, axis, f);
-      val[e] = field[f];
-      if (axis == 2) solid[e] = solid3(g, ((k - 1) * g.ny + j) * g.nx + i);
-      else solid[e] = solid3(g, (k * g.ny + yl) * g.nx + xl) | solid3(g, (k * g.ny + j) * g.nx + i);
+      val[e] = field[f0 + k * fs];
+      open[e] = 1.f;
+      solid[e] = false;
+      if (g.cut) {  // a test on each load would put them in series
+        open[e] = __ldg(ap + f0 + k * fs);
+        const int below = axis == 2 ? nxny : 0;
+        solid[e] = (__ldg(g.frac + k * nxny + yl * g.nx + xl - below) == 0.f) |
+                   (__ldg(g.frac + k * nxny + col - below) == 0.f);
+      }
     }
 #pragma unroll
     for (int e = 0; e < AHEAD; ++e) {
@@ -929,7 +937,7 @@ __global__ void k_extrapolate(Geo g, float* __restrict__ u, float* __restrict__ 
       const float z = axis == 2 ? ((float)(k - 1) + 0.5f) * g.dx : ((float)k + 0.5f) * g.dx;
       const bool solved = open[e] > 0.f && !solid[e] && (axis == 2 ? z < hr : (z < hl || z < hr));
       if (solved) { last = val[e]; has_last = true; }
-      else if (has_last) field[axis == 0 ? fu(g, i, j, k) : (axis == 1 ? fv(g, i, j, k) : fw(g, i, j, k))] = last;
+      else if (has_last) field[f0 + k * fs] = last;
     }
   }
 }
@@ -953,15 +961,20 @@ __global__ void k_transport_flux(Geo g, const float* __restrict__ u, const float
     float surface = 0.5f * (g.eta[y * g.nx + x] + g.eta[j * g.nx + i]);
     constexpr int AHEAD = 8;  // layers whose loads go out together
     bool done = false;
+    // an interior face of a column outside the sparse set is closed in every layer
+    const float live = col_active(g, x, y) && col_active(g, i, j) ? 1.f : 0.f;
+    const float* vel = axis == 0 ? u : v;
+    const float* ap = axis == 0 ? g.ou : g.ov;
+    const int f0 = axis == 0 ? fu(g, i, j, 0) : fv(g, i, j, 0), fs = axis == 0 ? g.ny * (g.nx + 1) : (g.ny + 1) * g.nx;
     for (int k0 = 0; k0 < g.nz && !done; k0 += AHEAD) {
       float uu[AHEAD], a[AHEAD];
 #pragma unroll
       for (int e = 0; e < AHEAD; ++e) {
         uu[e] = a[e] = 0.f;
         if (k0 + e >= g.nz) continue;
-        const int f = axis == 0 ? fu(g, i, j, k0 + e) : fv(g, i, j, k0 + e);
-        uu[e] = axis == 0 ? u[f] : v[f];
-        a[e] = open3(g, axis, f);
+        uu[e] = vel[f0 + (k0 + e) * fs];
+        a[e] = g.cut ? __ldg(ap + f0 + (k0 + e) * fs) : 1.f;
+        a[e] = live == 0.f ? 0.f : a[e];
       }
 #pragma unroll
       for (int e = 0; e < AHEAD; ++e) {
