@@ -1020,27 +1020,54 @@ __device__ __forceinline__ void level_ijk(const Lev& L, int c, int& i, int& j, i
   k = t / L.ny;
 }
 
+// What a SPEC pass reads of a cell's row: none of it is written during a solve, so it is loaded before KSTART, while
+// the pass before this one still runs.  (A kernel starts only when every block of the one before it is past its own
+// wait, so all that was written two kernels ago or earlier is there; the levels' rows are older.)  No block may return
+// before its KSTART: the kernel after it would then wait for too little.
+struct LevRow {
+  int i, j, k;
+  unsigned code;
+  float dg;
+  Ap6 ap;
+  bool skip;  // outside the level, or in the air
+  __device__ __forceinline__ void load(const Lev& L, const Air& air, int c, bool in) {
+    const int n = in ? c : 0;
+    level_ijk(L, n, i, j, k);
+    code = L.code[n];
+    dg = L.diag[n];
+    ap = level_ap6(L, i, j, k);
+    skip = !in || in_air(air, i, j, k);
+  }
+  __device__ __forceinline__ bool load_code(const Lev& L, const Air& air, int c) {
+    level_ijk(L, c, i, j, k);
+    if (in_air(air, i, j, k)) return false;
+    code = L.code[c];
+    dg = L.diag[c];
+    return true;
+  }
+};
+
 // The two pre-sweeps of a coarse level from x = 0, written to L.x (smooth3 twice after fill(0)).
 template <class T, bool SPEC>
 __global__ void __launch_bounds__(TPB) k_level_pre(Lev L, Air air, const Scalars* S, int gate) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  LevRow w;
+  if (SPEC) w.load(L, air, c, c < L.n);
   KSTART();
   if (!SPEC && gate && !S->active) return;
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= L.n) return;
+  if (SPEC ? w.skip : c >= L.n) return;
   auto X1 = [&](int n) { return level_x1<T>(L, n); };
   auto X1c = [&](int n, int, int, int) { return level_x1<T>(L, n); };
-  int i, j, k;
-  level_ijk(L, c, i, j, k);
-  if (in_air(air, i, j, k)) return;
-  const unsigned code = L.code[c];
-  const float dg = L.diag[c];
+  if (!SPEC && !w.load_code(L, air, c)) return;
+  const int i = w.i, j = w.j, k = w.k;
+  const unsigned code = w.code;
+  const float dg = w.dg;
   const float rc = Store<T>::ld(as<T>(L.r), c);
   float xc = X1(c);
   if (SPEC) {
-    const Ap6 ap = level_ap6(L, i, j, k);
     const Nb6 b = level_nb(L, i, j, k, c, X1c);
     if (gate && !S->active) return;
-    if (dg > 0.f) xc += OMEGA * (rc - level_row_sel(L, code, xc, b, ap)) / dg;
+    if (dg > 0.f) xc += OMEGA * (rc - level_row_sel(L, code, xc, b, w.ap)) / dg;
   } else if (dg > 0.f) {
     xc += OMEGA * (rc - level_row_code(L, code, i, j, k, c, X1)) / dg;
   }
@@ -1101,35 +1128,35 @@ __global__ void __launch_bounds__(TPB) k_level_sum8(Lev F, Lev C, Air air, const
 // stored t would be, and the first of them sums the eight in order (restrict3).
 template <class T, bool SPEC>
 __global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, Air air, const Scalars* S, int gate) {
-  KSTART();
-  if (!SPEC && gate && !S->active) return;
   const int q8 = blockIdx.x * blockDim.x + threadIdx.x;
   const int q = q8 >> 3, e = q8 & 7;
   bool own = q < C.n;
-  if (own) own = !in_air(air, q % C.nx, q / C.nx % C.ny, q / (C.nx * C.ny));
-  if (!__any_sync(0xffffffffu, own)) return;
-  float tv = 0.f;
   unsigned code = 0u;
   int i = 0, j = 0, k = 0, c = 0;
-  float rc = 0.f, pc = 0.f;
-  const LoadT<T> X{as<T>(F.x)};
-  if (own) {
+  Ap6 ap{};
+  if (own) {  // the row before the wait (LevRow)
     const int ci = q % C.nx, t = q / C.nx, cj = t % C.ny, ck = t / C.ny;
+    own = !in_air(air, ci, cj, ck);
     i = 2 * ci + (e & 1);
     j = 2 * cj + ((e >> 1) & 1);
     k = 2 * ck + (e >> 2);
     c = (k * F.ny + j) * F.nx + i;
     code = F.code[c];
+    if (SPEC) ap = level_ap6(F, i, j, k);
+  }
+  KSTART();
+  if (!SPEC && gate && !S->active) return;
+  if (!__any_sync(0xffffffffu, own)) return;
+  float tv = 0.f;
+  float rc = 0.f, pc = 0.f;
+  const LoadT<T> X{as<T>(F.x)};
+  if (own) {
     rc = Store<T>::ld(as<T>(F.r), c);
     pc = X(c);
   }
   if (SPEC) {
     Nb6 b{};
-    Ap6 ap{};
-    if (own) {
-      ap = level_ap6(F, i, j, k);
-      b = level_nb(F, i, j, k, c, [&](int n, int, int, int) { return X(n); });
-    }
+    if (own) b = level_nb(F, i, j, k, c, [&](int n, int, int, int) { return X(n); });
     if (gate && !S->active) return;
     if (own) tv = Store<T>::rt(rc - ((code & RC_WET) ? level_row_sel(F, code, pc, b, ap) : 0.f));
   } else if (own) {
@@ -1145,10 +1172,12 @@ __global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, Air air, 
 // Prolongation from C (x += parent) fused with the first post-sweep, L.x -> L.x2.
 template <class T, bool SPEC>
 __global__ void __launch_bounds__(TPB) k_level_post1(Lev L, Lev C, Air air, const Scalars* S, int gate) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  LevRow w;
+  if (SPEC) w.load(L, air, c, c < L.n);
   KSTART();
   if (!SPEC && gate && !S->active) return;
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= L.n) return;
+  if (SPEC ? w.skip : c >= L.n) return;
   auto XPc = [&](int n, int i, int j, int k) {
     return Store<T>::ld(as<T>(L.x), n) + Store<T>::ld(as<T>(C.x), ((k >> 1) * C.ny + (j >> 1)) * C.nx + (i >> 1));
   };
@@ -1157,18 +1186,16 @@ __global__ void __launch_bounds__(TPB) k_level_post1(Lev L, Lev C, Air air, cons
     level_ijk(L, n, i, j, k);
     return XPc(n, i, j, k);
   };
-  int i, j, k;
-  level_ijk(L, c, i, j, k);
-  if (in_air(air, i, j, k)) return;
-  const unsigned code = L.code[c];
-  const float dg = L.diag[c];
+  if (!SPEC && !w.load_code(L, air, c)) return;
+  const int i = w.i, j = w.j, k = w.k;
+  const unsigned code = w.code;
+  const float dg = w.dg;
   const float rc = Store<T>::ld(as<T>(L.r), c);
   float xc = XPc(c, i, j, k);
   if (SPEC) {
-    const Ap6 ap = level_ap6(L, i, j, k);
     const Nb6 b = level_nb(L, i, j, k, c, XPc);
     if (gate && !S->active) return;
-    if (dg > 0.f) xc += OMEGA * (rc - level_row_sel(L, code, xc, b, ap)) / dg;
+    if (dg > 0.f) xc += OMEGA * (rc - level_row_sel(L, code, xc, b, w.ap)) / dg;
   } else if (dg > 0.f) {
     xc += OMEGA * (rc - level_row_code(L, code, i, j, k, c, XP)) / dg;
   }
@@ -1178,24 +1205,24 @@ __global__ void __launch_bounds__(TPB) k_level_post1(Lev L, Lev C, Air air, cons
 // The second post-sweep, L.x2 -> L.x.
 template <class T, bool SPEC>
 __global__ void __launch_bounds__(TPB) k_level_post2(Lev L, Air air, const Scalars* S, int gate) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  LevRow w;
+  if (SPEC) w.load(L, air, c, c < L.n);
   KSTART();
   if (!SPEC && gate && !S->active) return;
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= L.n) return;
+  if (SPEC ? w.skip : c >= L.n) return;
   const LoadT<T> X{as<T>(L.x2)};
   auto Xc = [&](int n, int, int, int) { return X(n); };
-  int i, j, k;
-  level_ijk(L, c, i, j, k);
-  if (in_air(air, i, j, k)) return;
-  const unsigned code = L.code[c];
-  const float dg = L.diag[c];
+  if (!SPEC && !w.load_code(L, air, c)) return;
+  const int i = w.i, j = w.j, k = w.k;
+  const unsigned code = w.code;
+  const float dg = w.dg;
   const float rc = Store<T>::ld(as<T>(L.r), c);
   float xc = X(c);
   if (SPEC) {
-    const Ap6 ap = level_ap6(L, i, j, k);
     const Nb6 b = level_nb(L, i, j, k, c, Xc);
     if (gate && !S->active) return;
-    if (dg > 0.f) xc += OMEGA * (rc - level_row_sel(L, code, xc, b, ap)) / dg;
+    if (dg > 0.f) xc += OMEGA * (rc - level_row_sel(L, code, xc, b, w.ap)) / dg;
   } else if (dg > 0.f) {
     xc += OMEGA * (rc - level_row_code(L, code, i, j, k, c, X)) / dg;
   }
@@ -1208,14 +1235,13 @@ __global__ void __launch_bounds__(TPB) k_level_post2(Lev L, Air air, const Scala
 // stencil points), with k_level_post2's expression, rounded through the storage type as the stored
 // C.x would be; the warp shares the seven values; each child then sweeps its own row with
 // k_level_post1's expression.  C.x is never stored: only this pass would read it.
-template <class T>
+template <class T, bool WAIT = false>
 __device__ __forceinline__ void level_post21_at(const Lev& L, const Lev& C, const Air& air, int q8,
                                                 const Scalars* gate = nullptr) {
   const int q = q8 >> 3, e = q8 & 7;
   bool own = q < C.n;
   const int ci = own ? q % C.nx : 0, cj = own ? (q / C.nx) % C.ny : 0, ck = own ? q / (C.nx * C.ny) : 0;
   if (own) own = !in_air(air, ci, cj, ck);
-  if (!__any_sync(0xffffffffu, own)) return;
   // the C cell this lane sweeps: 0 the parent, 1..6 its x-, x+, y-, y+, z-, z+ neighbours
   int pi = ci, pj = cj, pk = ck;
   if (e == 1) pi -= 1; else if (e == 2) pi += 1; else if (e == 3) pj -= 1;
@@ -1231,9 +1257,6 @@ __device__ __forceinline__ void level_post21_at(const Lev& L, const Lev& C, cons
     pc = (pk * C.ny + pj) * C.nx + pi;
     pcode = C.code[pc];
     pdg = C.diag[pc];
-    pr = Store<T>::ld(as<T>(C.r), pc);
-    px2 = X2(pc);
-    pb = level_nb(C, pi, pj, pk, pc, [&](int n, int, int, int) { return X2(n); });
     pap = level_ap6(C, pi, pj, pk);
   }
   // the child's own row
@@ -1247,10 +1270,19 @@ __device__ __forceinline__ void level_post21_at(const Lev& L, const Lev& C, cons
   if (own) {
     code = L.code[c];
     dg = L.diag[c];
+    ap = level_ap6(L, i, j, k);
+  }
+  if (WAIT) KSTART();  // the rows before the wait (LevRow); in the one-launch loop there is none
+  if (!__any_sync(0xffffffffu, own)) return;
+  if (psweep) {
+    pr = Store<T>::ld(as<T>(C.r), pc);
+    px2 = X2(pc);
+    pb = level_nb(C, pi, pj, pk, pc, [&](int n, int, int, int) { return X2(n); });
+  }
+  if (own) {
     rc = Store<T>::ld(as<T>(L.r), c);
     xc0 = X(c);
     b = level_nb(L, i, j, k, c, [&](int n, int, int, int) { return X(n); });
-    ap = level_ap6(L, i, j, k);
   }
   if (gate && !gate->active) return;
   float xp = px2;  // C's final x at the lane's cell (k_level_post2)
@@ -1281,8 +1313,7 @@ __device__ __forceinline__ void level_post21_at(const Lev& L, const Lev& C, cons
 }
 template <class T>
 __global__ void __launch_bounds__(TPB) k_level_post21(Lev L, Lev C, Air air, const Scalars* S, int gate) {
-  KSTART();
-  level_post21_at<T>(L, C, air, blockIdx.x * blockDim.x + threadIdx.x, gate ? S : nullptr);
+  level_post21_at<T, true>(L, C, air, blockIdx.x * blockDim.x + threadIdx.x, gate ? S : nullptr);
 }
 
 // The same passes at one cell (or one lane) for the one-launch loop, which has no gate: every load before the row.
@@ -1719,13 +1750,13 @@ __device__ __forceinline__ void tail_cycle(const Lev (&Ls)[TAIL_REG_LEVELS], int
 template <class ST>
 __global__ void __launch_bounds__(TAIL_REG_THREADS) k_coarse_tail_reg(const __grid_constant__ TailLevs Ls_, int nl,
                                                                      const Scalars* S, int gate) {
-  KSTART();
   __shared__ TailShared sh;
   const Lev (&Ls)[TAIL_REG_LEVELS] = Ls_.L;
   const int c = threadIdx.x;
-  // the rows and the right-hand side are loaded before the loop's gate is read (it is checked before
+  // the rows before the wait (LevRow), the right-hand side before the loop's gate is read (it is checked before
   // anything is written to memory)
   tail_rows(Ls, nl, sh);
+  KSTART();
   if (c < Ls[0].n) sh.R[c] = Store<ST>::ld(as<ST>(Ls[0].r), c);
   if (gate && !S->active) return;
   __syncthreads();

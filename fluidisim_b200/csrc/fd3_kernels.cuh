@@ -29,9 +29,10 @@ enum Mode { RED_F64 = 0, RED_ORD = 1 };
 
 // Programmatic dependent launch (sm_90+): every kernel of the library is launched so that its CTAs
 // may be scheduled while the previous kernel on the stream is still running.  KSTART, the first
-// statement of every kernel, waits until that previous grid has completed and its memory is
+// statement of all but the coarse levels' passes (LevRow), waits until that previous grid has completed and its memory is
 // visible (griddepcontrol.wait; a no-op when launched without the attribute), then lets the next
-// kernel start scheduling (griddepcontrol.launch_dependents).  Nothing is read before the wait.
+// kernel start scheduling (griddepcontrol.launch_dependents).  Before the wait only what was
+// written two kernels ago or earlier may be read, and nothing may be written.
 #define KSTART()                                              \
   do {                                                        \
     asm volatile("griddepcontrol.wait;" ::: "memory");        \
