@@ -1035,7 +1035,7 @@ struct LevRow {
     level_ijk(L, n, i, j, k);
     code = L.code[n];
     dg = L.diag[n];
-    ap = level_ap6(L, i, j, k);
+    if (!(code & RC_UNIT)) ap = level_ap6(L, i, j, k);
     skip = !in || in_air(air, i, j, k);
   }
   __device__ __forceinline__ bool load_code(const Lev& L, const Air& air, int c) {
@@ -1142,7 +1142,7 @@ __global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, Air air, 
     k = 2 * ck + (e >> 2);
     c = (k * F.ny + j) * F.nx + i;
     code = F.code[c];
-    if (SPEC) ap = level_ap6(F, i, j, k);
+    if (SPEC && !(code & RC_UNIT)) ap = level_ap6(F, i, j, k);
   }
   KSTART();
   if (!SPEC && gate && !S->active) return;
@@ -1257,7 +1257,7 @@ __device__ __forceinline__ void level_post21_at(const Lev& L, const Lev& C, cons
     pc = (pk * C.ny + pj) * C.nx + pi;
     pcode = C.code[pc];
     pdg = C.diag[pc];
-    pap = level_ap6(C, pi, pj, pk);
+    if (!(pcode & RC_UNIT)) pap = level_ap6(C, pi, pj, pk);
   }
   // the child's own row
   const int i = 2 * ci + (e & 1), j = 2 * cj + ((e >> 1) & 1), k = 2 * ck + (e >> 2);
@@ -1270,7 +1270,7 @@ __device__ __forceinline__ void level_post21_at(const Lev& L, const Lev& C, cons
   if (own) {
     code = L.code[c];
     dg = L.diag[c];
-    ap = level_ap6(L, i, j, k);
+    if (!(code & RC_UNIT)) ap = level_ap6(L, i, j, k);
   }
   if (WAIT) KSTART();  // the rows before the wait (LevRow); in the one-launch loop there is none
   if (!__any_sync(0xffffffffu, own)) return;
@@ -1398,13 +1398,33 @@ __device__ __forceinline__ void level_sweep_at(const Lev& L, const float* xin_, 
   }
   Store<T>::st(xout, c, xc);
 }
-template <class T>
-__global__ void __launch_bounds__(TPB) k_level_sweep_c(Lev L, const float* __restrict__ xin, float* __restrict__ xout,
-                                                       int zero_in, const Scalars* S, int gate) {
+// SPEC as in the other passes, the first two sweeps being k_level_pre: at 45 x 25 x 19 cells the eight sweeps of a
+// cycle take 9.7 us less than with the loads behind the row code.
+template <class T, bool SPEC>
+__global__ void __launch_bounds__(TPB) k_level_sweep_c(Lev L, Air air, const float* __restrict__ xin,
+                                                       float* __restrict__ xout, int zero_in, const Scalars* S,
+                                                       int gate) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  LevRow w;
+  if (SPEC) w.load(L, air, c, c < L.n);
   KSTART();
+  if (!SPEC) {
+    if (gate && !S->active) return;
+    if (c < L.n) level_sweep_at<T>(L, xin, xout, zero_in, c);
+    return;
+  }
+  if (w.skip) return;
+  const float rc = Store<T>::ld(as<T>(L.r), c);
+  float xc = 0.f;
+  Nb6 b{};
+  if (!zero_in) {
+    const LoadT<T> X{reinterpret_cast<const T*>(xin)};
+    xc = X(c);
+    b = level_nb(L, w.i, w.j, w.k, c, [&](int n, int, int, int) { return X(n); });
+  }
   if (gate && !S->active) return;
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < L.n) level_sweep_at<T>(L, xin, xout, zero_in, c);
+  if (w.dg > 0.f) xc += OMEGA * (rc - (zero_in ? 0.f : level_row_sel(L, w.code, xc, b, w.ap))) / w.dg;
+  Store<T>::st(reinterpret_cast<T*>(xout), c, xc);
 }
 
 // All levels from `first` to `last` in one CTA (coarse_cycle3 restricted to them): each phase is a

@@ -464,9 +464,16 @@ void coarse_cycle_t(fd3_volume* V, int gate) {
   for (int l = 0; l < first_tail && l <= last; ++l) {
     Lev& L = Ls[l];
     if (l == last) {  // a large coarsest level: its 8 sweeps one by one
-      for (int s = 0; s < 8; ++s)
-        LAUNCH(V, k_level_sweep_c<T>, L.n, L, (const float*)((s % 2 == 0) ? L.x : L.x2), (s % 2 == 0) ? L.x2 : L.x,
-               s == 0 ? 1 : 0, S, gate);
+      const bool spec = L.n <= SPEC_MAX_CELLS;
+      int s = 0;
+      if (!half && spec) {  // the first two in one pass, which does not store the first (in f16 it is rounded)
+        launch_grid(V, "k_level_pre", blocks_for(L.n), TPB, k_level_pre<T, true>, L, air(l), S, gate);
+        s = 2;
+      }
+      for (; s < 8; ++s)
+        launch_grid(V, "k_level_sweep_c", blocks_for(L.n), TPB, spec ? k_level_sweep_c<T, true> : k_level_sweep_c<T, false>,
+                    L, air(l), (const float*)((s % 2 == 0) ? L.x : L.x2), (s % 2 == 0) ? L.x2 : L.x, s == 0 ? 1 : 0, S,
+                    gate);
     } else {
       const long long n8 = 8LL * Ls[l + 1].n;  // one thread per child of each next-level cell
       if (L.n <= SPEC_MAX_CELLS) {
