@@ -368,6 +368,9 @@ __device__ __forceinline__ void block_fmax3_atomic(float a, float b, float c, fl
 #ifndef FD3_RHS_MINB
 #define FD3_RHS_MINB 6
 #endif
+#ifndef FD3_RHS_MARCH_MINB
+#define FD3_RHS_MARCH_MINB 4
+#endif
 constexpr int CM_X = 32, CM_Y = 8, CM_K = 8;
 inline int cm_blocks(int nx, int ny, int nz) {
   return ((nx + CM_X - 1) / CM_X) * ((ny + CM_Y - 1) / CM_Y) * ((nz + CM_K - 1) / CM_K);
@@ -1799,21 +1802,9 @@ __global__ void k_loop_cond(cudaGraphConditionalHandle handle, Scalars* S) {
 // ------------------------------------------------------------------------------------------------
 // Set-up reductions with the in-kernel finish.
 
-// One row of rhs_mobile3 (delta3d_mobile.rs:215-241): rhs and prec of cell c, whose divergence is div(), its row
-// code into codes and p = 0 on a dry cell when those are not null; returns b.
-template <class Div>
-__device__ __forceinline__ float rhs_b2_at(const Geo& g, float scale, Div div, float* __restrict__ rhs,
-                                           float* __restrict__ prec, unsigned short* __restrict__ codes,
-                                           float* __restrict__ pdry, int c) {
-  int i, j, k; cell_ijk(g, c, i, j, k);
-  if (!wet3(g, i, j, k)) {
-    rhs[c] = 0.f; prec[c] = 0.f;
-    if (codes) codes[c] = 0;
-    if (pdry) pdry[c] = 0.f;
-    return 0.f;
-  }
-  RowE row[6]; mobile_row(g, i, j, k, row);
-  float b = scale * div();
+// rhs, prec and (codes not null) the row code and record of a wet cell, from its row and its scaled divergence b.
+__device__ __forceinline__ float rhs_row_store(const Geo& g, const RowE (&row)[6], float b, float* __restrict__ rhs,
+                                               float* __restrict__ prec, unsigned short* __restrict__ codes, int c) {
   float diag = 0.f;
 #pragma unroll
   for (int f = 0; f < 6; ++f) {
@@ -1836,6 +1827,23 @@ __device__ __forceinline__ float rhs_b2_at(const Geo& g, float scale, Div div, f
     }
   }
   return b;
+}
+
+// One row of rhs_mobile3 (delta3d_mobile.rs:215-241): rhs and prec of cell c, whose divergence is div(), its row
+// code into codes and p = 0 on a dry cell when those are not null; returns b.
+template <class Div>
+__device__ __forceinline__ float rhs_b2_at(const Geo& g, float scale, Div div, float* __restrict__ rhs,
+                                           float* __restrict__ prec, unsigned short* __restrict__ codes,
+                                           float* __restrict__ pdry, int c) {
+  int i, j, k; cell_ijk(g, c, i, j, k);
+  if (!wet3(g, i, j, k)) {
+    rhs[c] = 0.f; prec[c] = 0.f;
+    if (codes) codes[c] = 0;
+    if (pdry) pdry[c] = 0.f;
+    return 0.f;
+  }
+  RowE row[6]; mobile_row(g, i, j, k, row);
+  return rhs_row_store(g, row, scale * div(), rhs, prec, codes, c);
 }
 
 // The loop's r, d (two buffers) and q: zeroed where there is no row (Geo::ztop).  Null: left alone.
@@ -1867,6 +1875,113 @@ __global__ void __launch_bounds__(TPB, FD3_RHS_MINB) k_rhs_b2(Geo g, float scale
   if (!reduce) return;
   if (__syncthreads_or(c < g.n && b != 0.f) && threadIdx.x == 0) atomicOr(&S->any_nonzero, 1);
   reduce_finish<MODE>(Acc<MODE>::prod(b, b), c, g.n, red, S, FIN_B2);
+}
+
+// The same assembly for a projection with f64 sums, marching the columns as k_correct_metric does, `layers` to a block:
+// what is above a cell is below the next, the column tests and heights are read once, the apertures serve the row
+// and the divergence, and a block has one partial sum for its layers.  One thread per cell read every operand again
+// and met the block's reduction each time: 444 us of a 256^3 assembly, 185 us here (its bytes take 66 us at
+// 6.65 TB/s), 61 and 37 us at 128^3.  Four resident CTAs (64 registers): five spill and take 204 us.
+__global__ void __launch_bounds__(CM_X * CM_Y, FD3_RHS_MARCH_MINB) k_rhs_march(
+    Geo g, float scale, Faces vel, float* __restrict__ rhs, float* __restrict__ prec, Red red, Scalars* S,
+    unsigned short* __restrict__ codes, float* __restrict__ pdry, WorkVectors work, int layers) {
+  KSTART();
+  const int ntx = (g.nx + CM_X - 1) / CM_X, nty = (g.ny + CM_Y - 1) / CM_Y;
+  int blk = blockIdx.x;
+  const int bx = blk % ntx; blk /= ntx;
+  const int by = blk % nty; blk /= nty;
+  const int i = bx * CM_X + (int)(threadIdx.x & 31), j = by * CM_Y + (int)(threadIdx.x >> 5);
+  const int k0 = blk * layers, ke = min(k0 + layers, g.nz);
+  double sum = 0.0;
+  bool nonzero = false;
+  if (i < g.nx && j < g.ny) {
+    const int nxny = g.nx * g.ny, su = g.ny * (g.nx + 1), sv = (g.ny + 1) * g.nx, col = j * g.nx + i;
+    const int nb[4] = {-1, 1, -g.nx, g.nx};
+    RowIn o;
+    o.ok[0] = i > 0; o.ok[1] = i + 1 < g.nx; o.ok[2] = j > 0; o.ok[3] = j + 1 < g.ny;
+    o.hc = __ldg(g.eta + col);
+    const bool act = !g.act || __ldg(g.act + col) != 0;
+    bool open[4];  // the column beyond is in the domain and in the set
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      o.hn[f] = o.ok[f] ? __ldg(g.eta + col + nb[f]) : 0.f;
+      open[f] = o.ok[f] && (!g.act || __ldg(g.act + col + nb[f]) != 0);
+    }
+    int c = k0 * nxny + col, ful = fu(g, i, j, k0), fvf = fv(g, i, j, k0);
+    const bool cut = g.cut;
+    float frac = cut ? __ldg(g.frac + c) : 1.f;                     // of the cell,
+    float frac_d = cut && k0 > 0 ? __ldg(g.frac + c - nxny) : 1.f;  // of the one below;
+    float ow = cut ? __ldg(g.ow + c) : 1.f;                         // of its w face below
+    float wb = vel.w[c];
+    for (int k = k0; k < ke; ++k, c += nxny, ful += su, fvf += sv) {
+      if (!act || !(((float)k + 0.5f) * g.dx < o.hc)) {  // no water from here up: wet3 is a test of the height
+        for (int m = k; m < ke; ++m, c += nxny) {
+          rhs[c] = 0.f;
+          prec[c] = 0.f;
+          codes[c] = 0;
+          pdry[c] = 0.f;
+          if (work.v[0]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) work.v[q][c] = 0.f;
+          }
+        }
+        break;
+      }
+      const float u0 = vel.u[ful], u1 = vel.u[ful + 1], v0 = vel.v[fvf], v1 = vel.v[fvf + g.nx], wt = vel.w[c + nxny];
+      float a[4] = {1.f, 1.f, 1.f, 1.f}, fn[4] = {1.f, 1.f, 1.f, 1.f}, frac_u = 1.f, owu = 1.f;
+      if (cut) {
+        a[0] = __ldg(g.ou + ful);
+        a[1] = __ldg(g.ou + ful + 1);
+        a[2] = __ldg(g.ov + fvf);
+        a[3] = __ldg(g.ov + fvf + g.nx);
+        owu = __ldg(g.ow + c + nxny);
+        if (k + 1 < g.nz) frac_u = __ldg(g.frac + c + nxny);
+#pragma unroll
+        for (int f = 0; f < 4; ++f) fn[f] = o.ok[f] ? __ldg(g.frac + c + nb[f]) : 0.f;
+      }
+      if (frac == 0.f) {
+        rhs[c] = 0.f;
+        prec[c] = 0.f;
+        codes[c] = 0;
+        pdry[c] = 0.f;
+        if (work.v[0]) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) work.v[q][c] = 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          o.a[f] = open[f] ? a[f] : 0.f;
+          o.sol[f] = !open[f] || fn[f] == 0.f;
+        }
+        o.down = ow;
+        o.up = owu;
+        o.sol_down = k > 0 ? frac_d == 0.f : true;
+        o.sol_up = k + 1 < g.nz ? frac_u == 0.f : true;
+        RowE row[6];
+        mobile_row_from(g, i, j, k, o, row);
+        // divergence_at
+        const float fl = cut ? a[0] * u0 : u0, fr = cut ? a[1] * u1 : u1;
+        const float ff = cut ? a[2] * v0 : v0, fk = cut ? a[3] * v1 : v1;
+        const float fb = cut ? ow * wb : wb, ft = cut ? owu * wt : wt;
+        float d = ((fr - fl + ft - fb) + (fk - ff)) / g.dx;
+        if (cut && g.wall) d = d + wall_flux(g, i, j, k);
+        const float b = rhs_row_store(g, row, scale * d, rhs, prec, codes, c);
+        if (work.v[0] && prec[c] == 0.f) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) work.v[q][c] = 0.f;
+        }
+        nonzero |= b != 0.f;
+        sum += (double)b * (double)b;
+      }
+      frac_d = frac;
+      frac = frac_u;
+      ow = owu;
+      wb = wt;
+    }
+  }
+  if (__syncthreads_or(nonzero) && threadIdx.x == 0) atomicOr(&S->any_nonzero, 1);
+  reduce_finish<RED_F64>(sum, 0, 1, red, S, FIN_B2);
 }
 
 // res = rhs - A p with res.res (FIN_RR0 or FIN_ACTUAL), from the row codes.

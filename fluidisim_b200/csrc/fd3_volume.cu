@@ -79,7 +79,8 @@ struct ScopedDevice {
 // Coarse levels of at most this many cells issue their passes' loads before the row code and the
 // gate, and restrict their residual in the same pass that computes it (k_level_restrict8).  These
 // are the latency-bound levels: measured 2% and 1.4% faster at 128^3; the loads ahead of the code
-// were 1% slower on the throughput-bound 128^3 level of a 256^3 volume.
+// were 1% slower on the throughput-bound 128^3 level of a 256^3 volume (3% with the rows before the wait, 9456 us a
+// solve against 9180).
 #ifndef FD3_SPEC_MAX
 #define FD3_SPEC_MAX 262144
 #endif
@@ -1125,6 +1126,22 @@ float vscale_k(const fd3_volume* V) {
   return V->half() ? (float)(6.0 * std::sqrt((double)V->n) / ((double)V->dx * (double)V->dx)) : 0.f;
 }
 
+// rhs, prec and row codes from the staged faces, p = 0 on the dry cells.  The march takes eight layers to a block where
+// that leaves every SM four blocks, fewer down to two on smaller volumes; a volume too narrow for its tiles (more
+// blocks than partial sums) and the ordered sums keep the pass of one cell per thread.
+void assemble_rows(fd3_volume* V, const Geo& G, float scale, const WorkVectors& work) {
+  const Faces vel{V->us, V->vs, V->ws};
+  const int tiles = ((V->nx + CM_X - 1) / CM_X) * ((V->ny + CM_Y - 1) / CM_Y);
+  int layers = 8;
+  auto blocks = [&] { return (long long)tiles * ((V->nz + layers - 1) / layers); };
+  while (layers > 2 && blocks() < 4 * 148) layers /= 2;
+  if (!V->ord() && blocks() <= V->p64_cap)
+    LAUNCH_G(V, k_rhs_march, (int)blocks(), CM_X * CM_Y, G, scale, vel, V->rhs, V->prec, V->red(), V->dS, V->codes, V->p,
+             work, layers);
+  else
+    DISPATCH(V, k_rhs_b2, V->n, G, scale, vel, V->rhs, V->prec, V->red(), V->dS, 1, V->codes, V->p, work);
+}
+
 // project_mobile3 (delta3d_mobile.rs:465-609), or, with V->linear, project (delta3d.rs:1060-1196):
 // the same loop and outer logic on the linear rows, CG or Jacobi-PCG, from p = 0 everywhere.
 int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_report* rep) {
@@ -1139,8 +1156,7 @@ int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_r
     CK(cudaMemsetAsync(V->p, 0, (size_t)V->n * sizeof(float), V->stream));
   } else {
     // the assembly also zeroes p on the dry cells (delta3d_mobile.rs:486-495)
-    DISPATCH(V, k_rhs_b2, V->n, G, scale, Faces{V->us, V->vs, V->ws}, V->rhs, V->prec, V->red(), V->dS, 1, V->codes, V->p,
-             V->skip_air ? WorkVectors{{V->res, V->dir, V->dir2, V->tmp}} : WorkVectors{});
+    assemble_rows(V, G, scale, V->skip_air ? WorkVectors{{V->res, V->dir, V->dir2, V->tmp}} : WorkVectors{});
     if (V->skip_air)
       LAUNCH_G(V, k_tile_tops, ((V->nx + TILE_X - 1) / TILE_X) * ((V->ny + TILE_Y - 1) / TILE_Y), TILE_X * TILE_Y, G,
                V->ztop);
