@@ -87,11 +87,14 @@ typedef struct fd3_options {
   uint32_t reduction;     /* fd3_reduction */
   uint32_t mg_max_levels; /* coarse levels kept by fd3_enable_multigrid; 0 = every level the
                              reference's coarsening rule allows (delta3d_multigrid.rs:73-88) */
-  uint32_t use_graphs;    /* 1 = run the inner PCG loop as a CUDA graph with a WHILE node */
+  uint32_t use_graphs;    /* 1 = run the inner loop without the host: in one cooperative launch
+                             (f64 sums; with the multigrid up to 2^20 cells at kernels = 0, without it
+                             while the blocks of one launch, one per SM, hold the volume), else as a
+                             CUDA graph with a WHILE node */
   uint32_t kernels;       /* fine-level kernels in f64 mode: 0 = 2.5-D blocked (default): on volumes
-                             of 2^23 cells or more with f32 storage the TMA-staged kernels (nx % 8 ==
-                             0) or four cells per thread (nx % 4 == 0), else two cells per thread
-                             (one when nx is odd); 1 = one cell per thread (the family the ordered
+                             of 1,500,000 cells or more with f32 storage the TMA-staged kernels
+                             (nx % 8 == 0), from 2^23 cells four cells per thread (nx % 4 == 0), else
+                             two cells per thread (one when nx is odd); 1 = one cell per thread (the family the ordered
                              mode always uses); 2 = 2.5-D blocked with one cell per thread; 3 = 2.5-D
                              blocked with two cells per thread; 4 = 2.5-D blocked with four cells per
                              thread (nx % 4 == 0, f32 storage); 5 = 2.5-D blocked, two cells per
@@ -103,7 +106,8 @@ typedef struct fd3_options {
                              waits on the device (results are identical either way) */
   uint32_t storage;       /* fd3_storage of the V-cycle vectors */
   uint32_t no_tile_skip;  /* 1 = the blocked fine kernels process the tiles of columns outside the
-                             sparse set too; 0 (default) = they skip them (results are identical) */
+                             sparse set and the air above the surface too; 0 (default) = they skip
+                             both (results are identical) */
   uint32_t reserved[1];
 } fd3_options;
 
