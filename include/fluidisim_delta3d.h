@@ -251,7 +251,9 @@ int fd3_advect_for_tests(fd3_volume* v, float dt);
  * fd3_project_mobile projects it, concurrently.  Every volume keeps its own stream and device-side
  * loop; `threads` host workers (0 = up to 16) issue them, largest first.  statuses[i] and
  * reports[i] are volume i's; the return value is FD3_OK unless the arguments are invalid (a null
- * pointer, or one volume listed twice). */
+ * pointer, or one volume listed twice).  A volume whose loop is one cooperative launch (see
+ * use_graphs) has every SM while it runs, so such volumes follow one another; at kernels = 3 they
+ * overlap.  fd3_batch_* is the faster way for many volumes. */
 int fd3_project_batch(fd3_volume* const* volumes, size_t count, const float* scales, const float* k1s,
                       uint32_t max_iters, int threads, fd3_report* reports, int* statuses);
 /* The persistent batch (no reference counterpart): many volumes (patches) projected by ONE kernel
