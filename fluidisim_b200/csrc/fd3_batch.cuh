@@ -197,7 +197,7 @@ __device__ __noinline__ float batch_row_general(const BatchShared& sh, unsigned 
                                                 float ym, float yp, float zm, float zp) {
   const Geo& g = sh.P.g;
   const int t = sh.nx[0].div(c), k = sh.ny[0].div(t);
-  return row_general(g, code, c - t * g.nx, t - k * g.ny, k, pc, xm, xp, ym, yp, zm, zp);
+  return row_general<true>(g, code, c - t * g.nx, t - k * g.ny, k, pc, xm, xp, ym, yp, zm, zp);
 }
 template <class P>
 __device__ __forceinline__ float batch_row(const BatchShared& sh, unsigned code, int c, float pc, P p) {

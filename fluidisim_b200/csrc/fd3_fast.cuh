@@ -80,13 +80,17 @@ __device__ __forceinline__ void rec_store(const Geo& g, int c, const float (&w)[
   R[0] = make_float4(w[0], w[1], w[2], w[3]);
   R[1] = make_float4(w[4], w[5], 0.f, 0.f);
 }
+// The records come through the read-only path, which is defined only for memory that no thread writes while the kernel
+// runs; SAME_LAUNCH: this kernel wrote them itself (the persistent batch), so they are read with plain loads.
+template <bool SAME_LAUNCH = false>
 __device__ __forceinline__ float row_general(const Geo& g, unsigned code, int i, int j, int k, float pc, float xm,
                                              float xp, float ym, float yp, float zm, float zp) {
   float acc = 0.f;
   if (rec_kept(g, code)) {
     const float4* R = g.rec + 2 * (size_t)((k * g.ny + j) * g.nx + i);
-    const float4 a = __ldg(R);
-    const float2 b = __ldg(reinterpret_cast<const float2*>(R + 1));
+    const float2* R2 = reinterpret_cast<const float2*>(R + 1);
+    const float4 a = SAME_LAUNCH ? *R : __ldg(R);
+    const float2 b = SAME_LAUNCH ? *R2 : __ldg(R2);
     const float w[6] = {a.x, a.y, a.z, a.w, b.x, b.y}, v[6] = {xm, xp, ym, yp, zm, zp};
 #pragma unroll
     for (int f = 0; f < 6; ++f) {
