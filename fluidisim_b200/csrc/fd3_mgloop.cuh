@@ -1,17 +1,16 @@
 // The multigrid PCG loop in one cooperative launch, for volumes whose passes are latency.
 //
-// In the loop graph an iteration of a 128^3 volume is seventeen kernels, and 4 us of each is its launch boundary, the
-// gate, and the chain of loads before its first sum: 150 us per iteration, when the passes' work is a third of
-// that.  Here one CTA per SM stays for the whole loop, the passes are separated by grid meetings (GridTeam: 1.3 us, 2.1
-// with a sum), and the scalars are on chip.  The fine passes are the paired march's (fd3_zmarch2.cuh) with three teams
-// of 256 threads per CTA, each taking chunks of a tile in turn; the levels run one cell per thread, their warps
-// spread over the SMs; the levels of at most TAIL_REG_THREADS cells run in the first CTA, its rows kept in shared
-// memory for the whole loop.
+// In the loop graph an iteration is seventeen kernels or so, and 4 us of each is its launch boundary, the gate, and the
+// chain of loads before its first sum, when the passes' work is a third of that.  Here a grid of CTAs, one to an SM,
+// stays for the whole loop, the passes are separated by grid meetings (GridTeam: 1.3 us on 148 CTAs, 2.1 with a sum), and
+// the scalars are on chip.  The fine passes are the paired march's (fd3_zmarch2.cuh) with three teams of 256 threads per
+// CTA, each taking chunks of a tile in turn; the levels run one cell per thread, their warps spread over the CTAs; the
+// levels of at most TAIL_REG_THREADS cells run in the first CTA, its rows kept in shared memory for the whole loop.
 //
-// Every cell value is that of the separate kernels; the f64 sums are added in the order of the chunks here.  Whole
-// projections, separate kernels and one launch (B200): 64^3 basin 1.49 and 1.27 ms, a 12288-cell time step 0.90 and
-// 0.79, 96^3 1.89 and 1.85; above 2^20 cells the separate kernels, whose chunks the hardware deals as SMs free up,
-// are faster (a team's chunk takes 9 us, the slowest 15, at 128^3).
+// Every cell value is that of the separate kernels; the f64 sums have a part per chunk, added in the order of the chunks,
+// so the result is the same on any number of CTAs, and a volume beside others takes fewer (fd3_volume::mg_ctas).  Whole
+// projections, separate kernels and one launch alone on a B200: 64^3 1.04 and 0.98 ms, 48^3 1.00 and 0.91, 32^3 0.77 and
+// 0.73, 32 x 16 x 24 0.61 and 0.59.
 #pragma once
 
 #include "fd3_persist.cuh"
@@ -22,6 +21,8 @@ namespace fd3 {
 constexpr int MG_TEAMS = 3;
 constexpr int MG_THREADS = MG_TEAMS * Z2T;  // one CTA per SM, 80 registers
 constexpr int MG_LEVELS = 8;                // levels above the tail
+constexpr int MG_MIN_CTAS = 16;             // of a volume alone: 32 x 16 x 24 takes 0.59 ms on 16, 0.60 on 8, 0.77 on 4
+constexpr int MG_LEAST_SHARE = 8;           // beside many others (sixteen 64^3 at once, ms: 3.7 on 8, 5.9 on 4)
 
 struct MgLoop {
   Geo g;
@@ -43,7 +44,6 @@ struct MgShared {
   ZResid2 tr[MG_TEAMS][2];
   TailShared tail;
   GridShared grid;
-  int chunk;  // layers of a chunk
 };
 
 struct TeamSync {
@@ -54,8 +54,10 @@ struct TeamSync {
 };
 
 // Layers of a chunk: the even number that makes the longest team's march shortest, a chunk of K layers counting K + 2
-// (its halo layers) and the teams taking the chunks that hold water in turn.
-__device__ __forceinline__ int mg_pick_chunk(const Geo& g, int teams, int* cost) {
+// (its halo layers) and GRID_PARTS teams taking the chunks that hold water in turn; at most GRID_PARTS chunks.  It does
+// not depend on the grid, nor do the sums, whose parts are the chunks.
+__device__ __forceinline__ int mg_pick_chunk(const Geo& g, int* cost) {
+  constexpr int teams = GRID_PARTS;
   const int ntx = (g.nx + Z2X - 1) / Z2X, nty = (g.ny + Z2Y - 1) / Z2Y;
   if (threadIdx.x < 8) cost[threadIdx.x] = 0;
   __syncthreads();
@@ -70,8 +72,11 @@ __device__ __forceinline__ int mg_pick_chunk(const Geo& g, int teams, int* cost)
     const int k = 2 + 2 * q, c = (cost[q] + teams - 1) / teams * (k + 2);
     if (c < least) { least = c; best = k; }
   }
-  return best;
+  const int high = GRID_PARTS / (ntx * nty);  // chunks of a tile, at least one (mg_fits)
+  return max(best, 2 * (((g.nz + high - 1) / high + 1) / 2));
 }
+
+inline bool mg_fits(int nx, int ny) { return ((nx + Z2X - 1) / Z2X) * ((ny + Z2Y - 1) / Z2Y) <= GRID_PARTS; }
 
 template <class T>
 __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant__ MgLoop a) {
@@ -84,7 +89,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
   GridTeam<MG_THREADS> grid(a.slots, sh.grid);
   const int tid = threadIdx.x, team = tid / Z2T, tx = tid & 31, ty = (tid >> 5) & 7, teams = gridDim.x * MG_TEAMS;
   const int ntx = (g.nx + Z2X - 1) / Z2X, nty = (g.ny + Z2Y - 1) / Z2Y, tiles = ntx * nty;
-  const int K = mg_pick_chunk(g, teams, reinterpret_cast<int*>(sh.grid.warp));
+  const int K = mg_pick_chunk(g, reinterpret_cast<int*>(sh.grid.warp));
   __syncthreads();
   const int chunks = tiles * ((g.nz + K - 1) / K);
   const bool first_cta = blockIdx.x == 0;
@@ -93,14 +98,34 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
   T* z2 = static_cast<T*>(a.z2);
   const TeamSync sync{6 + team};
   // f(march) over the chunks of this thread's team: the chunks in order of height, dealt to the CTAs first
+  auto march_at = [&](int q) {
+    const int tile = q % tiles;
+    return March2<TeamSync>{g,  a.codes,       ztile2_at(g, tile % ntx, tile / ntx, q / tiles * K, K, tx, ty), tx,
+                            ty, sh.sbuf[team], sh.tr[team], sync};
+  };
   auto each_chunk = [&](auto f) {
     for (int q = team * gridDim.x + blockIdx.x; q < chunks; q += teams) {
-      const int tile = q % tiles;
-      const March2<TeamSync> march{g,  a.codes,       ztile2_at(g, tile % ntx, tile / ntx, q / tiles * K, K, tx, ty), tx,
-                                   ty, sh.sbuf[team], sh.tr[team], sync};
-      f(march);
+      f(march_at(q));
       sync();  // the planes are free for the next chunk
     }
+  };
+  // the same with the sum of what f(march) returns over every thread and chunk, a part per chunk; a meeting
+  auto sum_chunks = [&](bool& met, auto f) -> double {
+    int half = 0;
+    for (int q = team * gridDim.x + blockIdx.x; q < chunks; q += teams, half ^= 1) {
+      double acc = f(march_at(q));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (tx == 0) sh.grid.warp[0][tid >> 5][half] = acc;
+      sync();
+      if (tx == 0 && ty == 0) {  // the other half is written meanwhile, this one after the next chunk's sync
+        double part = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) part += sh.grid.warp[0][(tid >> 5) + w][half];
+        __stcg(grid.next_parts() + q, part);
+      }
+    }
+    return grid.sum_parts(chunks, met);
   };
   // f(i) for i = 0 .. n - 1 (a multiple of 32 rounded up), whole warps, spread over the SMs warp by warp
   auto each_warp = [&](int n, auto f) {
@@ -173,17 +198,19 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
     }
     each_chunk([&](const auto& m) { march_post1(m, a.prec, a.r, (const T*)z, L0, levels ? 1 : 0, z2, rs); });
     if (!grid.meet()) return false;
-    double acc = 0.0, none = 0.0;
-    each_chunk([&](const auto& m) { march_post2(m, a.prec, a.r, (const T*)z2, z, rs, acc); });
-    if (!grid.template sum<false>(acc, none)) return false;
-    rz = acc;
-    return true;
+    bool met;
+    rz = sum_chunks(met, [&](const auto& m) {
+      double acc = 0.0;
+      march_post2(m, a.prec, a.r, (const T*)z2, z, rs, acc);
+      return acc;
+    });
+    return met;
   };
 
   const double tolb2 = S->tolb2, phys = S->phys;
   const unsigned max_iters = S->max_iters;
   const float vk = S->vk;
-  double rr = S->rr, rn = rr, rz = 0.0, none = 0.0;
+  double rr = S->rr, rn = rr, rz = 0.0;
   unsigned it = S->it;
   int status = 0, brk = 0, mode = 0;
   float beta = 0.f;
@@ -201,15 +228,21 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
     rz = zn;
     const float* din = a.dir[it & 1];
     float* dout = a.dir[(it & 1) ^ 1];
-    double dq = 0.0;
-    each_chunk([&](const auto& m) { march_dir(m, (const T*)z, din, dout, a.q, mode, beta, dq); });
-    if (!grid.template sum<false>(dq, none)) { status = 100; break; }
+    bool met;
+    const double dq = sum_chunks(met, [&](const auto& m) {
+      double acc = 0.0;
+      march_dir(m, (const T*)z, din, dout, a.q, mode, beta, acc);
+      return acc;
+    });
+    if (!met) { status = 100; break; }
     if (!(dq > 0.0)) { brk = 1; break; }  // FIN_DQ
     const float alpha = (float)(rz / dq);
-    double acc = 0.0;
-    each_chunk([&](const auto& m) { chunk_update(g, m.t, alpha, a.p, a.r, dout, a.q, acc); });
-    if (!grid.template sum<false>(acc, none)) { status = 100; break; }
-    rn = acc;
+    rn = sum_chunks(met, [&](const auto& m) {
+      double acc = 0.0;
+      chunk_update(g, m.t, alpha, a.p, a.r, dout, a.q, acc);
+      return acc;
+    });
+    if (!met) { status = 100; break; }
     if (!isfinite(rn)) { status = 2; break; }  // FIN_RN
     if (vk > 0.f && rn > 0.0) vinv = (float)((double)vk / sqrt(rn));
     if (!((rn > tolb2 || rn > phys) && it + 1 < max_iters)) { rr = rn; ++it; break; }

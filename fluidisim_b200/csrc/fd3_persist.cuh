@@ -4,7 +4,7 @@
 // Without the multigrid an iteration is four short passes, and as separate kernels each pays a launch
 // boundary, a chain of dependent loads (gate, codes, operands) and the last block's merge of the
 // partials: 26 us per iteration at 215k cells, 19 at 65k, where the passes' bytes take 1 us from L2.
-// Here one CTA per SM keeps its cells' p, r, diagonal and row on chip for the whole loop, and the
+// Here CTAs, one to an SM, keep their cells' p, r, diagonal and row on chip for the whole loop, and the
 // iteration has two grid-wide meetings, each a reduction and a barrier at once (GridTeam::sum).
 // Between them a cell exchanges with its neighbours only z and the last direction, through L2.
 //
@@ -30,13 +30,17 @@ constexpr unsigned GRID_POLLS = 1u << 20;
 // partial, took 5.6 us (148 x 148 polls of the same lines), and mailboxes per reader 2.6 us.  The slots
 // alternate between two sets: a CTA writes a set again only after a later meeting, which every CTA has
 // reached only after reading it.
+constexpr int GRID_PARTS = 444;  // parts of a sum, at most (sum_parts): three teams on each of 148 SMs
 struct GridSlots {
   double2 part[2][GRID_MAX_CTAS];
+  double parts[2][GRID_PARTS];
   unsigned arrived;
 };
+constexpr int GRID_STAND_IN = 4;  // CTAs that one stands in for, at most
 struct GridShared {
-  double warp[32][2];
+  double warp[GRID_STAND_IN][32][2];
   double sum[2];
+  double parts[GRID_PARTS / 32 + 1];
 };
 template <int THREADS>
 struct GridTeam {
@@ -66,34 +70,39 @@ struct GridTeam {
     return !__syncthreads_or(late);
   }
   // Sums a (and b, when TWO) over every thread of the grid: the same totals, added in the same order, for
-  // every thread.  A meeting.
-  template <bool TWO>
-  __device__ __forceinline__ bool sum(double& a, double& b) {
+  // every thread, in a[0] and b[0].  A meeting.  The sum is that of `slots_used` CTAs with one value per thread; a thread
+  // that stands in for V of them (CTAs blockIdx.x + v gridDim.x) has the values of all: a[v] and b[v].
+  template <bool TWO, int V>
+  __device__ __forceinline__ bool sum(double (&a)[V], double (&b)[V], int slots_used) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (TWO) b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if (lane == 0) {
-      sh.warp[wid][0] = a;
-      if (TWO) sh.warp[wid][1] = b;
+    for (int v = 0; v < V; ++v) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        a[v] += __shfl_xor_sync(0xffffffffu, a[v], o);
+        if (TWO) b[v] += __shfl_xor_sync(0xffffffffu, b[v], o);
+      }
+      if (lane == 0) {
+        sh.warp[v][wid][0] = a[v];
+        if (TWO) sh.warp[v][wid][1] = b[v];
+      }
     }
     __syncthreads();
     double2* half = slots->part[meeting & 1u];
     bool late = false;
-    if (threadIdx.x == 0) {
+    const int slot = (int)(blockIdx.x + threadIdx.x * gridDim.x);
+    if ((int)threadIdx.x < V && (V == 1 || slot < slots_used)) {
       double2 p = make_double2(0.0, 0.0);
 #pragma unroll
       for (int q = 0; q < THREADS / 32; ++q) {
-        p.x += sh.warp[q][0];
-        if (TWO) p.y += sh.warp[q][1];
+        p.x += sh.warp[threadIdx.x][q][0];
+        if (TWO) p.y += sh.warp[threadIdx.x][q][1];
       }
-      __stcg(half + blockIdx.x, p);
-      late = !arrive_and_wait();
-    } else {
-      ++meeting;
+      __stcg(half + slot, p);
     }
+    if (V > 1 && wid == 0) __syncwarp();  // the other threads' slots before the first arrives
+    if (threadIdx.x == 0) late = !arrive_and_wait();
+    else ++meeting;
     if (__syncthreads_or(late)) return false;
     if (wid == 0) {
       constexpr int PER = (GRID_MAX_CTAS + 31) / 32;
@@ -101,28 +110,48 @@ struct GridTeam {
 #pragma unroll
       for (int e = 0; e < PER; ++e) {
         const int q = lane + 32 * e;
-        v[e] = q < (int)gridDim.x ? __ldcg(half + q) : make_double2(0.0, 0.0);
+        v[e] = q < (V == 1 ? (int)gridDim.x : slots_used) ? __ldcg(half + q) : make_double2(0.0, 0.0);
       }
-      a = b = 0.0;
+      double x = 0.0, y = 0.0;
 #pragma unroll
       for (int e = 0; e < PER; ++e) {
-        a += v[e].x;
-        if (TWO) b += v[e].y;
+        x += v[e].x;
+        if (TWO) y += v[e].y;
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (TWO) b += __shfl_xor_sync(0xffffffffu, b, o);
+        x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (TWO) y += __shfl_xor_sync(0xffffffffu, y, o);
       }
       if (lane == 0) {
-        sh.sum[0] = a;
-        sh.sum[1] = b;
+        sh.sum[0] = x;
+        sh.sum[1] = y;
       }
     }
     __syncthreads();
-    a = sh.sum[0];
-    b = sh.sum[1];
+    a[0] = sh.sum[0];
+    b[0] = sh.sum[1];
     return true;
+  }
+  // Where the parts of the next sum_parts go: parts 0 .. n - 1, each written by one thread of the grid.
+  __device__ __forceinline__ double* next_parts() { return slots->parts[meeting & 1u]; }
+  // The sum of n <= min(THREADS, GRID_PARTS) parts, in an order that depends on n alone: the same total for every
+  // thread of any grid.  A meeting.
+  __device__ __forceinline__ double sum_parts(int n, bool& met) {
+    const double* parts = next_parts();
+    met = meet();
+    if (!met) return 0.0;
+    const int warps = (n + 31) >> 5;
+    if ((int)threadIdx.x < 32 * warps) {
+      double v = (int)threadIdx.x < n ? __ldcg(parts + threadIdx.x) : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if ((threadIdx.x & 31) == 0) sh.parts[threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    double a = sh.parts[0];
+    for (int q = 1; q < warps; ++q) a += sh.parts[q];
+    return a;
   }
 };
 
@@ -183,10 +212,13 @@ __device__ __forceinline__ float apply_kept(const Geo& g, unsigned code, int c, 
 // Per iteration: d = z + beta d at the cell and, recomputed from z and the previous d, at its neighbours;
 // q = A d; d.q | p += alpha d, r -= alpha q, z = prec r; r.r and r.z together.  z and the two
 // alternating direction buffers live in global memory, read past L1 (other SMs write them).
-template <int CELLS>
+//
+// The sums are those of a grid of `ctas` CTAs, whatever the grid: with fewer, a CTA stands in for V of them and its threads
+// own the cells of as many (a batch runs its volumes on a part of the SMs each, and a volume has the same bits there).
+template <int CELLS, int V>
 __global__ void __launch_bounds__(GRID_THREADS, 1)
     k_cg_loop(const __grid_constant__ Geo g, const unsigned short* __restrict__ codes, const float* __restrict__ prec, float* p,
-              float* r, float* d0, float* d1, float* z, Scalars* S, GridSlots* slots) {
+              float* r, float* d0, float* d1, float* z, Scalars* S, GridSlots* slots, int ctas) {
   asm volatile("griddepcontrol.wait;" ::: "memory");  // no early start of the next kernel: its CTAs find no room
   if (!S->active) return;
   extern __shared__ float kept[];  // [CELLS][7][GRID_THREADS]: six coefficients and p
@@ -195,13 +227,24 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
   auto K = [&](int s, int f) -> float& { return kept[(s * 7 + f) * GRID_THREADS + threadIdx.x]; };
   constexpr int PAIR = CELLS < 2 ? 1 : 2;
   const int nxny = g.nx * g.ny;
-  const int T = gridDim.x * GRID_THREADS, t0 = blockIdx.x * GRID_THREADS + threadIdx.x;
+  // cell s of this thread (n or more: none): cell s % EACH of the thread's place in CTA s / EACH of those it stands in for
+  constexpr int EACH = CELLS / V;
+  const int T = (V == 1 ? (int)gridDim.x : ctas) * GRID_THREADS, t0 = blockIdx.x * GRID_THREADS + threadIdx.x;
+  auto cell = [&](int s) {
+    if (V == 1) return t0 + s * T;
+    const int v = s / EACH * (int)gridDim.x;
+    return (int)blockIdx.x + v < ctas ? t0 + v * GRID_THREADS + s % EACH * T : g.n;
+  };
   float rc[CELLS], mc[CELLS], dc[CELLS], qc[CELLS];
   unsigned code[CELLS];
-  double acc = 0.0, acc2 = 0.0;
+  double acc[V] = {}, acc2[V] = {};
+  auto clear = [&] {
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[v] = acc2[v] = 0.0;
+  };
 #pragma unroll
   for (int s = 0; s < CELLS; ++s) {
-    const int c = t0 + s * T;
+    const int c = cell(s);
     rc[s] = mc[s] = dc[s] = qc[s] = 0.f;
     code[s] = 0u;
     if (c < g.n) {
@@ -219,7 +262,7 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
         for (int f = 0; f < 6; ++f) K(s, f) = w[f];
       }
       z[c] = mc[s] * rc[s];
-      acc += (double)rc[s] * (double)mc[s] * (double)rc[s];
+      acc[s / EACH] += (double)rc[s] * (double)mc[s] * (double)rc[s];
     }
   }
   double rz, rr = S->rr;
@@ -230,19 +273,18 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
   float beta = 0.f;
   float* din = d0;
   float* dout = d1;
-  if (!team.sum<false>(acc, acc2)) status = 100;
-  rz = acc;
+  if (!team.template sum<false, V>(acc, acc2, ctas)) status = 100;
+  rz = acc[0];
   if (!status && !isfinite(rz)) status = 2;
   while (!status) {
-    acc = 0.0;
-    acc2 = 0.0;
+    clear();
     // PAIR cells' twelve loads each go out together; the stores of the direction come after them all
 #pragma unroll
     for (int s0 = 0; s0 < CELLS; s0 += PAIR) {
       float v[PAIR][6];
 #pragma unroll
       for (int e = 0; e < PAIR; ++e) {
-        const int s = s0 + e, c = t0 + s * T;
+        const int s = s0 + e, c = cell(s);
         if (s >= CELLS) continue;
         const int nb[6] = {c - 1, c + 1, c - g.nx, c + g.nx, c - nxny, c + nxny};
         float zn[6], dn[6];
@@ -257,52 +299,51 @@ __global__ void __launch_bounds__(GRID_THREADS, 1)
       }
 #pragma unroll
       for (int e = 0; e < PAIR; ++e) {
-        const int s = s0 + e, c = t0 + s * T;
+        const int s = s0 + e, c = cell(s);
         if (s >= CELLS) continue;
         const float zc = mc[s] * rc[s];
         const float d = beta == 0.f ? zc : zc + beta * dc[s];
         qc[s] = (code[s] & RC_WET) ? apply_kept(g, code[s], c, d, [&](int f) { return K(s, f); }, v[e]) : 0.f;
         dc[s] = d;
-        acc += (double)d * (double)qc[s];
+        acc[s / EACH] += (double)d * (double)qc[s];
       }
     }
 #pragma unroll
     for (int s = 0; s < CELLS; ++s) {
-      const int c = t0 + s * T;
+      const int c = cell(s);
       if (c < g.n) dout[c] = dc[s];
     }
-    if (!team.sum<false>(acc, acc2)) { status = 100; break; }
-    if (!(acc > 0.0)) { brk = 1; break; }  // FIN_DQ
-    const float alpha = (float)(rz / acc);
-    acc = 0.0;
-    acc2 = 0.0;
+    if (!team.template sum<false, V>(acc, acc2, ctas)) { status = 100; break; }
+    if (!(acc[0] > 0.0)) { brk = 1; break; }  // FIN_DQ
+    const float alpha = (float)(rz / acc[0]);
+    clear();
 #pragma unroll
     for (int s = 0; s < CELLS; ++s) {
-      const int c = t0 + s * T;
+      const int c = cell(s);
       if (c < g.n) {
         K(s, 6) += alpha * dc[s];
         const float rn = rc[s] - alpha * qc[s];
         rc[s] = rn;
         z[c] = mc[s] * rn;
-        acc += (double)rn * (double)rn;
-        acc2 += (double)rn * (double)mc[s] * (double)rn;
+        acc[s / EACH] += (double)rn * (double)rn;
+        acc2[s / EACH] += (double)rn * (double)mc[s] * (double)rn;
       }
     }
-    if (!team.sum<true>(acc, acc2)) { status = 100; break; }
-    if (!isfinite(acc)) { status = 2; break; }  // FIN_RN
+    if (!team.template sum<true, V>(acc, acc2, ctas)) { status = 100; break; }
+    if (!isfinite(acc[0])) { status = 2; break; }  // FIN_RN
     ++it;
-    rr = acc;
-    if (!((acc > tolb2 || acc > phys) && it < max_iters)) break;
-    if (!isfinite(acc2)) { status = 2; break; }  // FIN_RZ_ITER
-    beta = (float)(acc2 / rz);
-    rz = acc2;
+    rr = acc[0];
+    if (!((rr > tolb2 || rr > phys) && it < max_iters)) break;
+    if (!isfinite(acc2[0])) { status = 2; break; }  // FIN_RZ_ITER
+    beta = (float)(acc2[0] / rz);
+    rz = acc2[0];
     float* t = din;
     din = dout;
     dout = t;
   }
 #pragma unroll
   for (int s = 0; s < CELLS; ++s) {
-    const int c = t0 + s * T;
+    const int c = cell(s);
     if (c < g.n) { p[c] = K(s, 6); r[c] = rc[s]; }
   }
   // every CTA has met for the last time here, but one that gave up says so whichever it is

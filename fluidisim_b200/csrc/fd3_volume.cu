@@ -95,10 +95,11 @@ constexpr long long kQuadMinCells = 1LL << 23;
 // The TMA-staged kernels by default from this many cells (projections, ms, paired / TMA-staged: 112^3 basin 2.25 / 2.33;
 // 160 x 80 x 120 tank 4.26 / 4.08; 128^3 basin 2.60 / 2.53; 160^3 3.94 / 3.61; 256^3 wave 10.25 / 9.38).
 constexpr long long kTmaMinCells = 1500000;
-// The loop in one launch (k_mg_loop) up to this many cells (ms, separate kernels / one launch: 64^3 basin 1.49 / 1.27,
-// 80^3 1.63 / 1.51, 128 x 64 x 96 tank 1.84 / 1.78, 96^3 1.89 / 1.85, 112^3 2.25 / 2.22, 128^3 2.60 / 2.87, 160 x 80 x 120
-// tank 4.26 / 4.82): above, its slowest team's chunks cost more than the launches it saves.
-constexpr long long kLoopMaxCells = 1LL << 20;
+// The loop in one launch (k_mg_loop) up to this many cells (projections, ms, separate kernels / one launch on half of the
+// SMs, as it runs: 48^3 1.00 / 0.91, 64^3 1.04 / 0.98, 64 x 64 x 80 1.14 / 1.17, 128 x 64 x 48 1.11 / 1.25, 72^3 1.55 / 1.94).
+// With every SM it would win up to 400,000 cells (1.08, 1.02 and 1.57; 128 x 64 x 96 1.36 / 1.43, 96^3 1.56 / 1.65), but then
+// volumes on several streams would follow one another.
+constexpr long long kLoopMaxCells = 1LL << 18;
 
 // Coarse levels of at most this many cells are solved together by one CTA (k_coarse_tail).
 constexpr int TAIL_MAX_CELLS = 512;
@@ -166,8 +167,9 @@ struct fd3_volume {
   int p64_cap = 0;  // f64 partial slots
   float* p32 = nullptr;
   unsigned* count = nullptr;
-  GridSlots* slots = nullptr;  // the meetings of k_cg_loop
+  GridSlots* slots = nullptr;  // the meetings of k_cg_loop and k_mg_loop
   int grid_ctas = 0;          // CTAs of the cooperative launches (one per SM; 0: not to be had)
+  int workers = 1;            // volumes that fd3_project_batch projects at once, this one among them
   Scalars* dS = nullptr;
   Scalars* hS = nullptr;  // pinned
   int* dflag = nullptr;
@@ -265,7 +267,17 @@ struct fd3_volume {
   // kLoopMaxCells.  Profiling, use_graphs = 0 and kernels = 3 keep the separate kernels.
   bool mg_loop() const {
     return opt.kernels == 0 && paired() && mg_on() && (long long)n <= kLoopMaxCells && opt.use_graphs && !prof &&
-           grid_ctas > 0 && tail_reg && tail_first <= MG_LEVELS;
+           grid_ctas > 0 && tail_reg && tail_first <= MG_LEVELS && mg_fits(nx, ny);
+  }
+  // Its CTAs, which fill an SM each: a team (three to a CTA) per chunk of two layers, but at most half of the SMs, so that
+  // volumes on two streams run side by side, and an equal share of them among the workers of fd3_project_batch.  The
+  // result does not depend on it.  Measured (ms, 148 / 74 / 37 CTAs): 64^3 alone 0.94 / 0.98 / 1.23, two at once 1.90 / 1.12 /
+  // 1.39, sixteen 14.7 / 8.0 / 5.4 (3.4 at 9); 32^3 alone 0.70 / 0.70 / 0.71 (0.73 at 22, 0.75 at 16), sixteen 10.0 / 5.1 / 2.8
+  // (1.35 at 9).  256 patches by sixteen workers: 217 with every SM each, 65 as separate kernels, 42 so.
+  int mg_ctas() const {
+    const int chunks = ((nx + Z2X - 1) / Z2X) * ((ny + Z2Y - 1) / Z2Y) * ((nz + 1) / 2);
+    const int share = std::max(MG_LEAST_SHARE, grid_ctas / std::max(workers, 2));
+    return std::min({std::max(MG_MIN_CTAS, (chunks + MG_TEAMS - 1) / MG_TEAMS), share, grid_ctas});
   }
   bool one_launch() const { return cg_loop() || mg_loop(); }
   Red red() const { return Red{p64, p32, count}; }
@@ -309,11 +321,13 @@ int cooperative_ctas(int device, int* ctas) {
     int sms = 0, coop = 0, least = 1, resident = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
-    CK(cudaFuncSetAttribute(k_cg_loop<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(4)));
-    CK(cudaFuncSetAttribute(k_cg_loop<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(8)));
-    CK(cudaFuncSetAttribute(k_cg_loop<GRID_MAX_CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    CK(cudaFuncSetAttribute(k_cg_loop<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(4)));
+    CK(cudaFuncSetAttribute(k_cg_loop<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(4)));
+    CK(cudaFuncSetAttribute(k_cg_loop<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(4)));
+    CK(cudaFuncSetAttribute(k_cg_loop<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cg_smem(8)));
+    CK(cudaFuncSetAttribute(k_cg_loop<GRID_MAX_CELLS, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)cg_smem(GRID_MAX_CELLS)));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_cg_loop<GRID_MAX_CELLS>, GRID_THREADS,
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_cg_loop<GRID_MAX_CELLS, 1>, GRID_THREADS,
                                                      cg_smem(GRID_MAX_CELLS)));
     least = std::min(least, resident);
     for (auto k : {k_mg_loop<float>, k_mg_loop<__half>}) {
@@ -918,12 +932,12 @@ int build_loop_graph(fd3_volume* V) {
 }
 
 // The inner loop without the multigrid, prime included, as one cooperative launch.
-template <int CELLS>
+template <int CELLS, int STANDS_IN = 1>
 void launch_cg_loop(fd3_volume* V, int ctas) {
   cudaEvent_t a = nullptr, b = nullptr;
   if (V->prof) { a = next_event(V); cudaEventRecord(a, V->stream); }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ctas);
+  cfg.gridDim = dim3((ctas + STANDS_IN - 1) / STANDS_IN);
   cfg.blockDim = dim3(GRID_THREADS);
   cfg.dynamicSmemBytes = cg_smem(CELLS);
   cfg.stream = V->stream;
@@ -932,8 +946,8 @@ void launch_cg_loop(fd3_volume* V, int ctas) {
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_cg_loop<CELLS>, V->geo(), (const unsigned short*)V->codes, (const float*)V->prec, V->p,
-                     V->res, V->dir, V->dir2, V->tmp, V->dS, V->slots);
+  cudaLaunchKernelEx(&cfg, k_cg_loop<CELLS, STANDS_IN>, V->geo(), (const unsigned short*)V->codes, (const float*)V->prec,
+                     V->p, V->res, V->dir, V->dir2, V->tmp, V->dS, V->slots, ctas);
   if (V->prof) { b = next_event(V); cudaEventRecord(b, V->stream); V->pending.push_back({"k_cg_loop", a, b}); }
   V->launches++;
 }
@@ -941,7 +955,13 @@ void run_cg_loop(fd3_volume* V) {
   LAUNCH_G(V, k_grid_reset, 1, 1, V->slots);
   const int ctas = std::min(V->grid_ctas, (V->n + GRID_THREADS - 1) / GRID_THREADS);
   const int cells = (V->n + ctas * GRID_THREADS - 1) / (ctas * GRID_THREADS);
-  if (cells <= 1) launch_cg_loop<1>(V, ctas);
+  // Beside other volumes: a half of the CTAs, or a quarter, each standing in for the others.  Sixteen volumes by sixteen
+  // workers, ms, whole grids / so: 40,095 cells 10.1 / 3.2, 66,185 11.8 / 5.0, 77,775 8.4 / 5.5, 111,569 12.4 / 8.3.  From three
+  // cells per thread on the SMs are as full either way (215,025 cells: 20.5 whole, 23.2 on half as many).
+  if (cells <= 1 && V->workers >= 4) launch_cg_loop<4, 4>(V, ctas);
+  else if (cells <= 1 && V->workers > 1) launch_cg_loop<2, 2>(V, ctas);
+  else if (cells <= 2 && V->workers > 1) launch_cg_loop<4, 2>(V, ctas);
+  else if (cells <= 1) launch_cg_loop<1>(V, ctas);
   else if (cells <= 2) launch_cg_loop<2>(V, ctas);
   else if (cells <= 3) launch_cg_loop<3>(V, ctas);
   else if (cells <= 4) launch_cg_loop<4>(V, ctas);
@@ -966,7 +986,7 @@ void launch_mg_loop(fd3_volume* V) {
   a.S = V->dS;
   a.slots = V->slots;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(V->grid_ctas);
+  cfg.gridDim = dim3(V->mg_ctas());
   cfg.blockDim = dim3(MG_THREADS);
   cfg.dynamicSmemBytes = sizeof(MgShared);
   cfg.stream = V->stream;
@@ -2378,7 +2398,9 @@ int fd3_project_batch(fd3_volume* const* vols, size_t count, const float* scales
       if (q >= count) break;
       const size_t i = order[q];
       cudaSetDevice(vols[i]->device);
+      vols[i]->workers = (int)T;
       statuses[i] = fd3_project_mobile(vols[i], scales[i], k1s[i], max_iters, &reports[i]);
+      vols[i]->workers = 1;
     }
   };
   std::vector<std::thread> pool;
