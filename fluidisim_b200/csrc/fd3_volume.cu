@@ -128,7 +128,7 @@ struct fd3_volume {
   float *us = nullptr, *vs = nullptr, *ws = nullptr, *p = nullptr, *rhs = nullptr, *res = nullptr;
   float *dir = nullptr, *dir2 = nullptr, *tmp = nullptr, *prec = nullptr;
   unsigned short* codes = nullptr;  // row codes of the current projection
-  float4* rec = nullptr;            // its rows that are not plain (Geo::rec); none above kRecMaxCells
+  float4* rec = nullptr;            // its rows that are not plain (Geo::rec); none above kRecMaxCells or without memory
   float *sv_u = nullptr, *sv_v = nullptr, *sv_w = nullptr, *sv_p = nullptr, *sv_eta = nullptr, *sv_rof = nullptr;
   float *flux_x = nullptr, *flux_y = nullptr;
   // a volume configured with a solid: its node SDF buffer and the bottom-only base geometry the
@@ -285,6 +285,28 @@ struct fd3_volume {
 
 namespace {
 
+// The row records given back, when another array needs their memory: they save time, and without them the rows are
+// rebuilt.  The captured loop holds their address.
+bool drop_records(fd3_volume* V) {
+  auto at = std::find(V->allocations.begin(), V->allocations.end(), (void*)V->rec);
+  if (!V->rec || at == V->allocations.end()) return false;  // small records share a chunk
+  cudaStreamSynchronize(V->stream);
+  if (V->loop_exec) cudaGraphExecDestroy(V->loop_exec);
+  V->loop_exec = nullptr;
+  V->allocations.erase(at);
+  cudaFree(V->rec);
+  V->rec = nullptr;
+  return true;
+}
+cudaError_t device_alloc(fd3_volume* V, void** q, size_t size) {
+  for (;;) {
+    const cudaError_t e = cudaMalloc(q, size);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();  // reported from here, not by the next launch's check
+    if (!drop_records(V)) return e;
+  }
+}
+
 // Zeroed device memory of the volume's.  Arrays below kArenaMax share chunks of kArenaChunk bytes: a volume has some
 // fifty arrays, a cudaMalloc takes 0.2 ms and more, and a batch configures hundreds of small volumes.
 constexpr size_t kArenaMax = 1 << 20, kArenaChunk = 4 << 20;
@@ -293,8 +315,10 @@ int dalloc(fd3_volume* V, float** ptr, size_t count) {
   const bool share = bytes < kArenaMax;
   if (!share || V->arena_left < bytes) {
     void* q = nullptr;
-    const size_t size = share ? kArenaChunk : bytes;
-    CK(cudaMalloc(&q, size));
+    size_t size = share ? kArenaChunk : bytes;
+    cudaError_t e = device_alloc(V, &q, size);
+    if (e == cudaErrorMemoryAllocation && share) e = device_alloc(V, &q, size = bytes);  // no room for a whole chunk
+    CK(e);
     V->allocations.push_back(q);
     CK(cudaMemsetAsync(q, 0, size, V->stream));
     if (!share) {
@@ -1548,8 +1572,9 @@ int alloc_state(fd3_volume* V) {
   TRY(dalloc(V, &cq, (size_t)(V->n + 1) / 2)); V->codes = (unsigned short*)cq;
   TRY(dalloc(V, &cq, 4)); V->count = (unsigned*)cq;
   if (V->n <= kRecMaxCells) {
-    TRY(dalloc(V, &cq, (size_t)V->n * 8));
-    V->rec = (float4*)cq;
+    const int e = dalloc(V, &cq, (size_t)V->n * 8);
+    if (e && e != FD3_ERR_OUT_OF_MEMORY) return e;
+    V->rec = e ? nullptr : (float4*)cq;
   }
   TRY(dalloc(V, &V->sv_u, V->nu)); TRY(dalloc(V, &V->sv_v, V->nv)); TRY(dalloc(V, &V->sv_w, V->nw));
   TRY(dalloc(V, &V->sv_p, V->n)); TRY(dalloc(V, &V->sv_eta, V->ncol)); TRY(dalloc(V, &V->sv_rof, V->ncol));
