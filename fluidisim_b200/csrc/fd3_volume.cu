@@ -182,8 +182,8 @@ struct fd3_volume {
   fd3_report refused{};
   unsigned long long launches = 0;
   std::vector<void*> allocations;
-  char* arena = nullptr;  // what is left of the last shared chunk (dalloc)
-  size_t arena_left = 0;
+  char* block = nullptr;  // what is left of the last reserved block, and its bytes (reserve)
+  size_t reserved = 0;
   // opt-in per-kernel timing: events around every launch, collected at each synchronisation
   bool prof = false;
   std::vector<cudaEvent_t> ev_pool;
@@ -289,7 +289,7 @@ namespace {
 // rebuilt.  The captured loop holds their address.
 bool drop_records(fd3_volume* V) {
   auto at = std::find(V->allocations.begin(), V->allocations.end(), (void*)V->rec);
-  if (!V->rec || at == V->allocations.end()) return false;  // small records share a chunk
+  if (!V->rec || at == V->allocations.end()) return false;
   cudaStreamSynchronize(V->stream);
   if (V->loop_exec) cudaGraphExecDestroy(V->loop_exec);
   V->loop_exec = nullptr;
@@ -307,30 +307,39 @@ cudaError_t device_alloc(fd3_volume* V, void** q, size_t size) {
   }
 }
 
-// Zeroed device memory of the volume's.  Arrays below kArenaMax share chunks of kArenaChunk bytes: a volume has some
-// fifty arrays, a cudaMalloc takes 0.2 ms and more, and a batch configures hundreds of small volumes.
-constexpr size_t kArenaMax = 1 << 20, kArenaChunk = 4 << 20;
+// Zeroed device memory of the volume's: an array of floats, from the reserved block while it lasts.
+size_t padded(size_t count) { return (count * sizeof(float) + 16 + 255) & ~(size_t)255; }
 int dalloc(fd3_volume* V, float** ptr, size_t count) {
-  const size_t bytes = (count * sizeof(float) + 16 + 255) & ~(size_t)255;
-  const bool share = bytes < kArenaMax;
-  if (!share || V->arena_left < bytes) {
+  const size_t bytes = padded(count);
+  if (V->reserved < bytes) {
     void* q = nullptr;
-    size_t size = share ? kArenaChunk : bytes;
-    cudaError_t e = device_alloc(V, &q, size);
-    if (e == cudaErrorMemoryAllocation && share) e = device_alloc(V, &q, size = bytes);  // no room for a whole chunk
-    CK(e);
+    CK(device_alloc(V, &q, bytes));
     V->allocations.push_back(q);
-    CK(cudaMemsetAsync(q, 0, size, V->stream));
-    if (!share) {
-      *ptr = (float*)q;
-      return FD3_OK;
-    }
-    V->arena = (char*)q;
-    V->arena_left = size;
+    CK(cudaMemsetAsync(q, 0, bytes, V->stream));
+    *ptr = (float*)q;
+    return FD3_OK;
   }
-  *ptr = (float*)V->arena;
-  V->arena += bytes;
-  V->arena_left -= bytes;
+  *ptr = (float*)V->block;
+  V->block += bytes;
+  V->reserved -= bytes;
+  return FD3_OK;
+}
+// One block for the arrays that follow, of these many floats each, `times` over.  A volume has some fifty arrays; an
+// allocation each took 0.32 s for 128 patches of 16..96 cells a side with fields and hierarchy (0.26 in shared chunks of 4 MB),
+// 0.20 s so, and each array of little more than a MB held two: 64^3 with both takes 40 MB (48, with 8 of records less), 16^3
+// 0.6 MB (4.2 in a chunk of its own).  Without room for the block each array finds its own.
+int reserve(fd3_volume* V, const std::vector<std::pair<size_t, int>>& arrays) {
+  size_t bytes = 0;
+  for (auto& a : arrays) bytes += a.second * padded(a.first);
+  void* q = nullptr;
+  const cudaError_t e = device_alloc(V, &q, bytes);
+  V->reserved = 0;
+  if (e == cudaErrorMemoryAllocation) return FD3_OK;
+  CK(e);
+  V->allocations.push_back(q);
+  CK(cudaMemsetAsync(q, 0, bytes, V->stream));
+  V->block = (char*)q;
+  V->reserved = bytes;
   return FD3_OK;
 }
 
@@ -1562,6 +1571,16 @@ int check_finite_device(fd3_volume* V, const float* x, long long n, bool* ok) {
 
 // ------------------------------------------------------------------------------------ configure
 int alloc_state(fd3_volume* V) {
+  // one f64 partial per block of the largest reduction launch: linear (one cell per thread),
+  // 2.5-D blocked, or the grid-stride update
+  V->p64_cap = std::max(std::max(blocks_for(V->n), std::max(zblocks(V->nx, V->ny, V->nz), zblocks2(V->nx, V->ny, V->nz, 4))),
+                        UPDATE_BLOCKS);
+  const size_t n = V->n, half = (n + 1) / 2, p64 = (size_t)V->p64_cap * 2 + 64, p32 = (n + CHUNK - 1) / CHUNK + 64,
+               scalars = sizeof(Scalars) / sizeof(float) + 16, slots = (sizeof(GridSlots) + 3) / 4,
+               ntiles = (size_t)((V->nx + TILE_X - 1) / TILE_X) * ((V->ny + TILE_Y - 1) / TILE_Y),
+               qx = (size_t)(V->nx + 1) * V->ny, qy = (size_t)V->nx * (V->ny + 1);
+  TRY(reserve(V, {{V->ncol, 4}, {V->nu, 3}, {V->nv, 3}, {V->nw, 3}, {n, 8}, {half, 1}, {4, 1}, {qx, 1}, {qy, 1}, {p64, 1},
+                  {p32, 1}, {scalars, 1}, {16, 1}, {ntiles, 1}, {slots, 1}, {32, 1}}));
   TRY(dalloc(V, &V->eta, V->ncol)); TRY(dalloc(V, &V->rof, V->ncol));
   TRY(dalloc(V, &V->u, V->nu)); TRY(dalloc(V, &V->v, V->nv)); TRY(dalloc(V, &V->w, V->nw));
   TRY(dalloc(V, &V->us, V->nu)); TRY(dalloc(V, &V->vs, V->nv)); TRY(dalloc(V, &V->ws, V->nw));
@@ -1569,31 +1588,28 @@ int alloc_state(fd3_volume* V) {
   TRY(dalloc(V, &V->dir, V->n)); TRY(dalloc(V, &V->dir2, V->n)); TRY(dalloc(V, &V->tmp, V->n));
   TRY(dalloc(V, &V->prec, V->n));
   float* cq;
-  TRY(dalloc(V, &cq, (size_t)(V->n + 1) / 2)); V->codes = (unsigned short*)cq;
+  TRY(dalloc(V, &cq, half)); V->codes = (unsigned short*)cq;
   TRY(dalloc(V, &cq, 4)); V->count = (unsigned*)cq;
-  if (V->n <= kRecMaxCells) {
-    const int e = dalloc(V, &cq, (size_t)V->n * 8);
-    if (e && e != FD3_ERR_OUT_OF_MEMORY) return e;
-    V->rec = e ? nullptr : (float4*)cq;
-  }
   TRY(dalloc(V, &V->sv_u, V->nu)); TRY(dalloc(V, &V->sv_v, V->nv)); TRY(dalloc(V, &V->sv_w, V->nw));
   TRY(dalloc(V, &V->sv_p, V->n)); TRY(dalloc(V, &V->sv_eta, V->ncol)); TRY(dalloc(V, &V->sv_rof, V->ncol));
-  TRY(dalloc(V, &V->flux_x, (size_t)(V->nx + 1) * V->ny)); TRY(dalloc(V, &V->flux_y, (size_t)V->nx * (V->ny + 1)));
+  TRY(dalloc(V, &V->flux_x, qx)); TRY(dalloc(V, &V->flux_y, qy));
   float* q;
-  // one f64 partial per block of the largest reduction launch: linear (one cell per thread),
-  // 2.5-D blocked, or the grid-stride update
-  V->p64_cap = std::max(std::max(blocks_for(V->n), std::max(zblocks(V->nx, V->ny, V->nz), zblocks2(V->nx, V->ny, V->nz, 4))),
-                        UPDATE_BLOCKS);
-  TRY(dalloc(V, &q, (size_t)V->p64_cap * 2 + 64)); V->p64 = (double*)q;
-  TRY(dalloc(V, &V->p32, (size_t)(V->n + CHUNK - 1) / CHUNK + 64));
-  TRY(dalloc(V, &q, sizeof(Scalars) / sizeof(float) + 16)); V->dS = (Scalars*)q;
+  TRY(dalloc(V, &q, p64)); V->p64 = (double*)q;
+  TRY(dalloc(V, &V->p32, p32));
+  TRY(dalloc(V, &q, scalars)); V->dS = (Scalars*)q;
   TRY(dalloc(V, &q, 16)); V->dflag = (int*)q;
-  TRY(dalloc(V, &q, (size_t)((V->nx + TILE_X - 1) / TILE_X) * ((V->ny + TILE_Y - 1) / TILE_Y))); V->ztop = (int*)q;
-  TRY(dalloc(V, &q, (sizeof(GridSlots) + 3) / 4)); V->slots = (GridSlots*)q;
+  TRY(dalloc(V, &q, ntiles)); V->ztop = (int*)q;
+  TRY(dalloc(V, &q, slots)); V->slots = (GridSlots*)q;
   TRY(cooperative_ctas(V->device, &V->grid_ctas));
   CK(cudaMallocHost((void**)&V->hS, sizeof(Scalars)));
   CK(cudaMallocHost((void**)&V->hflag, 2 * sizeof(int)));
   TRY(dalloc(V, &q, 32)); V->fsc = (double*)q;
+  if (V->n <= kRecMaxCells) {  // by itself, so that it can be given back
+    V->reserved = 0;
+    const int e = dalloc(V, &q, n * 8);
+    if (e && e != FD3_ERR_OUT_OF_MEMORY) return e;
+    V->rec = e ? nullptr : (float4*)q;
+  }
   CK(cudaMallocHost((void**)&V->hfsc, 8 * sizeof(double)));
   memset(V->hS, 0, sizeof(Scalars));
   // eta = z0 everywhere (delta3d.rs:255)
@@ -1643,6 +1659,7 @@ int configure(const fd3_domain* dom, float rho, float g_eff, fd3_volume** out) {
 }
 
 int build_bottom_cut(fd3_volume* V, const float* bottom) {
+  TRY(reserve(V, {{V->n, 1}, {V->nu, 1}, {V->nv, 1}, {V->nw, 1}, {V->ncol, 2}, {(size_t)(V->nx + 1) * (V->ny + 1), 1}}));
   TRY(dalloc(V, &V->frac, V->n)); TRY(dalloc(V, &V->ou, V->nu)); TRY(dalloc(V, &V->ov, V->nv));
   TRY(dalloc(V, &V->ow, V->nw)); TRY(dalloc(V, &V->floor_, V->ncol));
   float *dbottom, *corner;
@@ -1873,8 +1890,8 @@ int fd3_configure_with_solid(const fd3_domain* domain, float rho, float g_eff, c
   TRY(fd3_configure_with_bottom(domain, rho, g_eff, bottom, blen, &V));
   auto fail = [&](int e) { release(V); delete V; return e; };
   float* dsdf;
-  int e = dalloc(V, &dsdf, slen);
-  if (e) return fail(e);
+  int e = reserve(V, {{slen, 1}, {V->n, 1}, {V->nu, 1}, {V->nv, 1}, {V->nw, 1}, {V->ncol, 3}});
+  if (e || (e = dalloc(V, &dsdf, slen))) return fail(e);
   if (cudaMemcpyAsync(dsdf, solid, slen * sizeof(float), cudaMemcpyHostToDevice, V->stream) != cudaSuccess)
     return fail(cuda_fail(cudaGetLastError(), "solid upload", __LINE__));
   SolidGeo S{V->nx, V->ny, V->nz, V->dx, dsdf, 0};
@@ -1997,27 +2014,36 @@ int fd3_set_stream(fd3_volume* v, void* stream) {
 int fd3_enable_multigrid(fd3_volume* V) {
   if (!V) return FD3_ERR_INVALID_ARGUMENT;
   if (V->has_mg) return FD3_OK;
-  TRY(dalloc(V, &V->z, V->n));
-  TRY(dalloc(V, &V->z2, V->n));
   int x = V->nx, y = V->ny, zz = V->nz;
   float h = V->dx;
+  std::vector<Lev> levels;
+  std::vector<std::pair<size_t, int>> arrays{{V->n, 2}};
   while (x % 2 == 0 && y % 2 == 0 && zz % 2 == 0 && x >= 4 && y >= 4 && zz >= 4 &&
-         (V->opt.mg_max_levels == 0 || V->levels.size() < V->opt.mg_max_levels)) {
-    int cx = x / 2, cy = y / 2, cz = zz / 2;
+         (V->opt.mg_max_levels == 0 || levels.size() < V->opt.mg_max_levels)) {
+    x /= 2;
+    y /= 2;
+    zz /= 2;
     h *= 2.f;
     Lev L{};
-    L.nx = cx; L.ny = cy; L.nz = cz; L.n = cx * cy * cz;
+    L.nx = x; L.ny = y; L.nz = zz; L.n = x * y * zz;
     L.inv = 1.f / (h * h);
-    TRY(dalloc(V, &L.ou, (size_t)(cx + 1) * cy * cz));
-    TRY(dalloc(V, &L.ov, (size_t)cx * (cy + 1) * cz));
-    TRY(dalloc(V, &L.ow, (size_t)cx * cy * (cz + 1)));
+    arrays.insert(arrays.end(), {{(size_t)(x + 1) * y * zz, 1}, {(size_t)x * (y + 1) * zz, 1}, {(size_t)x * y * (zz + 1), 1},
+                                 {L.n, 6}, {(size_t)(L.n + 1) / 2, 1}});
+    levels.push_back(L);
+  }
+  TRY(reserve(V, arrays));
+  TRY(dalloc(V, &V->z, V->n));
+  TRY(dalloc(V, &V->z2, V->n));
+  for (Lev& L : levels) {
+    TRY(dalloc(V, &L.ou, (size_t)(L.nx + 1) * L.ny * L.nz));
+    TRY(dalloc(V, &L.ov, (size_t)L.nx * (L.ny + 1) * L.nz));
+    TRY(dalloc(V, &L.ow, (size_t)L.nx * L.ny * (L.nz + 1)));
     TRY(dalloc(V, &L.kind, L.n)); TRY(dalloc(V, &L.diag, L.n));
     TRY(dalloc(V, &L.x, L.n)); TRY(dalloc(V, &L.x2, L.n)); TRY(dalloc(V, &L.r, L.n)); TRY(dalloc(V, &L.t, L.n));
     float* cq;
     TRY(dalloc(V, &cq, (size_t)(L.n + 1) / 2)); L.code = (unsigned short*)cq;
-    V->levels.push_back(L);
-    x = cx; y = cy; zz = cz;
   }
+  V->levels = levels;
   V->tail_first = (int)V->levels.size();
   while (V->tail_first > 0 && V->levels[V->tail_first - 1].n <= TAIL_MAX_CELLS) --V->tail_first;
   V->tail_reg = (int)V->levels.size() - V->tail_first <= TAIL_REG_LEVELS;

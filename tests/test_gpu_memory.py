@@ -1,5 +1,6 @@
 """A volume whose row records find no memory is configured without them and gives the same bits: the GPU is filled so that
-the records do not fit, at the configuration, or when the multigrid's arrays need their place."""
+the records do not fit, at the configuration, or when the multigrid's arrays need their place.  And small volumes hold
+what they use: a batch configures hundreds of them."""
 import numpy as np
 import pytest
 
@@ -60,3 +61,19 @@ def test_a_volume_without_room_for_its_records(when):
         fill = None
         torch.cuda.empty_cache()
     assert got[0] == want[0] and np.array_equal(got[1], want[1])
+
+
+def test_small_volumes_hold_what_they_use():
+    """64 volumes of 16^3 cells with cut cells and hierarchy: 128 B a cell of fields (32 floats), 32 of records and 23 of
+    coarse levels, 0.75 MB; twice that is the bound (a chunk of 4 MB each was 4.2)."""
+    import torch
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    volumes = [Volume3.configure_with_bottom(16, 16, 16, 0.1, 1025.0, 9.81, np.full(256, 0.1, np.float32)) for _ in range(64)]
+    for v in volumes:
+        v.enable_multigrid()
+    torch.cuda.synchronize()
+    each = (before - torch.cuda.mem_get_info()[0]) / 64
+    for v in volumes:
+        v.close()
+    assert each < 1.5e6
