@@ -20,9 +20,10 @@ constexpr int GRID_THREADS = 512;   // one CTA per SM: the meetings cost less wi
 constexpr int GRID_MAX_CTAS = 160;  // slots
 constexpr int GRID_MAX_CELLS = 12;  // cells of a thread (k_cg_loop's largest instance)
 constexpr size_t cg_smem(int cells) { return (size_t)cells * 7 * GRID_THREADS * sizeof(float); }
-// Polls before a CTA gives up (about a second): a meeting that never completes ends the kernel with
-// status 100 instead of hanging the GPU.
-constexpr unsigned GRID_POLLS = 1u << 20;
+// Polls before a CTA gives up: a meeting that never completes ends the kernel with status 100 (reported with its reason)
+// instead of hanging the GPU.  They are polls, not time, so that a grid suspended meanwhile does not give up; 2^20 take
+// 0.23 s.
+constexpr unsigned GRID_POLLS = 1u << 22;
 
 // The CTAs of a cooperative grid as one team, meeting at a counter that is 0 at the launch and never
 // reset.  A meeting is one release-add and an acquire-poll by one thread per CTA (1.3 us on 148 CTAs); a sum
@@ -58,8 +59,8 @@ struct GridTeam {
     unsigned seen, polls = 0;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&slots->arrived) : "memory");
-    } while (seen < target && ++polls < GRID_POLLS);
-    return seen >= target;
+    } while ((int)(seen - target) < 0 && ++polls < GRID_POLLS);
+    return (int)(seen - target) >= 0;
   }
   // A meeting without a sum.
   __device__ __forceinline__ bool meet() {
@@ -155,10 +156,11 @@ struct GridTeam {
   }
 };
 
-// The meeting counter to 0, before a launch that meets.
-__global__ void k_grid_reset(GridSlots* slots) {
+// The meeting counter to 0, before a launch that meets; below 0 by `absent` CTAs that will not come (for tests: every
+// meeting then runs out).
+__global__ void k_grid_reset(GridSlots* slots, unsigned absent) {
   KSTART();
-  slots->arrived = 0u;
+  slots->arrived = 0u - absent;
 }
 
 // A cell's row kept on chip, as Geo::rec keeps it: per face the aperture onto a fluid neighbour, or the ghost's

@@ -169,6 +169,7 @@ struct fd3_volume {
   unsigned* count = nullptr;
   GridSlots* slots = nullptr;  // the meetings of k_cg_loop and k_mg_loop
   int grid_ctas = 0;          // CTAs of the cooperative launches (one per SM; 0: not to be had)
+  unsigned absent = 0;        // CTAs that its meetings wait for in vain (for tests)
   int workers = 1;            // volumes that fd3_project_batch projects at once, this one among them
   Scalars* dS = nullptr;
   Scalars* hS = nullptr;  // pinned
@@ -985,7 +986,7 @@ void launch_cg_loop(fd3_volume* V, int ctas) {
   V->launches++;
 }
 void run_cg_loop(fd3_volume* V) {
-  LAUNCH_G(V, k_grid_reset, 1, 1, V->slots);
+  LAUNCH_G(V, k_grid_reset, 1, 1, V->slots, V->absent);
   const int ctas = std::min(V->grid_ctas, (V->n + GRID_THREADS - 1) / GRID_THREADS);
   const int cells = (V->n + ctas * GRID_THREADS - 1) / (ctas * GRID_THREADS);
   // Beside other volumes: a half of the CTAs, or a quarter, each standing in for the others.  Sixteen volumes by sixteen
@@ -1039,7 +1040,7 @@ int enqueue_loop(fd3_volume* V) {
     return FD3_OK;
   }
   if (V->mg_loop()) {
-    LAUNCH_G(V, k_grid_reset, 1, 1, V->slots);
+    LAUNCH_G(V, k_grid_reset, 1, 1, V->slots, V->absent);
     if (V->half()) launch_mg_loop<__half>(V);
     else launch_mg_loop<float>(V);
     return FD3_OK;
@@ -1054,6 +1055,13 @@ void count_loop(fd3_volume* V, unsigned ran) {
   if (!V->one_launch()) V->launches += (unsigned long long)((ran + 1) / 2) * V->body_nodes;
 }
 
+// What the device's loop or set-up reported, after a pull.
+int loop_status(fd3_volume* V) {
+  if (V->hS->status == FD3_ERR_CUDA)
+    g_last_cuda_error = "the solver's loop gave up: a block did not arrive at a grid-wide meeting";
+  return V->hS->status;
+}
+
 // Run the inner loop until S->active drops.
 int run_inner(fd3_volume* V, uint32_t it_before) {
   const bool graphs = V->cg_loop() || (V->opt.use_graphs && !V->prof);
@@ -1065,7 +1073,10 @@ int run_inner(fd3_volume* V, uint32_t it_before) {
   }
   // The device clears S->active within max_iters iterations (FIN_RN); the host bound is a guard.
   for (unsigned guard = 0;; ++guard) {
-    if (guard > V->hS->max_iters + 2u) return FD3_ERR_CUDA;
+    if (guard > V->hS->max_iters + 2u) {
+      g_last_cuda_error = "the solver's loop did not end within its iterations";
+      return FD3_ERR_CUDA;
+    }
     iteration(V, guard & 1);
     TRY(pull(V));
     if (!V->hS->active) break;
@@ -1231,12 +1242,12 @@ int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_r
     LAUNCH_G(V, k_loop_start_dev, 1, 1, V->dS, max_iters);
     TRY(enqueue_loop(V));
     TRY(outer_checks(V, k1, &ck));
-    if (V->hS->status) return V->hS->status;
+    TRY(loop_status(V));
     count_loop(V, std::max(V->hS->it, 1u));
     have_checks = true;
   } else {
     TRY(pull(V));
-    if (V->hS->status) return V->hS->status;
+    TRY(loop_status(V));
   }
   const double b2 = V->hS->b2;
   double rr = V->hS->rr;
@@ -1272,13 +1283,13 @@ int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_r
       if (speculate) {  // the loop and the checks behind it, one synchronisation (the checks keep it and rr)
         TRY(enqueue_loop(V));
         TRY(outer_checks(V, k1, &ck));
-        if (V->hS->status) return V->hS->status;
+        TRY(loop_status(V));
         count_loop(V, V->hS->it > it ? V->hS->it - it : 1);
         it = V->hS->it;
         rr = V->hS->rr;
       } else {
         TRY(run_inner(V, it));
-        if (V->hS->status) return V->hS->status;
+        TRY(loop_status(V));
         it = V->hS->it;
         rr = V->hS->rr;
         TRY(outer_checks(V, k1, &ck));
@@ -2443,6 +2454,8 @@ int fd3_project_batch(fd3_volume* const* vols, size_t count, const float* scales
   size_t T = threads > 0 ? (size_t)threads : 16;
   T = std::max<size_t>(1, std::min(T, count));
   std::atomic<size_t> next{0};
+  std::mutex text_lock;
+  std::string text;  // of a CUDA failure, for the caller's thread
   auto worker = [&]() {
     for (;;) {
       const size_t q = next.fetch_add(1);
@@ -2452,12 +2465,23 @@ int fd3_project_batch(fd3_volume* const* vols, size_t count, const float* scales
       vols[i]->workers = (int)T;
       statuses[i] = fd3_project_mobile(vols[i], scales[i], k1s[i], max_iters, &reports[i]);
       vols[i]->workers = 1;
+      if (statuses[i] >= FD3_ERR_CUDA) {
+        std::lock_guard<std::mutex> lock(text_lock);
+        text = g_last_cuda_error;
+      }
     }
   };
   std::vector<std::thread> pool;
   for (size_t t = 1; t < T; ++t) pool.emplace_back(worker);
   worker();
   for (auto& th : pool) th.join();
+  if (!text.empty()) g_last_cuda_error = text;
+  return FD3_OK;
+}
+
+int fd3_absent_blocks_for_tests(fd3_volume* V, uint32_t blocks) {
+  if (!V) return FD3_ERR_INVALID_ARGUMENT;
+  V->absent = blocks;
   return FD3_OK;
 }
 

@@ -332,6 +332,10 @@ int fd3_assemble_pressure_problem_noalloc(fd3_volume* v, const float* d_divergen
 /* v_cycle3 (delta3d_multigrid.rs:393) on `x`, set up as tests_delta3d.rs:1840-1873 does
  * (rhs = 0, rhs_mobile3(1), prepare_multigrid3, res = x).  Writes z = M^-1 x. */
 int fd3_vcycle_for_tests(fd3_volume* v, const float* x, float* z, size_t len);
+/* A failure of the one-launch loops on purpose (no reference counterpart): their grid-wide meetings wait for
+ * `blocks` blocks that do not exist, so each call that runs such a loop gives up after about a second and
+ * reports FD3_ERR_CUDA, with the reason in fd3_last_cuda_error.  0 ends it. */
+int fd3_absent_blocks_for_tests(fd3_volume* v, uint32_t blocks);
 /* Coarse level l after prepare_multigrid3: kind, diag, open_u/v/w (Level3, delta3d_multigrid.rs:37). */
 int fd3_level_geometry(const fd3_volume* v, uint32_t l, float* kind, float* diag, float* open_u,
                        float* open_v, float* open_w);
