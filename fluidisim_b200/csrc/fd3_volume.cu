@@ -253,7 +253,9 @@ struct fd3_volume {
   bool mg_on() const { return has_mg && !linear; }  // the linear path has no multigrid
   // Without the multigrid, the inner loop in one cooperative launch (k_cg_loop), up to the cells its
   // threads hold in registers; larger volumes, the ordered mode and use_graphs = 0 keep the four
-  // kernels per iteration.
+  // kernels per iteration.  It wins as far as it goes (us an iteration, four kernels / one launch): 504 cells 19.5 / 6.0,
+  // 40,095 18.7 / 5.5, 215,025 25.7 / 7.2, 303,525 (eight-cell instance) 27.0 / 14.9, 559,845 37.1 / 16.6, 689,325 (twelve)
+  // 42.2 / 29.8, 899,910 51.4 / 31.9.
   bool cg_loop() const {
     return !ord() && !mg_on() && opt.use_graphs && (long long)n <= (long long)grid_ctas * GRID_THREADS * GRID_MAX_CELLS;
   }
