@@ -1082,29 +1082,20 @@ __global__ void __launch_bounds__(TPB) k_level_pre(Lev L, Air air, const Scalars
 }
 
 // t = r - L x on every cell of a coarse level (0 on inactive rows), the restriction's operand.
-template <class T, bool SPEC>
+template <class T>
 __global__ void __launch_bounds__(TPB) k_level_resid(Lev L, Air air, const Scalars* S, int gate) {
   KSTART();
-  if (!SPEC && gate && !S->active) return;
+  if (gate && !S->active) return;
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= L.n) return;
   const LoadT<T> X{as<T>(L.x)};
-  auto Xc = [&](int n, int, int, int) { return X(n); };
   int i, j, k;
   level_ijk(L, c, i, j, k);
   if (in_air(air, i, j, k)) return;
   const unsigned code = L.code[c];
   const float rc = Store<T>::ld(as<T>(L.r), c);
-  const float pc = X(c);
   float lx = 0.f;
-  if (SPEC) {
-    const Ap6 ap = level_ap6(L, i, j, k);
-    const Nb6 b = level_nb(L, i, j, k, c, Xc);
-    if (gate && !S->active) return;
-    if (code & RC_WET) lx = level_row_sel(L, code, pc, b, ap);
-  } else if (code & RC_WET) {
-    lx = level_row_code(L, code, i, j, k, c, X);
-  }
+  if (code & RC_WET) lx = level_row_code(L, code, i, j, k, c, X);
   Store<T>::st(as<T>(L.t), c, rc - lx);
 }
 
@@ -1133,7 +1124,7 @@ __global__ void __launch_bounds__(TPB) k_level_sum8(Lev F, Lev C, Air air, const
 // the eight threads of a coarse cell (consecutive lanes, child e = lane % 8 in the reference's
 // CHILDREN order) each evaluate one child's t = r - L x, rounded through the storage type as the
 // stored t would be, and the first of them sums the eight in order (restrict3).
-template <class T, bool SPEC>
+template <class T>
 __global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, Air air, const Scalars* S, int gate) {
   const int q8 = blockIdx.x * blockDim.x + threadIdx.x;
   const int q = q8 >> 3, e = q8 & 7;
@@ -1149,10 +1140,9 @@ __global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, Air air, 
     k = 2 * ck + (e >> 2);
     c = (k * F.ny + j) * F.nx + i;
     code = F.code[c];
-    if (SPEC && !(code & RC_UNIT)) ap = level_ap6(F, i, j, k);
+    if (!(code & RC_UNIT)) ap = level_ap6(F, i, j, k);
   }
   KSTART();
-  if (!SPEC && gate && !S->active) return;
   if (!__any_sync(0xffffffffu, own)) return;
   float tv = 0.f;
   float rc = 0.f, pc = 0.f;
@@ -1161,14 +1151,10 @@ __global__ void __launch_bounds__(TPB) k_level_restrict8(Lev F, Lev C, Air air, 
     rc = Store<T>::ld(as<T>(F.r), c);
     pc = X(c);
   }
-  if (SPEC) {
-    Nb6 b{};
-    if (own) b = level_nb(F, i, j, k, c, [&](int n, int, int, int) { return X(n); });
-    if (gate && !S->active) return;
-    if (own) tv = Store<T>::rt(rc - ((code & RC_WET) ? level_row_sel(F, code, pc, b, ap) : 0.f));
-  } else if (own) {
-    tv = Store<T>::rt(rc - ((code & RC_WET) ? level_row_code(F, code, i, j, k, c, X) : 0.f));
-  }
+  Nb6 b{};
+  if (own) b = level_nb(F, i, j, k, c, [&](int n, int, int, int) { return X(n); });
+  if (gate && !S->active) return;
+  if (own) tv = Store<T>::rt(rc - ((code & RC_WET) ? level_row_sel(F, code, pc, b, ap) : 0.f));
   const int lane0 = threadIdx.x & 24;  // first lane of the eight
   float sum = 0.f;
 #pragma unroll
@@ -1323,7 +1309,9 @@ __global__ void __launch_bounds__(TPB) k_level_post21(Lev L, Lev C, Air air, con
   level_post21_at<T, true>(L, C, air, blockIdx.x * blockDim.x + threadIdx.x, gate ? S : nullptr);
 }
 
-// The same passes at one cell (or one lane) for the one-launch loop, which has no gate: every load before the row.
+// The same passes at one cell (or one lane) for the one-launch loop, which has no gate: every load before the row, none
+// for a cell in the air.  One body for both (the rows' loads ahead of the wait, as level_post21_at) spilled 100 bytes more
+// in the loop, where a spilled register is read from L2 after each meeting: a 32 x 16 x 24 step 690 -> 710 us.
 template <class T>
 __device__ __forceinline__ void level_pre_at(const Lev& L, const Air& air, int c) {
   int i, j, k;

@@ -90,7 +90,7 @@ struct Geo {
 };
 constexpr int TILE_X = 32, TILE_Y = 8;
 
-// The layers to process of the columns [x0, x0 + 64) x [y0, y0 + 8) (two tiles), and of one column.
+// The layers to process of the columns [x0, x0 + 64) x [y0, y0 + 8) (two tiles).
 __device__ __forceinline__ int tops64(const Geo& g, int x0, int y0) {
   if (!g.ztop) return g.nz;
   const int ntx = (g.nx + TILE_X - 1) / TILE_X, a = x0 / TILE_X, row = (y0 / TILE_Y) * ntx;

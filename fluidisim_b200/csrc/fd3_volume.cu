@@ -529,10 +529,10 @@ void coarse_cycle_t(fd3_volume* V, int gate) {
       const long long n8 = 8LL * Ls[l + 1].n;  // one thread per child of each next-level cell
       if (L.n <= SPEC_MAX_CELLS) {
         launch_grid(V, "k_level_pre", blocks_for(L.n), TPB, k_level_pre<T, true>, L, air(l), S, gate);
-        launch_grid(V, "k_level_restrict8", blocks_for(n8), TPB, k_level_restrict8<T, true>, L, Ls[l + 1], air(l + 1), S, gate);
+        launch_grid(V, "k_level_restrict8", blocks_for(n8), TPB, k_level_restrict8<T>, L, Ls[l + 1], air(l + 1), S, gate);
       } else {
         launch_grid(V, "k_level_pre", blocks_for(L.n), TPB, k_level_pre<T, false>, L, air(l), S, gate);
-        launch_grid(V, "k_level_resid", blocks_for(L.n), TPB, k_level_resid<T, false>, L, air(l), S, gate);
+        launch_grid(V, "k_level_resid", blocks_for(L.n), TPB, k_level_resid<T>, L, air(l), S, gate);
         LAUNCH(V, k_level_sum8<T>, Ls[l + 1].n, L, Ls[l + 1], air(l + 1), S, gate);
       }
     }
