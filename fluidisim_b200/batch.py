@@ -19,6 +19,7 @@ from .delta3d import REDUCE_F64, Delta3dError, Report, Volume3, _Report, library
 SIZE_CLASSES = [("small", 0, 48 ** 3), ("medium", 48 ** 3, 80 ** 3), ("large", 80 ** 3, 1 << 62)]
 # (kernels, mg_max_levels): fine-level kernel family and V-cycle depth (0 = every level)
 CANDIDATES = [(0, 0), (1, 0), (2, 0), (0, 3), (1, 3)]
+TOGETHER = 8  # patches projected at once while a candidate is timed
 
 
 def _bind(L):
@@ -180,21 +181,23 @@ class Tuned:
 
 def autotune(scenes_by_class: dict, repeats: int = 3, timer=None) -> dict:
     """Per size class, time every candidate (kernel family, V-cycle depth) on the class's largest
-    patch (best of `repeats` projections) and keep the fastest.  `timer(scene, kernels, levels)`
-    replaces the measurement (tests); by default it configures the patch and times
-    fd3_project_mobile with device synchronisation around each call."""
+    patch and keep the fastest: TOGETHER copies of it projected at once, as `project_batch` runs them (a
+    candidate that is faster alone may take more of the GPU), best of `repeats` sets.
+    `timer(scene, kernels, levels)` replaces the measurement (tests).  Tuned.ms is per patch."""
     def measure(scene, kernels, levels):
-        v = configure(scene, kernels, levels)
+        vols = [configure(scene, kernels, levels) for _ in range(TOGETHER)]
         scale, k1 = scenes.projection_scalars(scene)
         best = float("inf")
         for _ in range(repeats + 1):
-            v.set_velocity(scene["u"], scene["v"], scene["w"])
-            v.reset_pressure()
+            for v in vols:
+                v.set_velocity(scene["u"], scene["v"], scene["w"])
+                v.reset_pressure()
             t0 = time.perf_counter()
-            v.project_mobile3(scale, k1, 4000)
+            project_batch(vols, [scale] * TOGETHER, [k1] * TOGETHER, threads=TOGETHER)
             best = min(best, time.perf_counter() - t0)
-        v.close()
-        return best * 1e3
+        for v in vols:
+            v.close()
+        return best * 1e3 / TOGETHER
     timer = timer or measure
     out = {}
     for name, group in scenes_by_class.items():
