@@ -53,26 +53,29 @@ BYTES_PER_CELL = {
     "kz_fine_restrict": 2 + 4 + 4 + 0.5,       # code, r, z, coarse r (1/8 cell)
     "kz_fine_post1": 2 + 4 + 4 + 4 + 0.5 + 4,  # code, prec, r, z in, coarse x, z out
     "kz_fine_post2_rz": 2 + 4 + 4 + 4 + 4,     # code, prec, r, z in, z out
-    # the same passes with two cells per thread (f64 mode, the default when nx is even)
+    # the same passes with two cells per thread (f64 mode, the default when nx is even); the update and the residual
+    # run on their tiles beside the TMA-staged passes too
     "kx_dir_apply_dot": 2 + 4 + 4 + 4 + 4,
     "kx_fine_pre": 2 + 4 + 4 + 4,
     "kx_fine_restrict": 2 + 4 + 4 + 0.5,
     "kx_fine_post1": 2 + 4 + 4 + 4 + 0.5 + 4,
     "kx_fine_post2_rz": 2 + 4 + 4 + 4 + 4,
-    # the same passes with four cells per thread (f64 mode, the default when nx % 4 == 0, f32 storage)
+    "kx_update_rn": 4 * 6,
+    "kx_residual": 2 + 4 * 3,                  # code, p, rhs, res out
+    # the same passes with four cells per thread (f64 mode, from 2^23 cells when nx % 4 == 0 and nx % 8 != 0, f32 storage)
     "kq_dir_apply_dot": 2 + 4 + 4 + 4 + 4,
     "kq_fine_pre": 2 + 4 + 4 + 4,
     "kq_fine_restrict": 2 + 4 + 4 + 0.5,
     "kq_fine_post1": 2 + 4 + 4 + 4 + 0.5 + 4,
     "kq_fine_post2_rz": 2 + 4 + 4 + 4 + 4,
     "kq_residual": 2 + 4 * 3,
-    # the same passes on TMA-staged layers (f64 mode, the default from 2^23 cells with nx % 8 == 0)
+    # the same passes on TMA-staged layers (f64 mode, the default from 1,500,000 cells with nx % 8 == 0, f32 storage)
     "kt_dir_apply_dot": 2 + 4 + 4 + 4 + 4,
     "kt_fine_pre": 2 + 4 + 4 + 4,
     "kt_fine_restrict": 2 + 4 + 4 + 0.5,
     "kt_fine_post1": 2 + 4 + 4 + 4 + 0.5 + 4,
     "kt_fine_post2_rz": 2 + 4 + 4 + 4 + 4,
-    "kt_residual": 2 + 4 * 3,                  # code, p, rhs, res out
+    "kt_residual": 2 + 4 * 3,
     # one-cell-per-thread kernels (ordered mode, and f64 mode with kernels = 1)
     "k_dir_apply_dot": 2 + 4 + 4 + 4 + 4,
     "k_update_rn": 4 * 6,
@@ -89,6 +92,26 @@ BYTES_PER_CELL = {
     "k_rhs_march": 4 * 5 + GEOM + 2,           # the three faces in, rhs and prec out, geometry, row code
     "k_divergence": 4 * 3 + 4 + GEOM,          # three face families in, rhs out
 }
+
+
+def marched_cells(s):
+    """The cells that the two-cell and the TMA-staged passes visit: per tile of 64 x 8 columns the layers up to its
+    highest wet cell, rounded up to an even number; the air above is left alone."""
+    import numpy as np
+    eta = np.asarray(s["eta"], np.float32).reshape(s["ny"], s["nx"])
+    height = (np.arange(s["nz"], dtype=np.float32) + np.float32(0.5)) * np.float32(s["dx"])
+    tops = np.searchsorted(height, eta, side="left")  # layers whose centre lies below the surface
+    cells = 0
+    for j in range(0, s["ny"], 8):
+        for i in range(0, s["nx"], 64):
+            tile = tops[j:j + 8, i:i + 64]
+            cells += tile.size * min(int(tile.max() + 1) // 2 * 2, s["nz"])
+    return cells
+
+
+def alg_bytes_per_launch(name, s):
+    """The bytes a launch of a fine-level kernel has to move: its bytes per cell times the cells it visits."""
+    return BYTES_PER_CELL[name] * (marched_cells(s) if name[:3] in ("kx_", "kt_") else s["nx"] * s["ny"] * s["nz"])
 
 
 def merge_templates(entries):
@@ -628,7 +651,8 @@ def wave_measure(args, stream, flush):
         known = [(n, c, m) for n, c, m in prof if n in BYTES_PER_CELL and BYTES_PER_CELL[n] >= 8]
         name, count, msum = max(known, key=lambda e: e[2])
         avg = msum / count
-        ach = BYTES_PER_CELL[name] * cells / (avg * 1e-3) / 1e9
+        alg = alg_bytes_per_launch(name, s)
+        ach = alg / (avg * 1e-3) / 1e9
         traffic = None
         tf = os.path.join(ROOT, "profiles", "traffic_wave_256.txt")
         if os.path.exists(tf):
@@ -637,7 +661,7 @@ def wave_measure(args, stream, flush):
                 if len(parts) == 2 and not line.startswith("#") and parts[0] == name:
                     traffic = float(parts[1])
         return {"bound": "hbm", "kernel": name, "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                "peak_source": peak_kind, "avg_launch_ms": avg, "alg_bytes_per_launch": BYTES_PER_CELL[name] * cells,
+                "peak_source": peak_kind, "avg_launch_ms": avg, "alg_bytes_per_launch": alg,
                 "traffic": traffic, "timing": "instrumented replay of 2 projections without the loop graph"}
 
     pressures = {}
@@ -864,7 +888,7 @@ def run_b200(args):
     top = max(known, key=lambda e: e[2])
     name, count, ms = top
     cells = s["nx"] * s["ny"] * s["nz"]
-    alg_bytes = BYTES_PER_CELL[name] * cells
+    alg_bytes = alg_bytes_per_launch(name, s)
     avg_ms = ms / count
     peak, peak_kind = peaks()
     achieved = alg_bytes / (avg_ms * 1e-3) / 1e9
@@ -884,7 +908,8 @@ def run_b200(args):
         mixed_line, p16 = mixed_measure(args, s, stream, flush, plain_p.astype(np.float64), ms_per_step)
     if world == 1 and args.learned:
         learned_line = learned_fcg_measure(args, s, plain_p, stream)
-    parts_line = parts_measure(args, s, stream) if (world == 1 and args.parts) else None
+    # (the breaking wave leaves the domain in a step)
+    parts_line = parts_measure(args, s, stream) if (world == 1 and args.parts and args.workload == "basin") else None
     wave_line = wave_measure(args, stream, flush) if (world == 1 and args.wave and args.workload == "basin") else None
 
     if rank == 0:
@@ -1000,7 +1025,7 @@ def run_patches(args):
     ms_total, ci = batch.reduce_totals(sum(ms), my_ci, world, device="cuda")
     its = [r.iterations for r in reps]
     pb.close()
-    # the per-patch path on the same volumes: host workers issuing each patch's loop graph
+    # the per-patch path on the same volumes: host workers issuing each patch's loop
     streams_line = None
     if world == 1 and args.streams:
         tuned = batch.autotune(batch.by_class(mine))
@@ -1016,7 +1041,7 @@ def run_patches(args):
             m_, _ = timed_set(sstep, 1)
             ms_s.append(m_)
         streams_line = {"value": len(ps) / (np.mean(ms_s) * 1e-3), "unit": "patches/s", "ms_per_step": float(np.mean(ms_s)),
-                        "note": "fd3_project_batch: every patch its own stream and device-side loop graph, issued by "
+                        "note": "fd3_project_batch: every patch its own stream and device-side loop, issued by "
                                 "host workers; inputs set through set_velocity_device per patch",
                         "autotuned": {k: {"kernels": v.kernels, "mg_max_levels": v.levels, "ms": round(v.ms, 3)}
                                       for k, v in tuned.items()}}
@@ -1234,10 +1259,11 @@ def main():
                     help="training samples of the learned preconditioner (20,000 at 64^3, as config 4 asks)")
     ap.add_argument("--kernels", type=int, default=0,
                     help="fine-level kernel family (fd3_options.kernels): 0 the default (TMA-staged layers from "
-                         "2^23 cells, else two cells per thread), 3 two cells per thread, 4 four cells per thread, "
+                         "1,500,000 cells with nx %% 8 == 0, else two cells per thread), 3 two cells per thread, 4 four cells per thread, "
                          "5 TMA-staged layers, 2 one cell per thread in the same blocking")
     ap.add_argument("--graphs", type=int, default=1,
-                    help="1: the inner loop as a CUDA graph with a WHILE node; 0: host-driven (for ncu launch lists)")
+                    help="1: the inner loop without the host (one launch, or a CUDA graph with a WHILE node); 0: host-driven "
+                         "(for ncu launch lists)")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
     if args.size is None:
