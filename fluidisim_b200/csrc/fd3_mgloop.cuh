@@ -9,8 +9,8 @@
 //
 // Every cell value is that of the separate kernels; the f64 sums have a part per chunk, added in the order of the chunks,
 // so the result is the same on any number of CTAs, and a volume beside others takes fewer (fd3_volume::mg_ctas).  Whole
-// projections, separate kernels and one launch alone on a B200: 64^3 1.04 and 0.98 ms, 48^3 1.00 and 0.91, 32^3 0.77 and
-// 0.73, 32 x 16 x 24 0.61 and 0.59.
+// projections alone, separate kernels and one launch (B200): 64^3 1.04 and 0.94 ms, 48^3 1.00 and 0.89, 32^3 0.77 and 0.70,
+// 32 x 16 x 24 0.61 and 0.58.
 #pragma once
 
 #include "fd3_persist.cuh"
@@ -21,8 +21,7 @@ namespace fd3 {
 constexpr int MG_TEAMS = 3;
 constexpr int MG_THREADS = MG_TEAMS * Z2T;  // one CTA per SM, 80 registers
 constexpr int MG_LEVELS = 8;                // levels above the tail
-constexpr int MG_MIN_CTAS = 16;             // of a volume alone: 32 x 16 x 24 takes 0.59 ms on 16, 0.60 on 8, 0.77 on 4
-constexpr int MG_LEAST_SHARE = 8;           // beside many others (sixteen 64^3 at once, ms: 3.7 on 8, 5.9 on 4)
+constexpr int MG_LEAST_SHARE = 8;           // CTAs beside many other volumes (sixteen 64^3 at once, ms: 3.7 on 8, 5.9 on 4)
 
 struct MgLoop {
   Geo g;
@@ -54,26 +53,27 @@ struct TeamSync {
 };
 
 // Layers of a chunk: the even number that makes the longest team's march shortest, a chunk of K layers counting K + 2
-// (its halo layers) and GRID_PARTS teams taking the chunks that hold water in turn; at most GRID_PARTS chunks.  It does
-// not depend on the grid, nor do the sums, whose parts are the chunks.
-__device__ __forceinline__ int mg_pick_chunk(const Geo& g, int* cost) {
-  constexpr int teams = GRID_PARTS;
+// (its halo layers) and GRID_PARTS teams taking the chunks that hold water in turn; at most GRID_PARTS chunks up to the
+// highest water (top).  It does not depend on the grid, nor do the sums, whose parts are the chunks.
+__device__ __forceinline__ int mg_pick_chunk(const Geo& g, int* cost, int& top) {
   const int ntx = (g.nx + Z2X - 1) / Z2X, nty = (g.ny + Z2Y - 1) / Z2Y;
-  if (threadIdx.x < 8) cost[threadIdx.x] = 0;
+  if (threadIdx.x < 9) cost[threadIdx.x] = 0;
   __syncthreads();
   for (int q = threadIdx.x; q < 8 * ntx * nty; q += MG_THREADS) {
     const int k = 2 + 2 * (q & 7), t = q >> 3;
-    const int top = ztile2_at(g, t % ntx, t / ntx, 0, g.nz, 0, 0).k1;
-    if (top > 0) atomicAdd(cost + (q & 7), (top + k - 1) / k);
+    const int high = ztile2_at(g, t % ntx, t / ntx, 0, g.nz, 0, 0).k1;
+    if (high > 0) atomicAdd(cost + (q & 7), (high + k - 1) / k);
+    if (high > 0 && (q & 7) == 0) atomicMax(cost + 8, high);
   }
   __syncthreads();
   int best = 2, least = 0x7fffffff;
   for (int q = 0; q < 8; ++q) {
-    const int k = 2 + 2 * q, c = (cost[q] + teams - 1) / teams * (k + 2);
+    const int k = 2 + 2 * q, c = (cost[q] + GRID_PARTS - 1) / GRID_PARTS * (k + 2);
     if (c < least) { least = c; best = k; }
   }
+  top = cost[8];
   const int high = GRID_PARTS / (ntx * nty);  // chunks of a tile, at least one (mg_fits)
-  return max(best, 2 * (((g.nz + high - 1) / high + 1) / 2));
+  return max(best, 2 * (((top + high - 1) / high + 1) / 2));
 }
 
 inline bool mg_fits(int nx, int ny) { return ((nx + Z2X - 1) / Z2X) * ((ny + Z2Y - 1) / Z2Y) <= GRID_PARTS; }
@@ -89,9 +89,10 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
   GridTeam<MG_THREADS> grid(a.slots, sh.grid);
   const int tid = threadIdx.x, team = tid / Z2T, tx = tid & 31, ty = (tid >> 5) & 7, teams = gridDim.x * MG_TEAMS;
   const int ntx = (g.nx + Z2X - 1) / Z2X, nty = (g.ny + Z2Y - 1) / Z2Y, tiles = ntx * nty;
-  const int K = mg_pick_chunk(g, reinterpret_cast<int*>(sh.grid.warp));
+  int top;
+  const int K = mg_pick_chunk(g, reinterpret_cast<int*>(sh.grid.warp), top);
   __syncthreads();
-  const int chunks = tiles * ((g.nz + K - 1) / K);
+  const int chunks = tiles * max((top + K - 1) / K, 1);
   const bool first_cta = blockIdx.x == 0;
   if (first_cta && a.ntail > 0) tail_rows(a.tail, a.ntail, sh.tail);
   T* z = static_cast<T*>(a.z);

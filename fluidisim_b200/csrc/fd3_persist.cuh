@@ -91,19 +91,26 @@ struct GridTeam {
     __syncthreads();
     double2* half = slots->part[meeting & 1u];
     bool late = false;
-    const int slot = (int)(blockIdx.x + threadIdx.x * gridDim.x);
-    if ((int)threadIdx.x < V && (V == 1 || slot < slots_used)) {
+    auto store = [&](int v, int slot) {
       double2 p = make_double2(0.0, 0.0);
 #pragma unroll
       for (int q = 0; q < THREADS / 32; ++q) {
-        p.x += sh.warp[threadIdx.x][q][0];
-        if (TWO) p.y += sh.warp[threadIdx.x][q][1];
+        p.x += sh.warp[v][q][0];
+        if (TWO) p.y += sh.warp[v][q][1];
       }
       __stcg(half + slot, p);
+    };
+    if constexpr (V > 1) {
+      const int slot = (int)(blockIdx.x + threadIdx.x * gridDim.x);
+      if ((int)threadIdx.x < V && slot < slots_used) store(threadIdx.x, slot);
+      if (wid == 0) __syncwarp();  // the other threads' slots before the first arrives
     }
-    if (V > 1 && wid == 0) __syncwarp();  // the other threads' slots before the first arrives
-    if (threadIdx.x == 0) late = !arrive_and_wait();
-    else ++meeting;
+    if (threadIdx.x == 0) {
+      if constexpr (V == 1) store(0, blockIdx.x);
+      late = !arrive_and_wait();
+    } else {
+      ++meeting;
+    }
     if (__syncthreads_or(late)) return false;
     if (wid == 0) {
       constexpr int PER = (GRID_MAX_CTAS + 31) / 32;

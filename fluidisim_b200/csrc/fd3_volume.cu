@@ -95,11 +95,12 @@ constexpr long long kQuadMinCells = 1LL << 23;
 // The TMA-staged kernels by default from this many cells (projections, ms, paired / TMA-staged: 112^3 basin 2.25 / 2.33;
 // 160 x 80 x 120 tank 4.26 / 4.08; 128^3 basin 2.60 / 2.53; 160^3 3.94 / 3.61; 256^3 wave 10.25 / 9.38).
 constexpr long long kTmaMinCells = 1500000;
-// The loop in one launch (k_mg_loop) up to this many cells (projections, ms, separate kernels / one launch on half of the
-// SMs, as it runs: 48^3 1.00 / 0.91, 64^3 1.04 / 0.98, 64 x 64 x 80 1.14 / 1.17, 128 x 64 x 48 1.11 / 1.25, 72^3 1.55 / 1.94).
-// With every SM it would win up to 400,000 cells (1.08, 1.02 and 1.57; 128 x 64 x 96 1.36 / 1.43, 96^3 1.56 / 1.65), but then
-// volumes on several streams would follow one another.
-constexpr long long kLoopMaxCells = 1LL << 18;
+// The loop in one launch (k_mg_loop) up to this many cells (a projection alone, ms, separate kernels / one launch: 48^3
+// 1.00 / 0.89, 64^3 1.04 / 0.94, 64 x 64 x 80 1.14 / 1.11, 128 x 64 x 48 1.11 / 1.02, 96 x 64 x 64 1.23 / 1.18; 72^3 1.55 / 1.57,
+// 160 x 40 x 56 1.33 / 1.39, 80^3 1.35 / 1.38, 128 x 64 x 96 1.36 / 1.43, 96^3 1.56 / 1.65): above, its slowest team's chunks cost
+// more than the launches it saves.  Without a coarse level the fine passes are all it has, and many iterations of them:
+// 64 x 63 x 64 4.50 / 2.89, 108 x 54 x 81 6.37 / 4.18, 124 x 62 x 93 7.74 / 6.49, 100 x 101 x 100 8.89 / 7.76.
+constexpr long long kLoopMaxCells = 3LL << 17, kLoopMaxCellsFlat = 1LL << 20;
 
 // Coarse levels of at most this many cells are solved together by one CTA (k_coarse_tail).
 constexpr int TAIL_MAX_CELLS = 512;
@@ -113,6 +114,22 @@ static_assert(kRoundoff2D == BATCH_ROUNDOFF_2D && kRoundoff3D == BATCH_ROUNDOFF_
               "the persistent batch shares the outer loop's constants");
 
 }  // namespace
+
+// Projections in progress on a device, in all threads of the process.  The one-launch loops take their share of the SMs by
+// it; nothing else depends on it.
+class InProgress {
+ public:
+  explicit InProgress(int device) : n(on(device)) { n.fetch_add(1, std::memory_order_relaxed); }
+  ~InProgress() { n.fetch_sub(1, std::memory_order_relaxed); }
+  InProgress(const InProgress&) = delete;
+  static std::atomic<int>& on(int device) {
+    static std::atomic<int> counts[64];
+    return counts[device & 63];
+  }
+
+ private:
+  std::atomic<int>& n;
+};
 
 struct fd3_volume {
   int device = 0;
@@ -267,20 +284,25 @@ struct fd3_volume {
            (opt.no_tile_skip ? 256 : 0) | (skip_air ? 2048 : 0) | (quad() ? 512 : 0) | (tmaf() ? 1024 : 0);
   }
   // With the multigrid, the inner loop in one cooperative launch (k_mg_loop): the default on the paired march up to
-  // kLoopMaxCells.  Profiling, use_graphs = 0 and kernels = 3 keep the separate kernels.
+  // kLoopMaxCells, or kLoopMaxCellsFlat.  Profiling, use_graphs = 0 and kernels = 3 keep the separate kernels.
   bool mg_loop() const {
-    return opt.kernels == 0 && paired() && mg_on() && (long long)n <= kLoopMaxCells && opt.use_graphs && !prof &&
+    return opt.kernels == 0 && paired() && mg_on() && n <= (levels.empty() ? kLoopMaxCellsFlat : kLoopMaxCells) &&
+           opt.use_graphs && !prof &&
            grid_ctas > 0 && tail_reg && tail_first <= MG_LEVELS && mg_fits(nx, ny);
   }
-  // Its CTAs, which fill an SM each: a team (three to a CTA) per chunk of two layers, but at most half of the SMs, so that
-  // volumes on two streams run side by side, and an equal share of them among the workers of fd3_project_batch.  The
-  // result does not depend on it.  Measured (ms, 148 / 74 / 37 CTAs): 64^3 alone 0.94 / 0.98 / 1.23, two at once 1.90 / 1.12 /
-  // 1.39, sixteen 14.7 / 8.0 / 5.4 (3.4 at 9); 32^3 alone 0.70 / 0.70 / 0.71 (0.73 at 22, 0.75 at 16), sixteen 10.0 / 5.1 / 2.8
-  // (1.35 at 9).  256 patches by sixteen workers: 217 with every SM each, 65 as separate kernels, 42 so.
+  // Volumes that the GPU is projecting, this one among them: of fd3_project_batch's workers, or of callers' threads.
+  int at_once() const { return std::max(workers, InProgress::on(device).load(std::memory_order_relaxed)); }
+  // CTAs of the one-launch loop, which fill an SM each for the whole solve: beside other volumes an equal share of the
+  // SMs; alone half of them up to 2^17 cells whose chunks of two layers have a team (three to a CTA) each there, which leaves
+  // room for a volume that comes meanwhile and costs 1% or so, else every SM.  The result does not depend on it.  Measured (ms, 148 /
+  // 74 / 37 CTAs): 48^3 alone 0.89 / 0.90 / 0.96, two at once 1.72 / 0.95 / 1.00; 64^3 alone 0.94 / 0.98 / 1.23, two at once 1.90 /
+  // 1.12 / 1.39, sixteen 14.7 / 8.0 / 5.4 (3.4 at 9); 128 x 64 x 48 alone 1.02 / 1.25.  256 patches by sixteen workers: 217 with
+  // every SM each, 65 as separate kernels, 42 so.
   int mg_ctas() const {
+    const int together = at_once(), half = (grid_ctas + 1) / 2;
+    if (together > 1) return std::min(std::max(MG_LEAST_SHARE, grid_ctas / together), grid_ctas);
     const int chunks = ((nx + Z2X - 1) / Z2X) * ((ny + Z2Y - 1) / Z2Y) * ((nz + 1) / 2);
-    const int share = std::max(MG_LEAST_SHARE, grid_ctas / std::max(workers, 2));
-    return std::min({std::max(MG_MIN_CTAS, (chunks + MG_TEAMS - 1) / MG_TEAMS), share, grid_ctas});
+    return n <= 1 << 17 && chunks <= MG_TEAMS * half ? half : grid_ctas;
   }
   bool one_launch() const { return cg_loop() || mg_loop(); }
   Red red() const { return Red{p64, p32, count}; }
@@ -994,9 +1016,10 @@ void run_cg_loop(fd3_volume* V) {
   // Beside other volumes: a half of the CTAs, or a quarter, each standing in for the others.  Sixteen volumes by sixteen
   // workers, ms, whole grids / so: 40,095 cells 10.1 / 3.2, 66,185 11.8 / 5.0, 77,775 8.4 / 5.5, 111,569 12.4 / 8.3.  From three
   // cells per thread on the SMs are as full either way (215,025 cells: 20.5 whole, 23.2 on half as many).
-  if (cells <= 1 && V->workers >= 4) launch_cg_loop<4, 4>(V, ctas);
-  else if (cells <= 1 && V->workers > 1) launch_cg_loop<2, 2>(V, ctas);
-  else if (cells <= 2 && V->workers > 1) launch_cg_loop<4, 2>(V, ctas);
+  const int together = V->at_once();
+  if (cells <= 1 && together >= 4) launch_cg_loop<4, 4>(V, ctas);
+  else if (cells <= 1 && together > 1) launch_cg_loop<2, 2>(V, ctas);
+  else if (cells <= 2 && together > 1) launch_cg_loop<4, 2>(V, ctas);
   else if (cells <= 1) launch_cg_loop<1>(V, ctas);
   else if (cells <= 2) launch_cg_loop<2>(V, ctas);
   else if (cells <= 3) launch_cg_loop<3>(V, ctas);
@@ -1363,6 +1386,7 @@ int project_rows(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_r
 // With f64 reductions, an even nx and the multigrid, the passes leave the air above the surface alone
 // (Geo::ztop); fd3_options.no_tile_skip switches that off with the tiles'.
 int project_mobile3(fd3_volume* V, float scale, float k1, uint32_t max_iters, fd3_report* rep) {
+  const InProgress self(V->device);
   V->skip_air = V->mg_on() && V->paired() && !V->opt.no_tile_skip;
   const int e = project_rows(V, scale, k1, max_iters, rep);
   V->skip_air = false;

@@ -88,9 +88,9 @@ typedef struct fd3_options {
   uint32_t mg_max_levels; /* coarse levels kept by fd3_enable_multigrid; 0 = every level the
                              reference's coarsening rule allows (delta3d_multigrid.rs:73-88) */
   uint32_t use_graphs;    /* 1 = run the inner loop without the host: in one cooperative launch
-                             (f64 sums; with the multigrid up to 2^18 cells at kernels = 0, without it
-                             while the blocks of one launch, one per SM, hold the volume), else as a
-                             CUDA graph with a WHILE node */
+                             (f64 sums; with the multigrid up to 393,216 cells, or 2^20 without a
+                             coarse level, at kernels = 0, without it while the blocks of one launch,
+                             one per SM, hold the volume), else as a CUDA graph with a WHILE node */
   uint32_t kernels;       /* fine-level kernels in f64 mode: 0 = 2.5-D blocked (default): on volumes
                              of 1,500,000 cells or more with f32 storage the TMA-staged kernels
                              (nx % 8 == 0), from 2^23 cells four cells per thread (nx % 4 == 0), else
@@ -252,8 +252,8 @@ int fd3_advect_for_tests(fd3_volume* v, float dt);
  * loop; `threads` host workers (0 = up to 16) issue them, largest first.  statuses[i] and
  * reports[i] are volume i's; the return value is FD3_OK unless the arguments are invalid (a null
  * pointer, or one volume listed twice).  A volume whose loop is one cooperative launch (see
- * use_graphs) takes its share of the SMs: a part of them per worker, and its result does not depend on
- * how many.  fd3_batch_* is the faster way for many volumes. */
+ * use_graphs) has every SM while no other is being projected, else its share of them, and the same
+ * result with any.  fd3_batch_* is the faster way for many volumes. */
 int fd3_project_batch(fd3_volume* const* volumes, size_t count, const float* scales, const float* k1s,
                       uint32_t max_iters, int threads, fd3_report* reports, int* statuses);
 /* The persistent batch (no reference counterpart): many volumes (patches) projected by ONE kernel

@@ -32,7 +32,7 @@ def launches(shape, multigrid, linear=False, iterations=12, **options):
 
 
 @pytest.mark.parametrize("storage", [0, STORAGE_F16])
-@pytest.mark.parametrize("shape", [(32, 16, 24), (64, 64, 64)])
+@pytest.mark.parametrize("shape", [(32, 16, 24), (64, 64, 64), (128, 64, 48)])
 def test_multigrid_in_one_launch_up_to_the_line(shape, storage):
     n, its = launches(shape, True, storage=storage)
     assert n <= SETUP
@@ -40,9 +40,15 @@ def test_multigrid_in_one_launch_up_to_the_line(shape, storage):
     assert n >= 6 * its
 
 
-@pytest.mark.parametrize("shape", [(66, 64, 64), (128, 64, 48)])
+def test_without_a_coarse_level_the_line_is_higher():
+    assert launches((124, 62, 93), True)[0] <= SETUP
+    n, its = launches((102, 101, 102), True)
+    assert 102 * 101 * 102 > 2 ** 20 and n >= 6 * its
+
+
+@pytest.mark.parametrize("shape", [(130, 64, 48), (72, 72, 80)])
 def test_multigrid_above_the_line(shape):
-    assert 2 ** 18 < shape[0] * shape[1] * shape[2]
+    assert 3 * 2 ** 17 < shape[0] * shape[1] * shape[2]
     n, its = launches(shape, True)
     assert n >= 6 * its
     assert n == launches(shape, True, kernels=3)[0]
