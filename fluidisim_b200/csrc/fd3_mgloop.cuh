@@ -43,6 +43,11 @@ struct MgShared {
   ZResid2 tr[MG_TEAMS][2];
   TailShared tail;
   GridShared grid;
+  // The loop's scalars, the same for every thread (thread 0 writes them).  In registers they would be spilled in the passes,
+  // and a spilled register is read from L2 after each meeting: 150 bytes of spills less, 1% of a 64^3 projection.
+  double rr, rz, rn, tolb2, phys;
+  unsigned max_iters;
+  float vk, vinv;
 };
 
 struct TeamSync {
@@ -133,11 +138,10 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
     for (int w = (tid >> 5) * gridDim.x + blockIdx.x; 32 * w < n; w += gridDim.x * (MG_THREADS / 32)) f(32 * w + (tid & 31));
   };
   auto air = [&](int l) { return Air{l < 3 ? a.air.ztop : nullptr, l + 1, a.air.ntx}; };
-  float vinv = S->vinv;
 
   // z = M^-1 r with r.z in rz (v_cycle3); false when a meeting failed
   auto vcycle = [&](double& rz) -> bool {
-    const float rs = Store<T>::half ? vinv : 1.f;
+    const float rs = Store<T>::half ? sh.vinv : 1.f;
     const bool levels = a.nlev + a.ntail > 0;
     each_chunk([&](const auto& m) { march_pre(m, a.prec, a.r, z, rs); });
     if (!grid.meet()) return false;
@@ -208,10 +212,16 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
     return met;
   };
 
-  const double tolb2 = S->tolb2, phys = S->phys;
-  const unsigned max_iters = S->max_iters;
-  const float vk = S->vk;
-  double rr = S->rr, rn = rr, rz = 0.0;
+  if (tid == 0) {
+    sh.rr = S->rr;
+    sh.rz = 0.0;
+    sh.tolb2 = S->tolb2;
+    sh.phys = S->phys;
+    sh.max_iters = S->max_iters;
+    sh.vk = S->vk;
+    sh.vinv = S->vinv;
+  }
+  __syncthreads();
   unsigned it = S->it;
   int status = 0, brk = 0, mode = 0;
   float beta = 0.f;
@@ -222,11 +232,12 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
     if (!vcycle(zn)) { status = 100; break; }
     if (!isfinite(zn)) { status = 2; break; }
     if (mode) {  // FIN_RZ_ITER
-      beta = (float)(zn / rz);
-      rr = rn;
+      beta = (float)(zn / sh.rz);
+      if (tid == 0) sh.rr = sh.rn;
       ++it;
     }
-    rz = zn;
+    __syncthreads();
+    if (tid == 0) sh.rz = zn;
     const float* din = a.dir[it & 1];
     float* dout = a.dir[(it & 1) ^ 1];
     bool met;
@@ -237,24 +248,30 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_mg_loop(const __grid_constant
     });
     if (!met) { status = 100; break; }
     if (!(dq > 0.0)) { brk = 1; break; }  // FIN_DQ
-    const float alpha = (float)(rz / dq);
-    rn = sum_chunks(met, [&](const auto& m) {
+    const float alpha = (float)(sh.rz / dq);
+    const double rn = sum_chunks(met, [&](const auto& m) {
       double acc = 0.0;
       chunk_update(g, m.t, alpha, a.p, a.r, dout, a.q, acc);
       return acc;
     });
     if (!met) { status = 100; break; }
     if (!isfinite(rn)) { status = 2; break; }  // FIN_RN
-    if (vk > 0.f && rn > 0.0) vinv = (float)((double)vk / sqrt(rn));
-    if (!((rn > tolb2 || rn > phys) && it + 1 < max_iters)) { rr = rn; ++it; break; }
+    if (tid == 0 && sh.vk > 0.f && rn > 0.0) sh.vinv = (float)((double)sh.vk / sqrt(rn));
+    if (Store<T>::half) __syncthreads();  // vinv, before the next V-cycle reads it
+    if (!((rn > sh.tolb2 || rn > sh.phys) && it + 1 < sh.max_iters)) {
+      if (tid == 0) sh.rr = rn;
+      ++it;
+      break;
+    }
+    if (tid == 0) sh.rn = rn;
     mode = 1;
   }
   if (tid == 0 && (first_cta || status == 100)) {
-    S->rr = rr;
-    S->rz = rz;
+    S->rr = sh.rr;
+    S->rz = sh.rz;
     S->it = it;
     S->brk = brk;
-    S->vinv = vinv;
+    S->vinv = sh.vinv;
     if (status) S->status = status;
     S->active = 0;
   }

@@ -293,8 +293,8 @@ struct fd3_volume {
   // Volumes that the GPU is projecting, this one among them: of fd3_project_batch's workers, or of callers' threads.
   int at_once() const { return std::max(workers, InProgress::on(device).load(std::memory_order_relaxed)); }
   // CTAs of the one-launch loop, which fill an SM each for the whole solve: beside other volumes an equal share of the
-  // SMs; alone half of them up to 2^17 cells whose chunks of two layers have a team (three to a CTA) each there, which leaves
-  // room for a volume that comes meanwhile and costs 1% or so, else every SM.  The result does not depend on it.  Measured (ms, 148 /
+  // SMs; alone half of them up to 2^17 cells whose chunks of two layers have a team (three to a CTA) each there and whose
+  // levels end in the tail, which leaves room for a volume that comes meanwhile and costs 1% or so, else every SM.  The result does not depend on it.  Measured (ms, 148 /
   // 74 / 37 CTAs): 48^3 alone 0.89 / 0.90 / 0.96, two at once 1.72 / 0.95 / 1.00; 64^3 alone 0.94 / 0.98 / 1.23, two at once 1.90 /
   // 1.12 / 1.39, sixteen 14.7 / 8.0 / 5.4 (3.4 at 9); 128 x 64 x 48 alone 1.02 / 1.25.  256 patches by sixteen workers: 217 with
   // every SM each, 65 as separate kernels, 42 so.
@@ -302,7 +302,7 @@ struct fd3_volume {
     const int together = at_once(), half = (grid_ctas + 1) / 2;
     if (together > 1) return std::min(std::max(MG_LEAST_SHARE, grid_ctas / together), grid_ctas);
     const int chunks = ((nx + Z2X - 1) / Z2X) * ((ny + Z2Y - 1) / Z2Y) * ((nz + 1) / 2);
-    return n <= 1 << 17 && chunks <= MG_TEAMS * half ? half : grid_ctas;
+    return n <= 1 << 17 && chunks <= MG_TEAMS * half && tail_first < (int)levels.size() ? half : grid_ctas;
   }
   bool one_launch() const { return cg_loop() || mg_loop(); }
   Red red() const { return Red{p64, p32, count}; }
